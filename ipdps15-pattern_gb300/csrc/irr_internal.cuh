@@ -117,13 +117,9 @@ struct TiledShape {
 #ifndef IRR_HALO_STREAMMAX
 #define IRR_HALO_STREAMMAX 3584
 #endif
-#ifndef IRR_HALO_STAGES
-#define IRR_HALO_STAGES 2
-#endif
 constexpr int kHaloSlicesPerItem = IRR_HALO_SLICES;  // 64 rows per item at most
 constexpr int kHaloTabMax = IRR_HALO_TABMAX;         // table ids per item (~10 KB of positions)
 constexpr int kHaloStreamMax = IRR_HALO_STREAMMAX;   // words per item (14 KB)
-constexpr int kHaloStages = IRR_HALO_STAGES;         // shared-memory ring depth
 struct Staged {
     uint32_t* slice_off = nullptr;   // [slices + 1] word offsets (multiples of 32)
     uint32_t* words = nullptr;       // [nwords]

@@ -222,14 +222,14 @@ __device__ __forceinline__ InstHot hot_from(const SrcTable& t, const InstDesc* i
     return h;
 }
 
-// wrap_component (irr_law.cuh) without branches: both shifted forms are
-// formed and the one the sign of d calls for is selected.
-__device__ __forceinline__ float wrap_select(float a, float b, float d, float half, float shi,
-                                             float slo)
+// One component of the minimum image, as b - a: d itself within half the box,
+// else the negative of wrap_component (irr_law.cuh), bit for bit -- the larger
+// of the two coordinates is taken down by the side first, whichever it is, and
+// the sign is d's turned round.
+__device__ __forceinline__ float wrap_diff(float a, float b, float d, float half, float shi, float slo)
 {
-    const float up = __fsub_rn(__fsub_rn(__fsub_rn(a, shi), b), slo);  // d > half
-    const float dn = __fadd_rn(__fsub_rn(a, __fsub_rn(b, shi)), slo);  // d < -half
-    return d > half ? up : (d < -half ? dn : d);
+    const float m = __fsub_rn(__fsub_rn(__fsub_rn(fmaxf(a, b), shi), fminf(a, b)), slo);
+    return fabsf(d) > half ? (d > 0.f ? m : -m) : d;
 }
 
 template <bool PERIODIC>
@@ -245,32 +245,6 @@ __device__ __forceinline__ float rcp_approx(float x)
     return r;
 }
 
-// The rare cases of an entry pair: a pair past half the box (periodic) is
-// re-wrapped exactly, and a pair whose rd lies within `band` of the cutoff
-// takes the reference's FP64 decision.  Updates d, rd and the in-flags.
-template <bool PERIODIC>
-__device__ __forceinline__ void rare_pair(float4 a, float4 b0, float4 b1, const HotLaw& H,
-                                          const LawParams* __restrict__ cold, float2& dx,
-                                          float2& dy, float2& dz, float2& rd, bool& in0, bool& in1)
-{
-    if (PERIODIC && fmaxf(rd.x, rd.y) > H.half2) {
-        // every component of both slots through wrap_select (a component
-        // within half the box comes back unchanged, bit for bit)
-        const float half = cold->half, shi = cold->side_hi, slo = cold->side_lo;
-        dx.x = wrap_select(a.x, b0.x, dx.x, half, shi, slo);
-        dy.x = wrap_select(a.y, b0.y, dy.x, half, shi, slo);
-        dz.x = wrap_select(a.z, b0.z, dz.x, half, shi, slo);
-        dx.y = wrap_select(a.x, b1.x, dx.y, half, shi, slo);
-        dy.y = wrap_select(a.y, b1.y, dy.y, half, shi, slo);
-        dz.y = wrap_select(a.z, b1.z, dz.y, half, shi, slo);
-        rd = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-        in0 = rd.x < H.rc2;
-        in1 = rd.y < H.rc2;
-    }
-    if (fabsf(__fsub_rn(rd.x, H.rc2)) < H.band) in0 = exact_inside_g<PERIODIC>(a, b0, cold);
-    if (fabsf(__fsub_rn(rd.y, H.rc2)) < H.band) in1 = exact_inside_g<PERIODIC>(a, b1, cold);
-}
-
 // Two entries (b0, b1) of the row of node a, evaluated with packed FP32x2
 // arithmetic (each half rounds exactly as the scalar law in irr_law.cuh), and
 // accumulated into the lane's packed partials.  A slot with v == false
@@ -278,35 +252,86 @@ __device__ __forceinline__ void rare_pair(float4 a, float4 b0, float4 b1, const 
 //
 // The differences are formed by scalar subtractions written straight into
 // register pairs (the two positions come from separate loads, so a packed
-// subtraction would first have to move them into pairs).  A component
-// |d| > side/2 implies rd > (side/2)^2, so the wrap test is one compare on
-// rd; it and the cutoff-band test are folded into one branch to the rare
-// path (a pair across the box wall, beyond half the box, or within 2^-18 of
-// the cutoff).  (A warp vote in front of it measured slower.)
+// subtraction would first have to move them into pairs).  They are b - a, the
+// law's scalar is -s and the reciprocal -1/rd: every value is the exact
+// negative of the scalar law's, and their products are the same bits.
+struct PairDiff {
+    float2 x, y, z;  // b - a of the two entries
+    float2 rd;       // squared distances
+};
+
+__device__ __forceinline__ PairDiff pair_diff(float4 a, float4 b0, float4 b1)
+{
+    PairDiff d;
+    d.x = make_float2(__fsub_rn(b0.x, a.x), __fsub_rn(b1.x, a.x));
+    d.y = make_float2(__fsub_rn(b0.y, a.y), __fsub_rn(b1.y, a.y));
+    d.z = make_float2(__fsub_rn(b0.z, a.z), __fsub_rn(b1.z, a.z));
+    d.rd = __ffma2_rn(d.x, d.x, __ffma2_rn(d.y, d.y, __fmul2_rn(d.z, d.z)));
+    return d;
+}
+
+__device__ __forceinline__ void add_pair(const PairDiff& d, bool in0, bool in1, float2& ax, float2& ay,
+                                         float2& az)
+{
+    float2 r = make_float2(rcp_approx(-d.rd.x), rcp_approx(-d.rd.y));
+    const float2 e = __ffma2_rn(d.rd, r, make_float2(1.0f, 1.0f));
+    r = __ffma2_rn(r, e, r);             // -rd^-1 (one Newton step)
+    const float2 r2 = __fmul2_rn(r, r);  // rd^-2
+    float2 s = __fmul2_rn(__fmul2_rn(r2, r2), __ffma2_rn(r2, r, make_float2(0.5f, 0.5f)));
+    s.x = in0 ? s.x : 0.0f;
+    s.y = in1 ? s.y : 0.0f;
+    ax = __ffma2_rn(d.x, s, ax);
+    ay = __ffma2_rn(d.y, s, ay);
+    az = __ffma2_rn(d.z, s, az);
+}
+
+// The rare cases of an entry pair: a pair past half the box (periodic) is
+// re-wrapped exactly, and a pair whose rd lies within `band` of the cutoff
+// takes the reference's FP64 decision.  Updates d and the in-flags.
+template <bool PERIODIC>
+__device__ __forceinline__ void rare_pair(float4 a, float4 b0, float4 b1, const HotLaw& H,
+                                          const LawParams* __restrict__ cold, PairDiff& d, bool& in0,
+                                          bool& in1)
+{
+    if (PERIODIC && fmaxf(d.rd.x, d.rd.y) > H.half2) {
+        // most pairs across the wall cross it on one axis: the others are skipped
+        const float half = cold->half, shi = cold->side_hi, slo = cold->side_lo;
+        if (fmaxf(fabsf(d.x.x), fabsf(d.x.y)) > half) {
+            d.x.x = wrap_diff(a.x, b0.x, d.x.x, half, shi, slo);
+            d.x.y = wrap_diff(a.x, b1.x, d.x.y, half, shi, slo);
+        }
+        if (fmaxf(fabsf(d.y.x), fabsf(d.y.y)) > half) {
+            d.y.x = wrap_diff(a.y, b0.y, d.y.x, half, shi, slo);
+            d.y.y = wrap_diff(a.y, b1.y, d.y.y, half, shi, slo);
+        }
+        if (fmaxf(fabsf(d.z.x), fabsf(d.z.y)) > half) {
+            d.z.x = wrap_diff(a.z, b0.z, d.z.x, half, shi, slo);
+            d.z.y = wrap_diff(a.z, b1.z, d.z.y, half, shi, slo);
+        }
+        d.rd = __ffma2_rn(d.x, d.x, __ffma2_rn(d.y, d.y, __fmul2_rn(d.z, d.z)));
+        in0 = d.rd.x < H.rc2;
+        in1 = d.rd.y < H.rc2;
+    }
+    if (fabsf(__fsub_rn(d.rd.x, H.rc2)) < H.band) in0 = exact_inside_g<PERIODIC>(a, b0, cold);
+    if (fabsf(__fsub_rn(d.rd.y, H.rc2)) < H.band) in1 = exact_inside_g<PERIODIC>(a, b1, cold);
+}
+
+// A component |d| > side/2 implies rd > (side/2)^2, so the wrap test is one
+// compare on rd; it and the cutoff-band test are folded into one branch to
+// the rare path (a pair across the box wall, beyond half the box, or within
+// 2^-18 of the cutoff).  (A warp vote in front of it measured slower.)
 template <bool PERIODIC>
 __device__ __forceinline__ void lj_pair(float4 a, float4 b0, float4 b1, bool v0, bool v1, const HotLaw& H,
                                         const LawParams* __restrict__ cold, float2& ax, float2& ay,
                                         float2& az)
 {
-    float2 dx = make_float2(__fsub_rn(a.x, b0.x), __fsub_rn(a.x, b1.x));
-    float2 dy = make_float2(__fsub_rn(a.y, b0.y), __fsub_rn(a.y, b1.y));
-    float2 dz = make_float2(__fsub_rn(a.z, b0.z), __fsub_rn(a.z, b1.z));
-    float2 rd = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    const float2 t = __fadd2_rn(rd, make_float2(-H.rc2, -H.rc2));
+    PairDiff d = pair_diff(a, b0, b1);
+    const float2 t = __fadd2_rn(d.rd, make_float2(-H.rc2, -H.rc2));
     bool rare = fminf(fabsf(t.x), fabsf(t.y)) < H.band;
-    if (PERIODIC) rare = rare || fmaxf(rd.x, rd.y) > H.half2;
-    bool in0 = rd.x < H.rc2, in1 = rd.y < H.rc2;
-    if (rare) rare_pair<PERIODIC>(a, b0, b1, H, cold, dx, dy, dz, rd, in0, in1);
-    float2 r = make_float2(rcp_approx(rd.x), rcp_approx(rd.y));
-    const float2 e = __ffma2_rn(make_float2(-rd.x, -rd.y), r, make_float2(1.0f, 1.0f));
-    r = __ffma2_rn(r, e, r);                                     // rd^-1 (one Newton step)
-    const float2 r2 = __fmul2_rn(r, r);                          // rd^-2
-    float2 s = __fmul2_rn(__fmul2_rn(r2, r2), __ffma2_rn(r2, r, make_float2(-0.5f, -0.5f)));
-    s.x = (in0 && v0) ? s.x : 0.0f;
-    s.y = (in1 && v1) ? s.y : 0.0f;
-    ax = __ffma2_rn(dx, s, ax);
-    ay = __ffma2_rn(dy, s, ay);
-    az = __ffma2_rn(dz, s, az);
+    if (PERIODIC) rare = rare || fmaxf(d.rd.x, d.rd.y) > H.half2;
+    bool in0 = d.rd.x < H.rc2, in1 = d.rd.y < H.rc2;
+    if (rare) rare_pair<PERIODIC>(a, b0, b1, H, cold, d, in0, in1);
+    add_pair(d, in0 && v0, in1 && v1, ax, ay, az);
 }
 
 // The row's result from its G lanes' packed partials: the two halves of each
@@ -353,22 +378,66 @@ __device__ __forceinline__ float3 join_partials(float2 ax, float2 ay, float2 az)
     return make_float3(r.x, r.y, __fadd_rn(hz, cz));
 }
 
+// join_partials<4>, each lane left with one component: lane 0 x, 1 y, 2 and 3
+// z.  The exchanges are arranged so that a lane sums only the components it
+// keeps: after the halves, lanes 0 and 1 take x and y over (0, 2) and (1, 3)
+// while lanes 2 and 3 take z, then lane 0 x, lane 1 y.  The same pairs are
+// added as in join_partials and TwoSum's sum and error do not depend on the
+// order of its operands, so the bits are the same, with 6 shuffles instead of
+// 12 and one and a half instead of two rounds of sums (halo_kernel at 4M nodes
+// 363.4 -> 358.2 us, tiled_kernel at 864,000 atoms 123.8 -> 120.8 us).
+__device__ __forceinline__ float join4_scatter(float2 ax, float2 ay, float2 az, int lane)
+{
+    float2 h, c;
+    float hz, cz;
+    two_sum2(make_float2(ax.x, ay.x), make_float2(ax.y, ay.y), h, c);
+    two_sum(az.x, az.y, hz, cz);
+    const bool up = lane & 2;
+    const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, up ? h.x : hz, 2, 4),
+                                 __shfl_xor_sync(0xffffffffu, h.y, 2, 4));
+    const float2 oc = make_float2(__shfl_xor_sync(0xffffffffu, up ? c.x : cz, 2, 4),
+                                  __shfl_xor_sync(0xffffffffu, c.y, 2, 4));
+    h.x = up ? hz : h.x;
+    c.x = up ? cz : c.x;
+    float2 e;
+    two_sum2(h, o, h, e);
+    c = __fadd2_rn(__fadd2_rn(c, oc), e);
+    const float p = __shfl_xor_sync(0xffffffffu, lane == 0 ? h.y : h.x, 1, 4);
+    const float pc = __shfl_xor_sync(0xffffffffu, lane == 0 ? c.y : c.x, 1, 4);
+    const float k = lane == 1 ? h.y : h.x, kc = lane == 1 ? c.y : c.x;
+    float s, se;
+    two_sum(k, p, s, se);
+    return __fadd_rn(s, __fadd_rn(__fadd_rn(kc, pc), se));
+}
+
+// Row r's result from its G lanes' partials (valid rows only), written once.
+template <int G>
+__device__ __forceinline__ void write_row(float4* __restrict__ force, int64_t r, bool valid, float2 ax,
+                                          float2 ay, float2 az, int lane)
+{
+    if constexpr (G == 4) {
+        const float f = join4_scatter(ax, ay, az, lane);
+        if (valid) reinterpret_cast<float*>(force + r)[lane] = lane == 3 ? 0.f : f;
+    } else {
+        const float3 f = join_partials<G>(ax, ay, az);
+        if (valid && lane == 0) force[r] = make_float4(f.x, f.y, f.z, 0.f);
+    }
+}
+
 // One row: G lanes; each lane takes entry pairs (k, k + G) with stride 2G.
 // Entry k of the row is cols[k - shift].
 template <bool PERIODIC, int G>
-__device__ __forceinline__ float3 row_sum(const float4* __restrict__ pos, const int32_t* cols,
-                                          uint32_t shift, float4 a, uint32_t beg, uint32_t end,
-                                          int lane, const HotLaw& H,
-                                          const LawParams* __restrict__ cold)
+__device__ __forceinline__ void row_sum(const float4* __restrict__ pos, const int32_t* cols,
+                                        uint32_t shift, float4 a, uint32_t beg, uint32_t end, int lane,
+                                        const HotLaw& H, const LawParams* __restrict__ cold, float2& ax,
+                                        float2& ay, float2& az)
 {
-    float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
     for (uint32_t k = beg + lane; k < end; k += 2 * G) {
         const bool v1 = k + G < end;
         const float4 b0 = __ldg(pos + cols[k - shift]);
         const float4 b1 = v1 ? __ldg(pos + cols[k + G - shift]) : a;
         lj_pair<PERIODIC>(a, b0, b1, true, v1, H, cold, ax, ay, az);
     }
-    return join_partials<G>(ax, ay, az);
 }
 
 constexpr int kConsumerWarps = kConsumerSlices;
@@ -407,8 +476,9 @@ __device__ __forceinline__ void consume_item(const WorkItem& w, const InstHot& I
             beg = __ldg(row_off + r);
             end = __ldg(row_off + r + 1);
         }
-        const float3 f = row_sum<PERIODIC, G>(pos, cols, shift, a, beg, end, lane, H, cold);
-        if (valid && lane == 0) force[r] = make_float4(f.x, f.y, f.z, 0.f);
+        float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+        row_sum<PERIODIC, G>(pos, cols, shift, a, beg, end, lane, H, cold, ax, ay, az);
+        write_row<G>(force, r, valid, ax, ay, az, lane);
     }
 }
 
@@ -484,8 +554,7 @@ __device__ __forceinline__ void consume_sliced(const WorkItem& w, const InstHot&
                 lj_pair<PERIODIC>(a, b0, b1, t < n0, t < n1, H, cold, ax, ay, az);
             }
         }
-        const float3 f = join_partials<G>(ax, ay, az);
-        if (r < n && lane == 0) force[r] = make_float4(f.x, f.y, f.z, 0.f);
+        write_row<G>(force, r, r < n, ax, ay, az, lane);
     }
 }
 
@@ -619,26 +688,36 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) tiled_kernel(
 //
 // halo_kernel: the same persistent, warp-specialised owner-computes reduction
 // over the staged layout (irr_staged.cu).  Per work item the producer warp
-// bulk-copies the item's words (headers and 16-bit table offsets) into the
-// stage, and its 32 lanes gather the item's table -- the positions of every
-// node its rows touch, ~465 for 64 rows -- with 16-byte cp.async copies into
-// the stage's table; the stage's `full` barrier completes when the bulk copy's
-// bytes and all 32 lanes' copies have landed (1 + 32 arrivals).  The
-// consumers read each entry's position from shared memory (a 128-bit load at
-// a table offset), so the law's operands arrive in tens of cycles instead of
-// an L1 miss's hundreds, and the entry order of the layout spreads each
-// quarter-warp's 8 loads over the 8 bank groups.  G = 4 lanes per row.
-constexpr int kHaloStageWords = kHaloStreamMax + 4 * kHaloTabMax;  // 32-bit words per stage
+// bulk-copies the item's words (headers and 16-bit table offsets) into shared
+// memory, and its 32 lanes gather the item's table -- the positions of every
+// node its rows touch, ~465 for 64 rows -- behind them with 16-byte cp.async
+// copies; the item's `full` barrier completes when the bulk copy's bytes and
+// all 32 lanes' copies have landed (1 + 32 arrivals).  The consumers read each
+// entry's position from shared memory (a 128-bit load at a table offset), so
+// the law's operands arrive in tens of cycles instead of an L1 miss's
+// hundreds, and the entry order of the layout spreads each quarter-warp's 8
+// loads over the 8 bank groups.  G = 4 lanes per row.
+//
+// What bounds it: the issue slots of the law (83 % of the time with an
+// instant producer) and the refill of the stages, so the items lie in one ring
+// buffer, each taking the bytes it needs (~17 KB of the 24 KB limit at 64
+// neighbours per node) in whole 128-byte lines, up to kHaloSlots of them: three
+// fit where two stages of the limit's size did.  Everything else an item needs
+// (its table ids, descriptor, claim) goes through the producer's registers,
+// read one or two items ahead, so that the ring gets all of the shared memory
+// of a quarter SM.  4,194,304 nodes, 64 neighbours: 367.8 us with two stages
+// of 24 KB, 368.8 with a ring of 49,152 bytes, 358.6 with this one; 48 systems
+// of 2,000 to 120,000 nodes in one launch 153.5 -> 139.5 us, 65,536 nodes with
+// 32 neighbours 10.6 -> 9.9 us.
+constexpr int kHaloRingBytes = 56064;
+constexpr int kHaloSlots = 4;
 // The consumers add a table's address to both 16-bit halves of a word at once,
-// which needs every shared address of the CTA below 2^16: the stages, the id
-// buffers, the barriers and the system's reserved kilobyte.
-#ifndef IRR_HALO_PAIR_ADDR
-#define IRR_HALO_PAIR_ADDR 1
-#endif
-static_assert(!IRR_HALO_PAIR_ADDR ||
-                  kHaloStages * kHaloStageWords * 4 + kHaloStages * (kHaloTabMax + 8) * 4 + 1024 + 1024 <
-                      65536,
-              "shared addresses fit 16 bits");
+// and a slot's two addresses share a word, which needs every shared address of
+// the CTA below 2^16: the ring, the barriers, the metadata and the system's
+// reserved kilobyte.
+static_assert(kHaloRingBytes >= 4 * kHaloStreamMax + 16 * kHaloTabMax && kHaloRingBytes % 128 == 0 &&
+                  kHaloRingBytes + 1024 + 1024 < 65536,
+              "an item fits the ring, shared addresses fit 16 bits");
 static_assert(8 * kHaloSlicesPerItem <= 64, "a row's index in its item fits the header's 6 bits");
 
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src)
@@ -653,7 +732,7 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar)
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Shared loads kept after the stage's barrier wait (volatile, like load_pair).
+// Shared loads kept after the item's barrier wait (volatile, like load_pair).
 __device__ __forceinline__ uint32_t lds32(uint32_t addr)
 {
     uint32_t v;
@@ -670,142 +749,51 @@ __device__ __forceinline__ float4 lds128(uint32_t addr)
     return v;
 }
 
-// The slices of a staged work item (first row row0, nrows rows) that consumer
-// warp `lane32`'s warp claims from the stage's counter *claim (a warp done
-// with one slice takes the next unclaimed one, so the item's slices of
-// different lengths spread over the warps); `sw` is the stage (words, then
-// the table at word kHaloStreamMax) and soff the slices' word offsets within
-// it.  Two 16-bit table offsets of a word become shared addresses with one
-// add: every address of the CTA's shared window is below 2^16, so the low
-// half cannot carry into the high one.
-// Build-time variants (each an equal amount of work):
-//   IRR_HALO_DYNAMIC   1: warps claim slices from the stage's counter;
-//                      0: warp w takes slices w, w + 8, ...
-//   IRR_HALO_PAIR_ADDR 1: one add forms both table addresses of a word;
-//   IRR_HALO_UNROLL    the step loop's unroll factor;
-//   IRR_HALO_CWAIT     the consumers' stage wait polls with a sleep of up to
-//                      this many ns (0: suspend-hinted polls, no sleep);
-//   IRR_HALO_PWAIT     the same for the producer's wait for a free stage.
-// On the 4M-node workload (ms per step): static 0.396 vs dynamic 0.414 slice
-// claims; pair addresses 0.391 vs 0.396; 7 consumer warps 0.455 and 3 CTAs
-// per SM 0.415 vs 8 warps x 4 CTAs 0.396; rotated claims 0.3877 vs 0.3899;
-// the step loop unrolled by 2 (spills) 0.421; the steps that every row of a
-// slice fills split off into a loop without the entry masks (spills) 0.410;
-// sleep-free waits 0.393, and polls that sleep up to 128 ns to 2 us between
-// tests all 0.3875-0.3878; the entry masks as per-slice step-count bounds
-// (t < n0, t < n1 instead of 8t + lane < len) 0.4163, but as bounds on the
-// step's word address, which the loop advances anyway (no step counter or
-// index add left), 0.3736 vs 0.3876 -- the loop below; 3-stage
-// rings (3 CTAs per SM, or smaller items at 4) 0.395-0.431; 4 or 6 consumer
-// warps with 6 or 7 CTAs per SM 0.413-0.418; each item's steps cut evenly
-// across the warps (slices split between warps, piece sums joined in shared
-// memory) 0.722: the extra state around the step loop doubled its
-// instructions.  The words prefetched into L2 one item ahead: 0.3907 vs
-// 0.3873.  A table ring one buffer deeper than the word ring, each item's
-// table gathered one item ahead (limits 3072 words / 576 ids to fit 4 CTAs
-// per SM): 0.403, vs 0.3888 for this kernel at those limits and 0.3874 at
-// 3584 / 640 -- the refill is not bounded by the table gather alone.  What the warps still lose is the ring's coupling: a stage is
-// refilled only when its slowest warp is done (~4.3K cycles after the first),
-// and the refill takes ~3.6K cycles, so the first warps wait ~1.2K of each
-// item's ~7.6K cycles.
-#ifndef IRR_HALO_DYNAMIC
-#define IRR_HALO_DYNAMIC 0
-#endif
-// IRR_HALO_ROTATE 1: with static claims, warp w takes slice (w + k) mod 8 of
-// the CTA's k-th item (slice 0 holds an item's longest rows, so a fixed
-// assignment would always give warp 0 the longest slice).
-#ifndef IRR_HALO_ROTATE
-#define IRR_HALO_ROTATE 1
-#endif
-// IRR_HALO_PREFETCH 1: when the producer claims an item (one item ahead), it
-// also prefetches the item's words into L2, so that their bulk copy, issued
-// once a stage is free, reads L2 rather than DRAM.
-#ifndef IRR_HALO_PREFETCH
-#define IRR_HALO_PREFETCH 0
-#endif
-
-#ifndef IRR_HALO_UNROLL
-#define IRR_HALO_UNROLL 1
-#endif
-constexpr int kHaloUnroll = IRR_HALO_UNROLL;
-#ifndef IRR_HALO_CWAIT
-#define IRR_HALO_CWAIT 128
-#endif
-#ifndef IRR_HALO_PWAIT
-#define IRR_HALO_PWAIT 256
-#endif
-
-// A bounded wait that sleeps up to MAX_NS between polls, or (MAX_NS == 0)
-// polls with the suspend hint only.
-template <uint32_t MAX_NS>
-__device__ __forceinline__ bool mbar_wait_policy(uint64_t* bar, uint32_t parity, uint64_t limit_ns)
-{
-    if constexpr (MAX_NS == 0) return mbar_wait_bounded(bar, parity, limit_ns);
-    else return mbar_wait_backoff<MAX_NS>(bar, parity, limit_ns);
-}
+// Longest sleep between two tests of a barrier, ns (32 / 64 to 512 / 512: no
+// difference).
+constexpr uint32_t kConsumerSleep = 128, kProducerSleep = 256;
 
 // The two neighbours of a lane's step: one word of two 16-bit table byte
 // offsets, then the two positions from the table.
-__device__ __forceinline__ void halo_operands(uint32_t addr, uint32_t tab_u32, uint32_t tab_pair, float4& b0,
-                                              float4& b1)
+__device__ __forceinline__ void halo_operands(uint32_t addr, uint32_t tab_pair, float4& b0, float4& b1)
 {
-    if (IRR_HALO_PAIR_ADDR) {
-        const uint32_t wd = lds32(addr) + tab_pair;
-        b0 = lds128(wd & 0xffffu);
-        b1 = lds128(wd >> 16);
-    } else {
-        const uint32_t wd = lds32(addr);
-        b0 = lds128(tab_u32 + (wd & 0xffffu));
-        b1 = lds128(tab_u32 + (wd >> 16));
-    }
+    const uint32_t wd = lds32(addr) + tab_pair;
+    b0 = lds128(wd & 0xffffu);
+    b1 = lds128(wd >> 16);
 }
 
+// One slice: lane i * 4 + l of the warp serves row i.  addr: this lane's
+// header word; steps: words per lane after it.
+struct HaloSlice {
+    uint32_t addr;
+    uint32_t steps;
+    uint32_t tab_pair;  // the table's address in both halves
+    int row0;
+};
+
 template <bool PERIODIC>
-__device__ __forceinline__ void consume_halo(int row0, int nrows, const uint32_t* soff, int* claim,
-                                             const InstHot& I, const uint32_t* sw, int lane32,
-                                             int first)
+__device__ __forceinline__ void halo_slice(const HaloSlice& sl, const InstHot& I)
 {
-    const int lane = lane32 & 3;
-    float4* __restrict__ force = I.force;
-    const LawParams* __restrict__ cold = I.cold;
+    const int lane = threadIdx.x & 3;
     const HotLaw H = I.H;
-    const uint32_t words_u32 = smem_u32(sw);
-    const uint32_t tab_u32 = smem_u32(sw + kHaloStreamMax);
-    const uint32_t tab_pair = tab_u32 * 0x10001u;  // the table's address in both halves
-    const int ns = (nrows + 7) / 8;
-    for (int qs = first;; qs += kConsumerWarps) {
-        int q = qs;
-        if (IRR_HALO_DYNAMIC) {
-            if (lane32 == 0) q = atomicAdd(claim, 1);
-            q = __shfl_sync(0xffffffffu, q, 0);
-        }
-        if (q >= ns) break;
-        const uint32_t o0 = soff[q];
-        const uint32_t steps = ((soff[q + 1] - o0) >> 5) - 1;
-        uint32_t addr = words_u32 + 4u * (o0 + (uint32_t)lane32);
-        // header: own byte offset | len << 14 | row-in-item << 24 (1 << 31: padding)
-        const uint32_t hdr = lds32(addr);
-        const float4 a = lds128(tab_u32 + (hdr & 0x3fffu));
-        const uint32_t len = (hdr >> 14) & 0x3ffu;
-        const int64_t r = (int64_t)row0 + ((hdr >> 24) & 0x3fu);
-        float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
-        // entry 8t + lane (+ 4) of the row exists for t < n0 (n1): as bounds on
-        // step t's word address, base + 128 (t + 1), they cost no index
-        // arithmetic in the loop (8t + lane < len per step measured 3.5 %
-        // slower at 4M nodes)
-        const uint32_t n0 = len > (uint32_t)lane ? (len - (uint32_t)lane + 7u) >> 3 : 0u;
-        const uint32_t n1 = len > (uint32_t)lane + 4u ? (len - (uint32_t)lane + 3u) >> 3 : 0u;
-        const uint32_t lim0 = addr + 128u * n0, lim1 = addr + 128u * n1, end = addr + 128u * steps;
-#pragma unroll kHaloUnroll
-        for (; addr != end;) {
-            addr += 128u;
-            float4 b0, b1;
-            halo_operands(addr, tab_u32, tab_pair, b0, b1);
-            lj_pair<PERIODIC>(a, b0, b1, addr <= lim0, addr <= lim1, H, cold, ax, ay, az);
-        }
-        const float3 f = join_partials<4>(ax, ay, az);
-        if (!(hdr >> 31) && lane == 0) force[r] = make_float4(f.x, f.y, f.z, 0.f);
+    uint32_t addr = sl.addr;
+    // header: own byte offset | len << 14 | row-in-item << 24 (1 << 31: padding)
+    const uint32_t hdr = lds32(addr);
+    const float4 a = lds128((sl.tab_pair & 0xffffu) + (hdr & 0x3fffu));
+    const uint32_t len = (hdr >> 14) & 0x3ffu;
+    float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+    // entry 8t + lane (+ 4) of the row exists for 8t < len - lane (- 4): as
+    // bounds on step t's word address, base + 128 (t + 1)
+    const uint32_t lim0 = addr + 16u * ((len + 7u - (uint32_t)lane) & ~7u);
+    const uint32_t lim1 = addr + 16u * ((len + 3u - (uint32_t)lane) & ~7u);
+    const uint32_t end = addr + 128u * sl.steps;
+    for (; addr != end;) {
+        addr += 128u;
+        float4 b0, b1;
+        halo_operands(addr, sl.tab_pair, b0, b1);
+        lj_pair<PERIODIC>(a, b0, b1, addr <= lim0, addr <= lim1, H, I.cold, ax, ay, az);
     }
+    write_row<4>(I.force, (int64_t)sl.row0 + ((hdr >> 24) & 0x3fu), !(hdr >> 31), ax, ay, az, lane);
 }
 
 template <bool PERIODIC, class Src>
@@ -815,130 +803,148 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
 {
     constexpr bool ONE = std::is_same<Src, SrcOne>::value;
     constexpr bool TABLE = std::is_same<Src, SrcTable>::value;
-    extern __shared__ int4 smem_raw[];
-    uint32_t* stage_base = reinterpret_cast<uint32_t*>(smem_raw);
-    __shared__ uint64_t full[kHaloStages];
-    __shared__ uint64_t empty[kHaloStages];
-    __shared__ int s_item[kHaloStages];
-    // per stage: the item's (instance, first row, rows) and its slices' word
-    // offsets within the stage, so that the consumers read no global memory
-    __shared__ int4 s_meta[kHaloStages];
-    __shared__ uint32_t s_soff[kHaloStages][kHaloSlicesPerItem + 1];
-    // per stage: the item's table ids (bulk-copied in whole 16-byte words, so
-    // up to 3 ids before and after them), read by the producer's lanes
-    __shared__ __align__(16) int32_t s_ids[kHaloStages][kHaloTabMax + 8];
-    __shared__ uint64_t idsbar[kHaloStages];
-    __shared__ int s_claim[kHaloStages];  // the next unclaimed slice of the stage's item
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ uint64_t full[kHaloSlots];
+    __shared__ uint64_t empty[kHaloSlots];
+    // per slot: (instance, first row, slices -- 0: no more items, ring offset |
+    // table address << 16), and its slices (byte offset | steps << 16), so
+    // that the consumers read no global memory
+    __shared__ __align__(16) int4 s_meta[kHaloSlots];
+    __shared__ uint32_t s_slice[kHaloSlots][kHaloSlicesPerItem];
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kHaloStages; s++) {
+        for (int s = 0; s < kHaloSlots; s++) {
             mbar_init(&full[s], 33);  // the bulk copy's arrive + one per producer lane
             mbar_init(&empty[s], kConsumerWarps);
-            mbar_init(&idsbar[s], 1);
         }
     }
     __syncthreads();
 
     if (warp == kConsumerWarps) {
         if (withhold) return;
-        // Item k + 1 is prepared while item k's copies are in flight: its
-        // claim, its descriptor, its slices' word offsets (lane j holds the
-        // j-th) and the bulk copy of its table ids into s_ids, so that the
-        // lanes can issue item k + 1's position copies without waiting on
-        // memory once its stage is free.
-        int nxt = 0;
-        WorkItem wn{};
-        uint32_t soff_n = 0;
-        auto prepare = [&](int stage) {
-            nxt = __shfl_sync(0xffffffffu, nxt, 0);
-            if (nxt >= num_items) return;
-            wn = items[nxt];
-            const InstDesc* In;
-            if constexpr (ONE) In = &src.d;
-            else In = insts + wn.inst;
-            const int ns = (wn.nrows + 7) / 8;
-            soff_n = (lane <= ns && lane <= kHaloSlicesPerItem)
-                         ? __ldg(In->slice_off + wn.row0 / 8 + lane) - wn.ent0
-                         : 0u;
-            if (lane == 0) {  // whole 16-byte words around the item's ids
-                const uint32_t a0 = wn.tab0 & ~3u;
-                const uint32_t cnt = ((wn.tab0 & 3u) + wn.ntab + 3u) & ~3u;
-                bulk_load(s_ids[stage], In->tab + a0, cnt * 4u, &idsbar[stage]);
-                if (IRR_HALO_PREFETCH)
-                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(In->words + wn.ent0),
-                                 "r"(wn.nent * 4u)
-                                 : "memory");
-            }
+        // The chain from a claim to an item's positions is four dependent trips
+        // to memory (queue, descriptor, table ids, positions), ~3 us in a row,
+        // nearly as long as the consumers take over an item.  So it is spread
+        // over the iterations before: in iteration k, item k's positions are
+        // copied, item k + 1's table ids (20 to a lane) and slice offsets (lane
+        // j holds the j-th) are read into registers, item k + 2 is claimed and
+        // its descriptor is read.  An index of num_items or more: no more work.
+        auto claim = [&](int last) {
+            if (!queue) return last + (int)gridDim.x;
+            return lane == 0 ? (int)gridDim.x + atomicAdd(queue, 1) : 0;
         };
-        if (lane == 0) nxt = atomicAdd(queue, 1);
-        prepare(0);
+        auto describe = [&](int& it) {
+            if (queue) it = __shfl_sync(0xffffffffu, it, 0);
+            return items[it < num_items ? it : 0];
+        };
+        constexpr int kIds = (kHaloTabMax + 31) / 32;
+        int32_t ids[kIds];
+        uint32_t so = 0;
+        auto fetch = [&](const WorkItem& w) {
+            const InstDesc* I;
+            if constexpr (ONE) I = &src.d;
+            else I = insts + w.inst;
+            const int32_t* __restrict__ tab = I->tab + w.tab0 + lane;
+#pragma unroll
+            for (int j = 0; j < kIds; j++)
+                if (32 * j + lane < (int)w.ntab) ids[j] = __ldg(tab + 32 * j);
+            if (lane <= (w.nrows + 7) / 8) so = __ldg(I->slice_off + w.row0 / 8 + lane) - w.ent0;
+        };
+        int it = (int)blockIdx.x, it1 = claim(it);  // the grid is at most num_items
+        WorkItem w = items[it];
+        fetch(w);
+        WorkItem w1 = describe(it1);
+        const uint32_t ring0 = smem_u32(ring);
+        uint32_t head = 0;   // ring offset after the newest item
+        int live = 0;        // oldest item whose slot is not known to be free
         for (int k = 0;; k++) {
-            const int s = k % kHaloStages;
-            const int use = k / kHaloStages;
-            const int it = nxt < num_items ? nxt : num_items;
-            const WorkItem w = wn;
-            const uint32_t so = soff_n;
-            int ok = 1;
-            if (lane == 0 && use > 0)
-                ok = mbar_wait_policy<IRR_HALO_PWAIT>(&empty[s], (uint32_t)(use - 1) & 1u, wait_ns) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {  // a wait gave up: leave with none of this lane's copies in flight
-                if (lane == 0) atomicOr(status, kStatusWaitTimeout);
-                mbar_wait_backoff<256>(&idsbar[s], (uint32_t)use & 1u, wait_ns);
-                asm volatile("cp.async.wait_all;" ::: "memory");
-                return;
+            const int s = k % kHaloSlots;
+            const bool more = it < num_items;
+            int it2 = claim(it1);
+            // whole 128-byte lines, so that every item starts on one
+            const uint32_t size = more ? (4u * w.nent + 16u * w.ntab + 127u) & ~127u : 0u;
+            // room for the item: a free slot, and `size` bytes after the newest
+            // item or, wrapped, at the ring's start; else the oldest item's end
+            // is waited for
+            for (;;) {
+                if (live == k) {
+                    head = 0;
+                    break;
+                }
+                if (k - live < kHaloSlots) {
+                    const uint32_t tail = ((uint32_t)s_meta[live % kHaloSlots].w & 0xffffu) - ring0;
+                    if (head > tail) {
+                        if (size <= (uint32_t)kHaloRingBytes - head) break;
+                        if (size <= tail) {
+                            head = 0;
+                            break;
+                        }
+                    } else if (size <= tail - head) {
+                        break;
+                    }
+                }
+                int ok = 1;
+                if (lane == 0)
+                    ok = mbar_wait_backoff<kProducerSleep>(&empty[live % kHaloSlots],
+                                                           (uint32_t)(live / kHaloSlots) & 1u, wait_ns)
+                             ? 1
+                             : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) {  // a wait gave up: leave with none of this lane's copies in flight
+                    if (lane == 0) atomicOr(status, kStatusWaitTimeout);
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    return;
+                }
+                live++;
             }
-            if (lane == 0) s_item[s] = it;
-            if (it >= num_items) {  // no more work: complete the stage's phase for the consumers
-                if (lane == 0) mbar_arrive(&full[s]);
+            if (!more) {  // no more work: complete the slot's phase for the consumers
+                if (lane == 0) {
+                    s_meta[s] = make_int4(0, 0, 0, 0);
+                    mbar_arrive(&full[s]);
+                }
                 mbar_arrive(&full[s]);
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 return;
             }
-            if (lane == 0) nxt = atomicAdd(queue, 1);  // item k + 1: the claim is in flight
             const InstDesc* I;
             if constexpr (ONE) I = &src.d;
             else I = insts + w.inst;
-            uint32_t* sw = stage_base + s * kHaloStageWords;
-            // the metadata, written before the stage is published: lane 0's
-            // arrive (release) follows every lane's writes through __syncwarp
+            const uint32_t base = ring0 + head, tab = base + 4u * w.nent;
             const int ns = (w.nrows + 7) / 8;
-            if (lane <= ns && lane <= kHaloSlicesPerItem) s_soff[s][lane] = so;
-            if (lane == 0) {
-                s_meta[s] = make_int4(w.inst, w.row0, w.nrows, 0);
-                s_claim[s] = 0;  // every consumer has left the stage's previous item
-            }
+            // the metadata, written before the item is published: lane 0's
+            // arrive (release) follows every lane's writes through __syncwarp
+            const uint32_t next = __shfl_down_sync(0xffffffffu, so, 1);
+            if (lane < ns) s_slice[s][lane] = 4u * so | ((((next - so) >> 5) - 1u) << 16);
+            if (lane == 0) s_meta[s] = make_int4(w.inst, w.row0, ns, (int)(base | (tab << 16)));
             __syncwarp();
-            if (lane == 0) bulk_load(sw, I->words + w.ent0, w.nent * 4u, &full[s]);
-            // the table: its ids arrived by the bulk copy of the iteration before
-            if (!mbar_wait_backoff<64>(&idsbar[s], (uint32_t)use & 1u, wait_ns)) {
-                if (lane == 0) atomicOr(status, kStatusWaitTimeout);
-                asm volatile("cp.async.wait_all;" ::: "memory");
-                return;  // the consumers' wait for this stage runs out too
-            }
-            const uint32_t tab_u32 = smem_u32(sw + kHaloStreamMax);
-            const int32_t* ids = s_ids[s] + (w.tab0 & 3u);
+            if (lane == 0) bulk_load(ring + head, I->words + w.ent0, w.nent * 4u, &full[s]);
             const float4* __restrict__ pos = I->pos;
-            for (uint32_t j = lane; j < w.ntab; j += 32) cp_async16(tab_u32 + 16u * j, pos + ids[j]);
+#pragma unroll
+            for (int j = 0; j < kIds; j++)
+                if (32 * j + lane < (int)w.ntab) cp_async16(tab + 512u * j + 16u * lane, pos + ids[j]);
             cp_async_arrive(&full[s]);
-            prepare((k + 1) % kHaloStages);
+            head += size;
+            it = it1;
+            w = w1;
+            if (it < num_items) fetch(w);
+            it1 = it2;
+            w1 = describe(it1);
         }
     }
 
     int cur = -1;
     InstHot hot{};
     for (int k = 0;; k++) {
-        const int s = k % kHaloStages;
-        if (!mbar_wait_policy<IRR_HALO_CWAIT>(&full[s], (uint32_t)(k / kHaloStages) & 1u, wait_ns)) {
+        const int s = k % kHaloSlots;
+        if (!mbar_wait_backoff<kConsumerSleep>(&full[s], (uint32_t)(k / kHaloSlots) & 1u, wait_ns)) {
             if (lane == 0) atomicOr(status, kStatusWaitTimeout);
-            mbar_wait_policy<IRR_HALO_CWAIT>(&full[s], (uint32_t)(k / kHaloStages) & 1u, wait_ns);
+            mbar_wait_backoff<kConsumerSleep>(&full[s], (uint32_t)(k / kHaloSlots) & 1u, wait_ns);
             return;
         }
-        const int it = s_item[s];
-        if (it >= num_items) return;
-        const int4 m = s_meta[s];  // instance, first row, rows
+        const int4 m = s_meta[s];
+        if (m.z == 0) return;
         if constexpr (ONE) {
             hot = load_hot(&src.d);
         } else if constexpr (TABLE) {
@@ -947,8 +953,15 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
             hot = load_hot(insts + m.x);
             cur = m.x;
         }
-        consume_halo<PERIODIC>(m.y, m.z, s_soff[s], &s_claim[s], hot, stage_base + s * kHaloStageWords, lane,
-                               IRR_HALO_ROTATE ? (warp + k) % kConsumerWarps : warp);
+        // warp w takes slice (w + k) mod 8 of the CTA's k-th item: slice 0
+        // holds an item's longest rows, so a fixed assignment would always give
+        // one warp the longest slice
+        for (int q = (warp + k) % kConsumerWarps; q < m.z; q += kConsumerWarps) {
+            const uint32_t sl = s_slice[s][q], w = (uint32_t)m.w;
+            halo_slice<PERIODIC>(HaloSlice{(w & 0xffffu) + (sl & 0xffffu) + 4u * (uint32_t)lane, sl >> 16,
+                                           (w >> 16) * 0x10001u, m.y},
+                                 hot);
+        }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
     }
@@ -960,11 +973,10 @@ cudaError_t launch_halo_src(const InstDesc* d_insts, const WorkItem* d_items, in
                             const WaitPolicy& wp)
 {
     auto kern = halo_kernel<PERIODIC, Src>;
-    const size_t smem = (size_t)kHaloStages * kHaloStageWords * sizeof(uint32_t);
-    IRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    IRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kHaloRingBytes));
     if (grid <= 0 || num_items <= 0) return cudaSuccess;
-    kern<<<grid, kPipeThreads, smem, s>>>(d_insts, d_items, num_items, d_queue, d_status,
-                                          wp.wait_ns, wp.withhold, src);
+    kern<<<std::min(grid, num_items), kPipeThreads, kHaloRingBytes, s>>>(d_insts, d_items, num_items, d_queue, d_status,
+                                                    wp.wait_ns, wp.withhold, src);
     return cudaGetLastError();
 }
 
@@ -1067,7 +1079,7 @@ cudaError_t launch_tiled(const TiledShape& shape, const InstDesc* d_insts,
                          int* d_status, cudaStream_t s, const InstDesc* host_insts, int num_insts,
                          const WaitPolicy& wp)
 {
-    if (!d_queue) return cudaErrorInvalidValue;
+    if (!d_queue && !shape.staged) return cudaErrorInvalidValue;
     if (shape.staged) {
         if (shape.lanes_per_row != 4) return cudaErrorInvalidValue;
         return shape.periodic ? launch_halo_p<true>(d_insts, d_items, num_items, d_queue, grid,
