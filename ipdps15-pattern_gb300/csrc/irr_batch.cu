@@ -144,7 +144,6 @@ int upload_items(irr_batch* b, const TiledShape& shape)
 
 int launch_step(irr_batch* b, const TiledShape& shape)
 {
-    B_CUDA(b, cudaMemsetAsync(b->d_queue, 0, sizeof(int), b->stream), "queue");
     B_CUDA(b, launch_tiled(shape, b->d_insts, b->d_items, b->num_items, b->d_queue,
                            b->sms * kCtasPerSm, b->d_status, b->stream, b->host_insts.data(),
                            (int)b->host_insts.size()), "batched kernel");
@@ -261,9 +260,11 @@ int irr_batch_create(int device, irr_batch** out)
     if (!dev_guard.ok() ||
         cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&b->d_queue, sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&b->d_queue, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(int), b->own_stream) != cudaSuccess ||
         cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess ||
-        cudaMemset(b->d_status, 0, sizeof(int)) != cudaSuccess) {
+        cudaMemsetAsync(b->d_status, 0, sizeof(int), b->own_stream) != cudaSuccess ||
+        cudaStreamSynchronize(b->own_stream) != cudaSuccess) {
         cudaGetLastError();
         irr_batch_destroy(b);
         return IRR_ERR_CUDA;

@@ -322,7 +322,6 @@ int launch_reduction(irr_handle* h)
         H_CUDA(h, launch_plain(h->d_pos, h->d_edges, h->e, h->d_force, h->law, h->stream), "plain kernel");
         return IRR_OK;
     }
-    H_CUDA(h, cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream), "clear work queue");
     const WaitPolicy wp = h->wait;
     h->wait.withhold = 0;  // one step only
     H_CUDA(h, launch_tiled(h->shape, h->d_inst, h->d_items, h->num_items, h->d_queue,
@@ -671,8 +670,9 @@ int irr_create(const irr_config* cfg, irr_handle** out)
     if (!dev_guard.ok() ||
         cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess ||
-        cudaMemset(h->d_status, 0, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&h->d_status, 4 * sizeof(int)) != cudaSuccess ||
+        cudaMemsetAsync(h->d_status, 0, 4 * sizeof(int), h->own_stream) != cudaSuccess ||
+        cudaStreamSynchronize(h->own_stream) != cudaSuccess) {
         cudaGetLastError();
         if (h->own_stream) cudaStreamDestroy(h->own_stream);
         if (h->d_status) cudaFree(h->d_status);
@@ -684,13 +684,7 @@ int irr_create(const irr_config* cfg, irr_handle** out)
     h->shape.lanes_per_row = c.lanes_per_row ? c.lanes_per_row : 4;
     h->shape.block_nodes = c.block_nodes ? c.block_nodes : 1024;
     h->shape.stage_smem = c.stage_smem < 0 ? 1 : (c.stage_smem ? 1 : 0);
-    if (cudaMalloc(&h->d_queue, sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaStreamDestroy(h->own_stream);
-        cudaFree(h->d_status);
-        delete h;
-        return IRR_ERR_CUDA;
-    }
+    h->d_queue = h->d_status + 2;
     *out = h;
     return IRR_OK;
 }
@@ -704,7 +698,6 @@ int irr_destroy(irr_handle* h)
     dfree(h->d_raw);
     dfree(h->d_edges);
     dfree(h->d_status);
-    dfree(h->d_queue);
     dfree(h->d_out);
     dfree(h->d_coord);
     free_pipe(h);

@@ -50,8 +50,8 @@ struct irr_handle {
     InstDesc inst{};             // host copy of *d_inst (the single-instance launch parameter)
     WorkItem* d_items = nullptr;
     int num_items = 0;
-    int* d_status = nullptr;
-    int* d_queue = nullptr;      // work-queue cursor, cleared before each launch
+    int* d_status = nullptr;     // [0] status word, [2, 3] the work queue
+    int* d_queue = nullptr;      // d_status + 2 (each launch leaves it cleared)
     irr::WaitPolicy wait{};      // device-side wait limit; withhold: the next step only
     void* d_out = nullptr;       // result staging for host reads
     size_t out_cap = 0;

@@ -58,6 +58,7 @@ __global__ void kick_drift_kernel(double* __restrict__ x, double* __restrict__ v
                                   const float4* __restrict__ f, int64_t n, double dt, double L,
                                   float4* __restrict__ pos4)
 {
+    grid_begin();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         md_kick_drift_atom<KICKS>(x, v, f, i, dt, L, pos4);
@@ -393,7 +394,6 @@ int md_forces(irr_md* m)
         MD_CUDA(m, launch_plain(m->pos4, m->half, m->edges, m->force, m->law, m->stream), "plain kernel");
         return IRR_OK;
     }
-    MD_CUDA(m, cudaMemsetAsync(m->d_queue, 0, sizeof(int), m->stream), "queue");
     MD_CUDA(m, launch_tiled(m->shape, m->d_inst, m->d_items, m->num_items, m->d_queue,
                             m->sms * kCtasPerSm, m->d_status, m->stream, &m->inst, 1), "force kernel");
     return IRR_OK;
@@ -401,9 +401,8 @@ int md_forces(irr_md* m)
 
 int md_kick_drift(irr_md* m)
 {
-    kick_drift_kernel<1><<<grid_of(m->n), 256, 0, m->stream>>>(m->x, m->v, m->force, m->n,
-                                                               m->cfg.dt, m->cfg.side, m->pos4);
-    MD_CUDA(m, cudaGetLastError(), "kick-drift");
+    MD_CUDA(m, launch_chained(kick_drift_kernel<1>, grid_of(m->n), 256, 0, m->stream, m->x, m->v, m->force,
+                              m->n, m->cfg.dt, m->cfg.side, m->pos4), "kick-drift");
     m->since_rebuild++;
     return IRR_OK;
 }
@@ -411,9 +410,8 @@ int md_kick_drift(irr_md* m)
 // md_kick of the previous step and md_kick_drift of this one in one pass.
 int md_kick_kick_drift(irr_md* m)
 {
-    kick_drift_kernel<2><<<grid_of(m->n), 256, 0, m->stream>>>(m->x, m->v, m->force, m->n,
-                                                               m->cfg.dt, m->cfg.side, m->pos4);
-    MD_CUDA(m, cudaGetLastError(), "kick-drift");
+    MD_CUDA(m, launch_chained(kick_drift_kernel<2>, grid_of(m->n), 256, 0, m->stream, m->x, m->v, m->force,
+                              m->n, m->cfg.dt, m->cfg.side, m->pos4), "kick-drift");
     m->steps++;
     m->since_rebuild++;
     return IRR_OK;
@@ -530,10 +528,11 @@ int irr_md_create(const irr_md_config* cfg, const double* pos, const double* vel
     if (e == cudaSuccess) e = irr_malloc_async(&m->ids, sizeof(int32_t) * n, os);
     if (e == cudaSuccess) e = irr_malloc_async(&m->ids_tmp, sizeof(int32_t) * n, os);
     if (e == cudaSuccess) e = irr_malloc_async(&m->d_inst, sizeof(InstDesc), os);
-    if (e == cudaSuccess) e = irr_malloc_async(&m->d_queue, sizeof(int), os);
+    if (e == cudaSuccess) e = irr_malloc_async(&m->d_queue, 2 * sizeof(int), os);
     if (e == cudaSuccess) e = irr_malloc_async(&m->d_status, sizeof(int), os);
     if (e == cudaSuccess) e = irr_malloc_async(&m->d_acc, (4 + 3 * kEnergyBlocks) * sizeof(double), os);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->d_status, 0, sizeof(int), m->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->d_queue, 0, 2 * sizeof(int), m->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(m->x, pos, b3, cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(m->v, vel, b3, cudaMemcpyHostToDevice, m->stream);
     if (e != cudaSuccess) {

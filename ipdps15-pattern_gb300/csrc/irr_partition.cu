@@ -453,6 +453,7 @@ __global__ void fill_rows_kernel(const int2* edges, int64_t e, const int32_t* in
 __global__ void load_nodes_kernel(const char* raw, int elm, const int32_t* perm, int64_t n,
                                   float4* dst)
 {
+    grid_begin();
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
          k += (int64_t)gridDim.x * blockDim.x) {
         const int64_t src = perm ? perm[k] : k;
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(kMoveThreads) load_nodes_scatter_kernel(
     float4* __restrict__ dst)
 {
     __shared__ float4 tile[3 * kMoveThreads];
+    grid_begin();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t head = 0;  // records moved in whole tiles
     if (vec12) {
@@ -530,6 +532,7 @@ __global__ void __launch_bounds__(kMoveThreads) store_result_kernel(
     const float4* force, const int32_t* inv, int64_t n, int elm, int vec12, char* out)
 {
     __shared__ float4 tile[3 * kMoveThreads];
+    grid_begin();
     int64_t head = 0;
     if (vec12) {
         constexpr int64_t kTile = 4 * kMoveThreads;
@@ -996,9 +999,8 @@ cudaError_t launch_load_nodes(const void* raw, int elm_size, const int32_t* perm
                               float4* dst, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    load_nodes_kernel<<<grid_for(n), 256, 0, s>>>(static_cast<const char*>(raw), elm_size, perm, n,
-                                                  dst);
-    return cudaGetLastError();
+    return launch_chained(load_nodes_kernel, grid_for(n), 256, 0, s, static_cast<const char*>(raw), elm_size, perm,
+                          n, dst);
 }
 
 cudaError_t launch_store_result(const float4* force, const int32_t* inv, int64_t n,
@@ -1006,9 +1008,8 @@ cudaError_t launch_store_result(const float4* force, const int32_t* inv, int64_t
 {
     if (n <= 0) return cudaSuccess;
     const int vec12 = elm_size == 12 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-    store_result_kernel<<<grid_for(n, kMoveThreads), kMoveThreads, 0, s>>>(force, inv, n, elm_size,
-                                                                          vec12, static_cast<char*>(out));
-    return cudaGetLastError();
+    return launch_chained(store_result_kernel, grid_for(n, kMoveThreads), kMoveThreads, 0, s, force, inv, n, elm_size,
+                          vec12, static_cast<char*>(out));
 }
 
 cudaError_t launch_load_nodes_scatter(const void* rec, int elm_size, const int32_t* inv, int64_t n,
@@ -1016,9 +1017,8 @@ cudaError_t launch_load_nodes_scatter(const void* rec, int elm_size, const int32
 {
     if (n <= 0) return cudaSuccess;
     const int vec12 = elm_size == 12 && (reinterpret_cast<uintptr_t>(rec) & 15u) == 0;
-    load_nodes_scatter_kernel<<<grid_for(n, kMoveThreads), kMoveThreads, 0, s>>>(
-        static_cast<const char*>(rec), elm_size, vec12, inv, n, dst);
-    return cudaGetLastError();
+    return launch_chained(load_nodes_scatter_kernel, grid_for(n, kMoveThreads), kMoveThreads, 0, s,
+                          static_cast<const char*>(rec), elm_size, vec12, inv, n, dst);
 }
 
 void* host_device_view(const void* p)

@@ -29,6 +29,7 @@
 //   ordered rows whose columns ascend, the lanes of one gather also land on
 //   few cache lines.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 #include <vector>
 
@@ -441,13 +442,6 @@ __device__ __forceinline__ void row_sum(const float4* __restrict__ pos, const in
 }
 
 constexpr int kConsumerWarps = kConsumerSlices;
-// Items per queue claim (a run of consecutive node blocks on one SM shares
-// neighbourhood positions in its L1, but runs of 2, 4 and 8 measured slower
-// than single items on the 4M-node workload: load balance wins).
-#ifndef IRR_CLAIM_CHUNK
-#define IRR_CLAIM_CHUNK 1
-#endif
-constexpr int kClaimChunk = IRR_CLAIM_CHUNK;
 constexpr int kPipeThreads = (kConsumerWarps + 1) * 32;
 
 // The rows of one work item that belong to consumer warp `cw`.
@@ -558,10 +552,22 @@ __device__ __forceinline__ void consume_sliced(const WorkItem& w, const InstHot&
     }
 }
 
+// A CTA leaves the queue (one thread of its producer warp, after its last
+// claim): the last one to leave clears it for the next launch, so that a step
+// needs no clearing launch of its own (3.3 us a step at 864 nodes).
+__device__ __forceinline__ void leave_queue(int* queue)
+{
+    __threadfence();
+    if (atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
+        queue[0] = 0;
+        queue[1] = 0;
+    }
+}
+
 // Persistent owner-computes kernel, warp-specialised.  Warp kConsumerWarps is
-// the producer: its lane 0 claims runs of kClaimChunk consecutive work items
-// from *queue, and for each item waits until its ring stage is empty,
-// publishes the item id and
+// the producer: its lane 0 claims work items from the queue (the next one's
+// index and descriptor are read while it waits), and for each item waits until
+// its ring stage is empty, publishes the item and
 // either bulk-copies the item's entry segment (widened to 16-byte bounds)
 // into the stage -- the stage's `full` mbarrier completes on the byte count --
 // or, for items read from global memory, just arrives.  The consumer warps
@@ -575,6 +581,7 @@ __device__ __forceinline__ void consume_sliced(const WorkItem& w, const InstHot&
 // runs out and the launch ends with kStatusWaitTimeout and nothing in flight.
 //
 // Src (SrcGlobal, SrcOne, SrcTable): where the instance fields come from.
+enum : int { kStageEnd = 0, kStageGlobal = 1, kStageShared = 2 };
 template <bool PERIODIC, int G, class Src>
 __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) tiled_kernel(
     const InstDesc* __restrict__ insts, const WorkItem* __restrict__ items, int num_items,
@@ -588,8 +595,8 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) tiled_kernel(
     constexpr int kStageInts = kStageEntries + kColPad;
     __shared__ uint64_t full[kStages];
     __shared__ uint64_t empty[kStages];
-    __shared__ int s_item[kStages];
-    __shared__ int s_smem[kStages];
+    __shared__ WorkItem s_work[kStages];
+    __shared__ int s_mode[kStages];
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
 
@@ -600,45 +607,52 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) tiled_kernel(
         }
     }
     __syncthreads();
+    grid_wait();
 
     if (warp == kConsumerWarps) {
-        if (lane != 0 || withhold) return;
-        int next_item = 0, chunk_left = 0;
+        if (lane != 0) return;
+        if (withhold) {
+            leave_queue(queue);
+            return;
+        }
+        int it = (int)blockIdx.x;  // the grid is at most num_items
+        WorkItem w = items[it];
+        int it1 = (int)gridDim.x + atomicAdd(queue, 1);
         for (int k = 0;; k++) {
             const int s = k % kStages;
             const int use = k / kStages;
+            // the next item's descriptor and the claim after it are in flight
+            // while this item waits for its stage
+            const WorkItem w1 = items[it1 < num_items ? it1 : 0];
+            const int it2 = it1 < num_items ? (int)gridDim.x + atomicAdd(queue, 1) : it1;
             if (use > 0 && !mbar_wait_bounded(&empty[s], (uint32_t)(use - 1) & 1u, wait_ns)) {
                 atomicOr(status, kStatusWaitTimeout);
+                leave_queue(queue);
                 return;  // nothing of this stage is in flight: its last copy was consumed
             }
-            if (chunk_left == 0) {  // a run of kClaimChunk consecutive items
-                const long long first = (long long)atomicAdd(queue, 1) * kClaimChunk;
-                next_item = first < num_items ? (int)first : num_items;
-                chunk_left = kClaimChunk;
+            if (it >= num_items) {
+                s_mode[s] = kStageEnd;
+                mbar_arrive(&full[s]);
+                leave_queue(queue);
+                return;
             }
-            const int it = next_item++;
-            chunk_left--;
-            s_item[s] = it;
-            bool issue = false;
-            if (it < num_items && use_stages) {
-                const WorkItem w = items[it];
-                issue = !(w.flags & kItemDirect);
-                if (issue) {
-                    s_smem[s] = 1;
-                    const uint32_t a0 = w.ent0 & ~3u;
-                    const uint32_t words = ((w.ent0 + w.nent - a0) + 3u) & ~3u;
-                    const InstDesc* I;
-                    if constexpr (ONE) I = &src.d;
-                    else I = insts + w.inst;
-                    const int32_t* ent = (w.flags & kItemSliced) ? I->scol : I->col;
-                    bulk_load(stage_base + s * kStageInts, ent + a0, words * 4u, &full[s]);
-                }
-            }
-            if (!issue) {
-                s_smem[s] = 0;
+            s_work[s] = w;
+            if (use_stages && !(w.flags & kItemDirect)) {
+                s_mode[s] = kStageShared;
+                const uint32_t a0 = w.ent0 & ~3u;
+                const uint32_t words = ((w.ent0 + w.nent - a0) + 3u) & ~3u;
+                const InstDesc* I;
+                if constexpr (ONE) I = &src.d;
+                else I = insts + w.inst;
+                const int32_t* ent = (w.flags & kItemSliced) ? I->scol : I->col;
+                bulk_load(stage_base + s * kStageInts, ent + a0, words * 4u, &full[s]);
+            } else {
+                s_mode[s] = kStageGlobal;
                 mbar_arrive(&full[s]);
             }
-            if (it >= num_items) return;
+            it = it1;
+            w = w1;
+            it1 = it2;
         }
     }
 
@@ -651,9 +665,9 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) tiled_kernel(
             mbar_wait_bounded(&full[s], (uint32_t)(k / kStages) & 1u, wait_ns);
             return;
         }
-        const int it = s_item[s];
-        if (it >= num_items) return;
-        const WorkItem w = items[it];
+        const int mode = s_mode[s];
+        if (mode == kStageEnd) return;
+        const WorkItem w = s_work[s];
         const InstDesc* I;
         if constexpr (ONE) {
             I = &src.d;
@@ -669,12 +683,12 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) tiled_kernel(
             }
         }
         if (w.flags & kItemSliced) {
-            if (s_smem[s])
+            if (mode == kStageShared)
                 consume_sliced<PERIODIC, G, true>(w, hot, stage_base + s * kStageInts, w.ent0, warp,
                                                   lane);
             else
                 consume_sliced<PERIODIC, G, false>(w, hot, I->scol, 0u, warp, lane);
-        } else if (s_smem[s]) {
+        } else if (mode == kStageShared) {
             consume_item<PERIODIC, G>(w, hot, stage_base + s * kStageInts, w.ent0 & ~3u, warp, lane);
         } else {
             consume_item<PERIODIC, G>(w, hot, I->col, 0u, warp, lane);
@@ -821,9 +835,13 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
         }
     }
     __syncthreads();
+    grid_wait();
 
     if (warp == kConsumerWarps) {
-        if (withhold) return;
+        if (withhold) {
+            if (queue && lane == 0) leave_queue(queue);
+            return;
+        }
         // The chain from a claim to an item's positions is four dependent trips
         // to memory (queue, descriptor, table ids, positions), ~3 us in a row,
         // nearly as long as the consumers take over an item.  So it is spread
@@ -893,7 +911,10 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
                              : 0;
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) {  // a wait gave up: leave with none of this lane's copies in flight
-                    if (lane == 0) atomicOr(status, kStatusWaitTimeout);
+                    if (lane == 0) {
+                        atomicOr(status, kStatusWaitTimeout);
+                        if (queue) leave_queue(queue);
+                    }
                     asm volatile("cp.async.wait_all;" ::: "memory");
                     return;
                 }
@@ -903,6 +924,7 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
                 if (lane == 0) {
                     s_meta[s] = make_int4(0, 0, 0, 0);
                     mbar_arrive(&full[s]);
+                    if (queue) leave_queue(queue);
                 }
                 mbar_arrive(&full[s]);
                 asm volatile("cp.async.wait_all;" ::: "memory");
@@ -967,17 +989,41 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
     }
 }
 
+// A kernel's shared-memory limit, set once per device (2 us a call).
+class DeviceOnce {
+public:
+    cudaError_t max_shared(const void* kern, int bytes)
+    {
+        int dev = 0;
+        IRR_CUDA_TRY(cudaGetDevice(&dev));
+        const bool known = dev >= 0 && dev < 64;
+        const uint64_t bit = known ? 1ull << dev : 0;
+        if (done_.load(std::memory_order_acquire) & bit) return cudaSuccess;
+        IRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        done_.fetch_or(bit, std::memory_order_release);
+        return cudaSuccess;
+    }
+
+private:
+    std::atomic<uint64_t> done_{0};
+};
+
 template <bool PERIODIC, class Src>
 cudaError_t launch_halo_src(const InstDesc* d_insts, const WorkItem* d_items, int num_items,
                             int* d_queue, int grid, int* d_status, cudaStream_t s, const Src& src,
                             const WaitPolicy& wp)
 {
     auto kern = halo_kernel<PERIODIC, Src>;
-    IRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kHaloRingBytes));
+    static DeviceOnce once;
+    IRR_CUDA_TRY(once.max_shared(reinterpret_cast<const void*>(kern), kHaloRingBytes));
     if (grid <= 0 || num_items <= 0) return cudaSuccess;
-    kern<<<std::min(grid, num_items), kPipeThreads, kHaloRingBytes, s>>>(d_insts, d_items, num_items, d_queue, d_status,
-                                                    wp.wait_ns, wp.withhold, src);
-    return cudaGetLastError();
+    // claims run two items ahead of a CTA's positions, which with a few items
+    // per CTA leaves some with three and others with one: up to 4 items per CTA
+    // they are dealt out in turn (65,536 nodes, 1.7 items per CTA: 10.0 -> 8.7
+    // us; 4M nodes, 108 per CTA, dealt out: 386 -> 429)
+    int* const queue = num_items <= 4 * grid ? nullptr : d_queue;
+    return launch_chained(kern, (unsigned)std::min(grid, num_items), kPipeThreads, kHaloRingBytes, s, d_insts,
+                          d_items, num_items, queue, d_status, wp.wait_ns, wp.withhold, src);
 }
 
 template <bool PERIODIC>
@@ -1009,13 +1055,11 @@ cudaError_t launch_tiled_src(const TiledShape& shape, const InstDesc* d_insts,
     auto kern = tiled_kernel<PERIODIC, G, Src>;
     const size_t smem =
         shape.stage_smem ? (size_t)kStages * (kStageEntries + kColPad) * sizeof(int32_t) : 0;
-    if (smem > 48 * 1024)
-        IRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    static DeviceOnce once;
+    if (smem > 48 * 1024) IRR_CUDA_TRY(once.max_shared(reinterpret_cast<const void*>(kern), (int)smem));
     if (grid <= 0 || num_items <= 0) return cudaSuccess;
-    kern<<<grid, kPipeThreads, smem, s>>>(d_insts, d_items, num_items, d_queue, d_status,
-                                          shape.stage_smem, wp.wait_ns, wp.withhold, src);
-    return cudaGetLastError();
+    return launch_chained(kern, (unsigned)std::min(grid, num_items), kPipeThreads, smem, s, d_insts, d_items,
+                          num_items, d_queue, d_status, shape.stage_smem, wp.wait_ns, wp.withhold, src);
 }
 
 template <bool PERIODIC, int G>
@@ -1079,7 +1123,7 @@ cudaError_t launch_tiled(const TiledShape& shape, const InstDesc* d_insts,
                          int* d_status, cudaStream_t s, const InstDesc* host_insts, int num_insts,
                          const WaitPolicy& wp)
 {
-    if (!d_queue && !shape.staged) return cudaErrorInvalidValue;
+    if (!d_queue) return cudaErrorInvalidValue;
     if (shape.staged) {
         if (shape.lanes_per_row != 4) return cudaErrorInvalidValue;
         return shape.periodic ? launch_halo_p<true>(d_insts, d_items, num_items, d_queue, grid,

@@ -285,7 +285,7 @@ int force_and_kick(const std::vector<irr_md*>& ms, const std::vector<irr_md*>& r
             tick_items_kernel<<<(unsigned)(want < 4096 ? want : 4096), 256, 0, s>>>(B.jobs.d, (int)ms.size(),
                                                                                     nitems, B.d_items);
         }
-        if (cudaGetLastError() != cudaSuccess || cudaMemsetAsync(d_queue, 0, sizeof(int), s) != cudaSuccess ||
+        if (cudaGetLastError() != cudaSuccess ||
             launch_tiled(shape, B.insts.d, B.d_items, (int)nitems, d_queue, sms * kCtasPerSm, d_status, s,
                          B.insts.h, (int)ms.size()) != cudaSuccess)
             return IRR_ERR_CUDA;
@@ -495,8 +495,10 @@ int irr_serve_run(const irr_serve_config* cfg, irr_serve_stats* st, irr_serve_jo
     int *d_queue = nullptr, *d_status = nullptr;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&d_queue, sizeof(int)) != cudaSuccess || cudaMalloc(&d_status, sizeof(int)) != cudaSuccess ||
-        cudaMemset(d_status, 0, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&d_queue, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&d_status, sizeof(int)) != cudaSuccess ||
+        cudaMemsetAsync(d_queue, 0, 2 * sizeof(int), s) != cudaSuccess ||
+        cudaMemsetAsync(d_status, 0, sizeof(int), s) != cudaSuccess) {
         cudaGetLastError();
         return IRR_ERR_CUDA;
     }
