@@ -86,6 +86,21 @@ void free_layout(irr_handle* h)
     h->inited = false;
 }
 
+// Whether the load kernels can read records of elm bytes at p in place: memory
+// the device addresses as its own, at the alignment their loads want.  Other
+// pointers go through the staging copy, whose checks are the runtime's.
+bool device_records(const void* p, int elm)
+{
+    const uintptr_t align = elm == 12 ? 4 : (elm == 16 ? 16 : 8);
+    if (reinterpret_cast<uintptr_t>(p) % align) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) && a.devicePointer == p;
+}
+
 // Node records: positions (12/16/24 bytes) for the built-in laws; any
 // multiple of 4 bytes up to 1024 for a user map.
 bool valid_node_elm(const irr_handle* h, int elm)
@@ -235,6 +250,16 @@ int set_nodes_common(irr_handle* h, const void* src, int elm, int64_t n, cudaMem
             h->raw_pending = false;
             return IRR_OK;
         }
+    }
+    if (kind == cudaMemcpyDeviceToDevice && h->inited && n > 0 && !h->user_launch && device_records(src, elm)) {
+        // device records straight into execution order, without the staging
+        // copy (14 us of 446 at 4M nodes, 2.8 of 16.5 at 65,536).  Gathered by
+        // the execution order; read in order and scattered, as host records
+        // are, costs 68 instead of 39 us at 4M nodes.
+        H_CUDA(h, launch_load_nodes(src, elm, h->part.perm, n, h->d_pos, h->stream), "load node data");
+        h->raw_elm = elm;
+        h->raw_pending = false;
+        return IRR_OK;
     }
     int rc = ensure_raw(h, (size_t)(n > 0 ? n : 1) * (size_t)elm);
     if (rc) return rc;
