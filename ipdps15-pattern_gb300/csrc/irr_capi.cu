@@ -343,8 +343,7 @@ void result_rows(const irr_handle* h, int64_t* lo, int64_t* count)
 int launch_reduction(irr_handle* h)
 {
     if (h->cfg.exec == IRR_EXEC_PLAIN) {
-        H_CUDA(h, cudaMemsetAsync(h->d_force, 0, (size_t)(h->n > 0 ? h->n : 1) * sizeof(float4), h->stream), "clear results");
-        H_CUDA(h, launch_plain(h->d_pos, h->d_edges, h->e, h->d_force, h->law, h->stream), "plain kernel");
+        H_CUDA(h, launch_plain(h->d_pos, h->d_edges, h->e, h->d_force, h->n, h->law, h->sms, h->stream), "plain kernel");
         return IRR_OK;
     }
     const WaitPolicy wp = h->wait;

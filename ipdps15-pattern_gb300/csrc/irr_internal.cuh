@@ -260,8 +260,9 @@ struct WaitPolicy {
 };
 
 // -- reduction kernels (irr_reduce.cu) --
-cudaError_t launch_plain(const float4* pos, const int2* edges, int64_t e, float4* force,
-                         const LawParams& law, cudaStream_t s);
+// Clears the n results and adds every edge's contributions.
+cudaError_t launch_plain(const float4* pos, const int2* edges, int64_t e, float4* force, int64_t n,
+                         const LawParams& law, int sms, cudaStream_t s);
 // A persistent grid of `grid` CTAs takes items from the queue d_queue[0]
 // (d_queue[0, 1]: 0 at the first launch; each launch leaves them 0 again), CTA
 // b's first item being b.  host_insts (a host copy of the num_insts descriptors of

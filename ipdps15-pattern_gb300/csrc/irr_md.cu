@@ -390,8 +390,7 @@ int md_rebuild(irr_md* m)
 int md_forces(irr_md* m)
 {
     if (m->cfg.exec_plain) {
-        MD_CUDA(m, cudaMemsetAsync(m->force, 0, sizeof(float4) * m->n, m->stream), "clear forces");
-        MD_CUDA(m, launch_plain(m->pos4, m->half, m->edges, m->force, m->law, m->stream), "plain kernel");
+        MD_CUDA(m, launch_plain(m->pos4, m->half, m->edges, m->force, m->n, m->law, m->sms, m->stream), "plain kernel");
         return IRR_OK;
     }
     MD_CUDA(m, launch_tiled(m->shape, m->d_inst, m->d_items, m->num_items, m->d_queue,
