@@ -121,13 +121,17 @@ int upload_items(irr_batch* b, const TiledShape& shape)
 {
     std::vector<WorkItem> items;
     for (size_t k = 0; k < b->handles.size(); k++) {
-        const irr_handle* h = b->handles[k];
+        irr_handle* h = b->handles[k];
         if (shape.staged) {
-            for (WorkItem w : h->st.items) {
+            std::vector<WorkItem> own;
+            B_CUDA(b, staged_items_to_host(h->d_items, h->num_items, &own, h->stream), "work items");
+            for (WorkItem w : own) {
                 w.inst = (int32_t)k;
                 items.push_back(w);
             }
         } else {
+            const int rc = irr_host_row_off(h);
+            if (rc) return bfail(b, rc, std::string("row offsets: ") + irr_last_error(h));
             make_instance_items(h->host_row_off.data(), h->sl, h->n, (int)k, shape, items);
         }
     }

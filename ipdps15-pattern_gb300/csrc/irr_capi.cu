@@ -185,11 +185,19 @@ int upload_inst(irr_handle* h)
 
 int upload_items(irr_handle* h)
 {
+    if (h->shape.staged) {  // built on the device with the layout (kept while the layout is)
+        if (h->st.items) {
+            dfree(h->d_items);
+            h->d_items = h->st.items;
+            h->st.items = nullptr;
+        }
+        h->num_items = (int)h->st.nitems;
+        return IRR_OK;
+    }
     std::vector<WorkItem> items;
-    if (h->shape.staged)
-        items = h->st.items;
-    else
-        make_instance_items(h->host_row_off.data(), h->sl, h->n, 0, h->shape, items);
+    int rc = irr_host_row_off(h);
+    if (rc) return rc;
+    make_instance_items(h->host_row_off.data(), h->sl, h->n, 0, h->shape, items);
     dfree(h->d_items);
     h->num_items = 0;
     H_CUDA(h, cudaMalloc(&h->d_items, sizeof(WorkItem) * (items.size() ? items.size() : 1)), "allocate work items");
@@ -513,6 +521,17 @@ bool user_result_ok(const irr_handle* h, int elm_size)
 
 }  // namespace
 
+int irr_host_row_off(irr_handle* h)
+{
+    if (!h->host_row_off.empty()) return IRR_OK;
+    std::vector<uint32_t> off((size_t)h->n + 1);
+    H_CUDA(h, cudaMemcpyAsync(off.data(), h->part.row_off, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost,
+                              h->stream), "copy row offsets");
+    H_CUDA(h, cudaStreamSynchronize(h->stream), "copy row offsets");
+    h->host_row_off.swap(off);
+    return IRR_OK;
+}
+
 int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int staged_ok)
 {
     TraceRange trace_("irr_layout");
@@ -530,8 +549,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     if (want == IRR_LAYOUT_STAGED || (want == IRR_LAYOUT_AUTO && kAutoStaged && staged_ok)) {
         if (lanes_per_row == 4 && h->shape.stage_smem) {
             if (!h->st.words) {
-                const cudaError_t se = build_staged(h->part.row_off, h->part.col, h->host_row_off.data(),
-                                                    n, &h->st, h->stream);
+                cudaError_t se = build_staged(h->part.row_off, h->part.col, n, false, &h->st, h->stream);
                 if (se != cudaSuccess) {
                     cudaGetLastError();
                     free_staged(&h->st);
@@ -550,7 +568,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
             return fail(h, IRR_ERR_ARG, "the staged layout needs 4 lanes per row and stage_smem");
         }
     }
-    h->shape.staged = staged ? 1 : 0;
+    h->shape.staged = staged ? (h->st.wide ? 2 : 1) : 0;
     if (staged) {
         free_sliced(&h->sl);
     } else {
@@ -882,11 +900,6 @@ int irr_init(irr_handle* h)
     }
     H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, h->part.perm, n, h->d_pos, s), "gather node data");
     h->raw_pending = false;
-    // node blocks -> work items (cut on the row offsets)
-    h->host_row_off.resize((size_t)n + 1);
-    H_CUDA(h, cudaMemcpyAsync(h->host_row_off.data(), h->part.row_off, sizeof(uint32_t) * (n + 1),
-                              cudaMemcpyDeviceToHost, s), "copy row offsets");
-    H_CUDA(h, cudaStreamSynchronize(s), "copy row offsets");
     H_CUDA(h, cudaMalloc(&h->d_inst, sizeof(InstDesc)), "allocate instance descriptor");
     h->shape.periodic = h->law.periodic;
     h->inited = true;
@@ -1099,19 +1112,23 @@ int irr_get_staged(irr_handle* h, int64_t* counts, int32_t* items, uint32_t* sli
     DeviceGuard dev_guard(h->device);
     const Staged& st = h->st;
     if (counts) {
-        counts[0] = (int64_t)st.items.size();
+        counts[0] = st.nitems;
         counts[1] = st.nwords;
         counts[2] = st.nids;
     }
-    if (items)
-        for (size_t k = 0; k < st.items.size(); k++) {
-            const WorkItem& w = st.items[k];
+    if (items) {
+        std::vector<WorkItem> host;
+        H_CUDA(h, staged_items_to_host(h->d_items, st.nitems, &host, h->stream), "copy work items");
+        for (size_t k = 0; k < host.size(); k++) {
+            const WorkItem& w = host[k];
             const int32_t v[6] = {w.row0, w.nrows, (int32_t)w.ent0, (int32_t)w.nent, (int32_t)w.tab0,
                                   (int32_t)w.ntab};
             memcpy(items + 6 * k, v, sizeof(v));
         }
-    if (slice_off && !st.host_off.empty())
-        memcpy(slice_off, st.host_off.data(), sizeof(uint32_t) * st.host_off.size());
+    }
+    if (slice_off && st.slice_off)
+        H_CUDA(h, cudaMemcpyAsync(slice_off, st.slice_off, sizeof(uint32_t) * (st.slices + 1), cudaMemcpyDeviceToHost,
+                                  h->stream), "copy slice offsets");
     if (words && st.nwords > 0)
         H_CUDA(h, cudaMemcpyAsync(words, st.words, sizeof(uint32_t) * st.nwords, cudaMemcpyDeviceToHost, h->stream), "copy words");
     if (ids && st.nids > 0)

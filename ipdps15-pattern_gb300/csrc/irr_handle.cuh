@@ -43,7 +43,7 @@ struct irr_handle {
     float4* d_pos = nullptr;     // execution order
     float4* d_force = nullptr;
     PartitionOut part{};
-    std::vector<uint32_t> host_row_off;  // host copy of part.row_off (cuts work items)
+    std::vector<uint32_t> host_row_off;  // host copy of part.row_off (irr_host_row_off)
     irr::Sliced sl{};                    // sliced layout, when in use
     irr::Staged st{};                    // staged layout, when in use
     InstDesc* d_inst = nullptr;
@@ -97,4 +97,7 @@ struct irr_handle {
 // that the three always agree.  staged_ok = 0 keeps an AUTO handle off the
 // staged layout (a handle configured IRR_LAYOUT_STAGED then fails with
 // IRR_ERR_STATE).  Partitioned, initialised handles only.
+// Brings the row offsets to the host, where CSR and sliced work items are cut
+// from them (once per partition; the staged layout needs none).
+int irr_host_row_off(irr_handle* h);
 int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int staged_ok = 1);

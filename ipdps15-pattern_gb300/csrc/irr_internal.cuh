@@ -141,7 +141,7 @@ struct TiledShape {
     int stage_smem;      // 1: entry segments bulk-copied into a shared-memory ring
     int block_nodes;     // max rows per work item
     int periodic;
-    int staged = 0;      // 1: staged layout (the halo kernel; 4 lanes per row)
+    int staged = 0;      // 1: staged layout (the halo kernel; 4 lanes per row), 2: to the wide limits
 };
 
 // Staged ("halo") layout of one instance, for 4 lanes per row and slices of 8
@@ -166,20 +166,28 @@ struct Staged {
     uint32_t* slice_off = nullptr;   // [slices + 1] word offsets (multiples of 32)
     uint32_t* words = nullptr;       // [nwords]
     int32_t* ids = nullptr;          // [nids] the items' tables, concatenated
+    WorkItem* items = nullptr;       // [nitems] (instance 0), flags kItemStaged; taken over by the handle
     int64_t slices = 0;
     int64_t nwords = 0;
     int64_t nids = 0;
-    std::vector<uint32_t> host_off;  // host copy of slice_off
-    std::vector<WorkItem> items;     // the items (instance 0), flags kItemStaged
+    int64_t nitems = 0;
+    bool wide = false;               // built to the wide limits
 };
+// The wide limits, for rows that touch more nodes: an item takes up to the
+// whole ring of the halo kernel, whose other CTAs on the SM compute while one
+// loads.
+constexpr int kHaloWideTabMax = 1008;
+constexpr int kHaloWideStreamMax = 9984;
 // Builds st from a CSR (rows in execution order, columns ascending) on the
-// device; host_row_off is the host copy of row_off.  Synchronises s.
-// cudaErrorNotSupported (nothing allocated) when a slice alone exceeds the
-// limits above -- a row of more than ~440 entries, or 8 rows touching more
-// than kHaloTabMax distinct nodes.
-cudaError_t build_staged(const uint32_t* row_off, const int32_t* col, const uint32_t* host_row_off,
-                         int64_t n, Staged* st, cudaStream_t s);
+// device.  Synchronises s.  cudaErrorNotSupported (nothing allocated) when a
+// slice alone exceeds the limits above -- a row of more than ~440 entries
+// (wide: 1023), or 8 rows touching more than kHaloTabMax (wide:
+// kHaloWideTabMax) distinct nodes.
+cudaError_t build_staged(const uint32_t* row_off, const int32_t* col, int64_t n, bool wide, Staged* st,
+                         cudaStream_t s);
 void free_staged(Staged* st, cudaStream_t s = nullptr);
+// Items copied to the host; synchronises s.
+cudaError_t staged_items_to_host(const WorkItem* d_items, int64_t count, std::vector<WorkItem>* items, cudaStream_t s);
 
 // Shape of the owner-computes kernel; each can be set at build time
 // (-DIRR_STAGES=... etc.) to build and time variants.
