@@ -104,14 +104,19 @@ int upload_insts(irr_batch* b)
 // Every instance's layout for G lanes per row, staged or not (each handle
 // rebuilds its own descriptor and items with it), then the batch's instance
 // table.  IRR_ERR_CAPACITY (no failure recorded) when the staged layout was
-// asked for and some instance's graph does not fit it.
-int set_lanes(irr_batch* b, int lanes, int staged)
+// asked for and some instance's graph does not fit it, or fits other limits
+// than the others' (one launch runs one kernel).  staged: in 0 or 1, out the
+// TiledShape value the instances have.
+int set_lanes(irr_batch* b, int lanes, int& staged)
 {
     for (irr_handle* h : b->handles) {
-        if (h->shape.lanes_per_row == lanes && h->shape.staged == staged) continue;  // already laid out
-        const int rc = irr_ensure_layout(h, lanes, h->shape.block_nodes, staged);
-        if (rc) return bfail(b, rc, std::string("instance layout: ") + irr_last_error(h));
-        if (h->shape.staged != staged) return IRR_ERR_CAPACITY;
+        if (h->shape.lanes_per_row != lanes || (h->shape.staged != 0) != (staged != 0)) {  // not laid out so yet
+            const int rc = irr_ensure_layout(h, lanes, h->shape.block_nodes, staged ? 1 : 0);
+            if (rc) return bfail(b, rc, std::string("instance layout: ") + irr_last_error(h));
+        }
+        if (staged && (!h->shape.staged || (h != b->handles.front() && h->shape.staged != staged)))
+            return IRR_ERR_CAPACITY;
+        if (staged) staged = h->shape.staged;
     }
     return upload_insts(b);
 }
@@ -202,7 +207,7 @@ int autotune(irr_batch* b)
         if (it != g_tune_cache.end()) b->shape = it->second;
         if (it != g_tune_cache.end()) {
             const int rc = set_lanes(b, b->shape.lanes_per_row, b->shape.staged);
-            return rc ? rc : upload_items(b, b->shape);
+            if (rc != IRR_ERR_CAPACITY) return rc ? rc : upload_items(b, b->shape);
         }
     }
     const int lanes[] = {4, 8, 16};
@@ -211,11 +216,12 @@ int autotune(irr_batch* b)
     double best_ms = 1e30;
     // the staged layout first (4 lanes per row; items are its own), where every instance takes it
     {
-        int rc = set_lanes(b, 4, 1);
+        int staged = 1;
+        int rc = set_lanes(b, 4, staged);
         if (rc == IRR_OK) {
             TiledShape s = b->shape;
             s.lanes_per_row = 4;
-            s.staged = 1;
+            s.staged = staged;
             const double ms = time_shape(b, s, 3);
             if (ms < 0) return bfail(b, IRR_ERR_CUDA, "autotune launch");
             best_ms = ms;
@@ -225,7 +231,8 @@ int autotune(irr_batch* b)
         }
     }
     for (int g : lanes) {
-        const int rc = set_lanes(b, g, 0);
+        int none = 0;
+        const int rc = set_lanes(b, g, none);
         if (rc) return rc;
         for (int r : rows) {
             TiledShape s = b->shape;
@@ -347,7 +354,7 @@ int irr_batch_finalize(irr_batch* b, int autotune_shape)
         rc = set_lanes(b, b->shape.lanes_per_row, b->shape.staged);
         if (rc == IRR_ERR_CAPACITY) {
             b->shape.staged = 0;
-            rc = set_lanes(b, b->shape.lanes_per_row, 0);
+            rc = set_lanes(b, b->shape.lanes_per_row, b->shape.staged);
         }
         if (!rc) rc = upload_items(b, b->shape);
     }

@@ -550,6 +550,12 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
         if (lanes_per_row == 4 && h->shape.stage_smem) {
             if (!h->st.words) {
                 cudaError_t se = build_staged(h->part.row_off, h->part.col, n, false, &h->st, h->stream);
+                // rows that touch more nodes than its tables hold: the wide limits
+                // (256,000 nodes with 248 neighbours each: 263 us sliced, 136 so).
+                // Where both apply they differ little (90 to 180 neighbours: 40
+                // to 84 us against 40 to 83) and the narrow ones are kept.
+                if (se == cudaErrorNotSupported && want == IRR_LAYOUT_AUTO)
+                    se = build_staged(h->part.row_off, h->part.col, n, true, &h->st, h->stream);
                 if (se != cudaSuccess) {
                     cudaGetLastError();
                     free_staged(&h->st);

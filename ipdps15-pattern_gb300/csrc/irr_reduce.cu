@@ -774,7 +774,8 @@ constexpr int kHaloSlots = 4;
 // and a slot's two addresses share a word, which needs every shared address of
 // the CTA below 2^16: the ring, the barriers, the metadata and the system's
 // reserved kilobyte.
-static_assert(kHaloRingBytes >= 4 * kHaloStreamMax + 16 * kHaloTabMax && kHaloRingBytes % 128 == 0 &&
+static_assert(kHaloRingBytes >= 4 * kHaloStreamMax + 16 * kHaloTabMax &&
+                  kHaloRingBytes >= 4 * kHaloWideStreamMax + 16 * kHaloWideTabMax && kHaloRingBytes % 128 == 0 &&
                   kHaloRingBytes + 1024 + 1024 < 65536,
               "an item fits the ring, shared addresses fit 16 bits");
 static_assert(8 * kHaloSlicesPerItem <= 64, "a row's index in its item fits the header's 6 bits");
@@ -855,7 +856,10 @@ __device__ __forceinline__ void halo_slice(const HaloSlice& sl, const InstHot& I
     write_row<4>(I.force, (int64_t)sl.row0 + ((hdr >> 24) & 0x3fu), !(hdr >> 31), ax, ay, az, lane);
 }
 
-template <bool PERIODIC, class Src>
+// WIDE: items to the wide limits, each up to the whole ring: a CTA loads and
+// computes in turn while the SM's other CTAs compute.  Its table's ids are too
+// many for the producer's registers and are read when there is room for them.
+template <bool PERIODIC, bool WIDE, class Src>
 __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
     const InstDesc* __restrict__ insts, const WorkItem* __restrict__ items, int num_items,
     int* queue, int* status, uint64_t wait_ns, int withhold, const __grid_constant__ Src src)
@@ -902,17 +906,19 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
             if (queue) it = __shfl_sync(0xffffffffu, it, 0);
             return items[it < num_items ? it : 0];
         };
-        constexpr int kIds = (kHaloTabMax + 31) / 32;
+        constexpr int kIds = WIDE ? 1 : (kHaloTabMax + 31) / 32;
         int32_t ids[kIds];
         uint32_t so = 0;
         auto fetch = [&](const WorkItem& w) {
             const InstDesc* I;
             if constexpr (ONE) I = &src.d;
             else I = insts + w.inst;
-            const int32_t* __restrict__ tab = I->tab + w.tab0 + lane;
+            if constexpr (!WIDE) {
+                const int32_t* __restrict__ tab = I->tab + w.tab0 + lane;
 #pragma unroll
-            for (int j = 0; j < kIds; j++)
-                if (32 * j + lane < (int)w.ntab) ids[j] = __ldg(tab + 32 * j);
+                for (int j = 0; j < kIds; j++)
+                    if (32 * j + lane < (int)w.ntab) ids[j] = __ldg(tab + 32 * j);
+            }
             if (lane <= (w.nrows + 7) / 8) so = __ldg(I->slice_off + w.row0 / 8 + lane) - w.ent0;
         };
         int it = (int)blockIdx.x, it1 = claim(it);  // the grid is at most num_items
@@ -988,9 +994,15 @@ __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
             __syncwarp();
             if (lane == 0) bulk_load(ring + head, I->words + w.ent0, w.nent * 4u, &full[s]);
             const float4* __restrict__ pos = I->pos;
+            if constexpr (WIDE) {
+                const int32_t* __restrict__ src_ids = I->tab + w.tab0;
+#pragma unroll 8
+                for (uint32_t j = lane; j < w.ntab; j += 32) cp_async16(tab + 16u * j, pos + __ldg(src_ids + j));
+            } else {
 #pragma unroll
-            for (int j = 0; j < kIds; j++)
-                if (32 * j + lane < (int)w.ntab) cp_async16(tab + 512u * j + 16u * lane, pos + ids[j]);
+                for (int j = 0; j < kIds; j++)
+                    if (32 * j + lane < (int)w.ntab) cp_async16(tab + 512u * j + 16u * lane, pos + ids[j]);
+            }
             cp_async_arrive(&full[s]);
             head += size;
             it = it1;
@@ -1053,12 +1065,12 @@ private:
     std::atomic<uint64_t> done_{0};
 };
 
-template <bool PERIODIC, class Src>
+template <bool PERIODIC, bool WIDE, class Src>
 cudaError_t launch_halo_src(const InstDesc* d_insts, const WorkItem* d_items, int num_items,
                             int* d_queue, int grid, int* d_status, cudaStream_t s, const Src& src,
                             const WaitPolicy& wp)
 {
-    auto kern = halo_kernel<PERIODIC, Src>;
+    auto kern = halo_kernel<PERIODIC, WIDE, Src>;
     static DeviceOnce once;
     IRR_CUDA_TRY(once.max_shared(reinterpret_cast<const void*>(kern), kHaloRingBytes));
     if (grid <= 0 || num_items <= 0) return cudaSuccess;
@@ -1071,13 +1083,13 @@ cudaError_t launch_halo_src(const InstDesc* d_insts, const WorkItem* d_items, in
                           d_items, num_items, queue, d_status, wp.wait_ns, wp.withhold, src);
 }
 
-template <bool PERIODIC>
+template <bool PERIODIC, bool WIDE>
 cudaError_t launch_halo_p(const InstDesc* d_insts, const WorkItem* d_items, int num_items,
                           int* d_queue, int grid, int* d_status, cudaStream_t s,
                           const InstDesc* host_insts, int num_insts, const WaitPolicy& wp)
 {
     if (host_insts && num_insts == 1)
-        return launch_halo_src<PERIODIC>(d_insts, d_items, num_items, d_queue, grid, d_status, s,
+        return launch_halo_src<PERIODIC, WIDE>(d_insts, d_items, num_items, d_queue, grid, d_status, s,
                                          SrcOne{host_insts[0]}, wp);
     if (host_insts && num_insts > 1 && num_insts <= kTableInsts) {
         static thread_local SrcTable t;
@@ -1085,10 +1097,10 @@ cudaError_t launch_halo_p(const InstDesc* d_insts, const WorkItem* d_items, int 
             const InstDesc& d = host_insts[k];
             t.h[k] = HotEntry{d.pos, HotLaw{d.law.half2, d.law.rc2, d.law.band}, 0.f};
         }
-        return launch_halo_src<PERIODIC>(d_insts, d_items, num_items, d_queue, grid, d_status, s, t,
+        return launch_halo_src<PERIODIC, WIDE>(d_insts, d_items, num_items, d_queue, grid, d_status, s, t,
                                          wp);
     }
-    return launch_halo_src<PERIODIC>(d_insts, d_items, num_items, d_queue, grid, d_status, s,
+    return launch_halo_src<PERIODIC, WIDE>(d_insts, d_items, num_items, d_queue, grid, d_status, s,
                                      SrcGlobal{0}, wp);
 }
 
@@ -1167,10 +1179,9 @@ cudaError_t launch_tiled(const TiledShape& shape, const InstDesc* d_insts,
     if (!d_queue) return cudaErrorInvalidValue;
     if (shape.staged) {
         if (shape.lanes_per_row != 4) return cudaErrorInvalidValue;
-        return shape.periodic ? launch_halo_p<true>(d_insts, d_items, num_items, d_queue, grid,
-                                                    d_status, s, host_insts, num_insts, wp)
-                              : launch_halo_p<false>(d_insts, d_items, num_items, d_queue, grid,
-                                                     d_status, s, host_insts, num_insts, wp);
+        auto launch = shape.staged == 2 ? (shape.periodic ? launch_halo_p<true, true> : launch_halo_p<false, true>)
+                                        : (shape.periodic ? launch_halo_p<true, false> : launch_halo_p<false, false>);
+        return launch(d_insts, d_items, num_items, d_queue, grid, d_status, s, host_insts, num_insts, wp);
     }
     return shape.periodic ? launch_tiled_p<true>(shape, d_insts, d_items, num_items, d_queue, grid,
                                                  d_status, s, host_insts, num_insts, wp)
