@@ -250,13 +250,16 @@ inline bool sliced_pays(const Sliced& sl, int64_t entries)
 // cudaFreeAsync stay in the pool for the next allocation instead of going back
 // to the driver at every synchronisation (the default pool's behaviour), so a
 // rebuild that frees and re-allocates ~300 MB of layout does not re-map it.
-// The pool keeps the library's peak footprint until the process exits.
+// The pool keeps what is freed until a handle is destroyed (irr_pool_trim).
 cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s);
 template <class T>
 inline cudaError_t irr_malloc_async(T** p, size_t bytes, cudaStream_t s)
 {
     return irr_malloc_async(reinterpret_cast<void**>(p), bytes, s);
 }
+
+// Gives back to the driver what the pool of `device` holds unused above 8 GB.
+void irr_pool_trim(int device);
 
 // How long a kernel's device-side waits may last before it gives up
 // (kStatusWaitTimeout), and the one-shot test of that path: withhold != 0
@@ -372,14 +375,13 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
 // A shard's partition: rows whose caller id is outside [lo, hi) lose their
 // entries (row_off and col rebuilt, order kept); *m_out = entries left.
 cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_t* m_out, cudaStream_t s);
-// Half neighbour list (irr_neighbor.cu); *d_edges is cudaMalloc'd, or, with
-// stream_ordered, cudaMallocAsync'd on s (free it with cudaFreeAsync).
+// Half neighbour list (irr_neighbor.cu); *d_edges is from the pool, allocated
+// on s, which is synchronised.
 // sort_rows == false returns the same pairs (i < j) in no particular order,
 // for a caller that re-sorts them anyway, like the partitioner (found by a
 // half-stencil search when the box has at least 3 cells per axis).
 cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float cut2,
-                                int2** d_edges, int64_t* num_edges, cudaStream_t s,
-                                bool stream_ordered = false, bool sort_rows = true);
+                                int2** d_edges, int64_t* num_edges, cudaStream_t s, bool sort_rows = true);
 // Full neighbour rows of a periodic box of at least 3 cells per axis (and no
 // more cells than nodes), for the MD rebuild: out->perm (new -> old) orders
 // the nodes by the Hilbert index of their cell, out->row_off / out->col hold

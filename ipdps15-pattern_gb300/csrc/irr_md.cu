@@ -309,7 +309,7 @@ int md_rebuild(irr_md* m)
         // included); the others keep the execution order.
         int2* d_edges = nullptr;
         MD_CUDA(m, build_neighbor_list(m->pos4, m->n, (float)m->cfg.side, list_cut2, &d_edges, &e, s,
-                                       true, false),
+                                       false),
                 "neighbour build");
         reorder = m->rebuilds % (m->cfg.reorder_every > 1 ? m->cfg.reorder_every : 1) == 0;
         pe = build_partition(m->pos4, m->n, d_edges, e, reorder ? 1 : 0, &p, s);

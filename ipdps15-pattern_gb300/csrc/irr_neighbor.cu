@@ -526,8 +526,6 @@ int grid_of(int64_t n)
 
 }  // namespace
 
-// Builds the list; *d_edges is cudaMalloc'd, or cudaMallocAsync'd on s when
-// stream_ordered (2 * *num_edges int32).
 namespace {
 
 // The cell grid of a list cutoff: cells at least as wide as the cutoff (so a
@@ -587,8 +585,7 @@ cudaError_t make_grid(const float4* pos, int64_t n, float box, float cut2, Grid*
 }  // namespace
 
 cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float cut2,
-                                int2** d_edges, int64_t* num_edges, cudaStream_t s,
-                                bool stream_ordered, bool sort_rows)
+                                int2** d_edges, int64_t* num_edges, cudaStream_t s, bool sort_rows)
 {
     *d_edges = nullptr;
     *num_edges = 0;
@@ -640,10 +637,7 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
     }
     int2* edges = nullptr;
     if (total > 0) {
-        if (stream_ordered)
-            IRR_CUDA_TRY(irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
-        else
-            IRR_CUDA_TRY(cudaMalloc((void**)&edges, sizeof(int2) * total));
+        IRR_CUDA_TRY(irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
         if (sort_rows) {
             uint32_t longest = 0;
             IRR_CUDA_TRY(max_row_len(cnt, n, &longest, s));
@@ -813,11 +807,11 @@ int irr_neighbor_build(int device, void* stream, const void* pos, int pos_elm, i
     cudaError_t e = cudaSuccess;
     const void* src = pos;
     if (n > 0 && !pos_on_device) {
-        e = cudaMalloc(&raw, (size_t)n * pos_elm);
+        e = irr::irr_malloc_async(&raw, (size_t)n * pos_elm, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(raw, pos, (size_t)n * pos_elm, cudaMemcpyHostToDevice, s);
         src = raw;
     }
-    if (e == cudaSuccess && n > 0) e = cudaMalloc((void**)&p4, sizeof(float4) * (size_t)n);
+    if (e == cudaSuccess && n > 0) e = irr::irr_malloc_async(&p4, sizeof(float4) * (size_t)n, s);
     if (e == cudaSuccess && n > 0) e = irr::launch_load_nodes(src, pos_elm, nullptr, n, p4, s);
     int2* edges = nullptr;
     int64_t cnt = 0;
@@ -826,12 +820,12 @@ int irr_neighbor_build(int device, void* stream, const void* pos, int pos_elm, i
     if (e != cudaSuccess) {
         cudaGetLastError();
         rc = (e == cudaErrorMemoryAllocation) ? IRR_ERR_NOMEM : (e == cudaErrorInvalidValue ? IRR_ERR_CAPACITY : IRR_ERR_CUDA);
-        if (edges) cudaFree(edges);
+        if (edges) cudaFreeAsync(edges, s);
         edges = nullptr;
         cnt = 0;
     }
-    if (raw) cudaFree(raw);
-    if (p4) cudaFree(p4);
+    if (raw) cudaFreeAsync(raw, s);
+    if (p4) cudaFreeAsync(p4, s);
     *d_edges = (int32_t*)edges;
     *num_edges = cnt;
     return rc;
@@ -841,7 +835,8 @@ int irr_device_free(int device, void* d_ptr)
 {
     if (!d_ptr) return IRR_OK;
     irr::DeviceGuard dev_guard(device);
-    if (!dev_guard.ok() || cudaFree(d_ptr) != cudaSuccess) {
+    // pool memory is freed without waiting for its last use
+    if (!dev_guard.ok() || cudaDeviceSynchronize() != cudaSuccess || cudaFree(d_ptr) != cudaSuccess) {
         cudaGetLastError();
         return IRR_ERR_CUDA;
     }

@@ -1078,4 +1078,17 @@ cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s)
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
+void irr_pool_trim(int device)
+{
+    constexpr uint64_t kKeep = 8ull << 30;
+    if (device < 0 || device >= kMaxPoolDevices) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    cudaMemPool_t pool = g_pools[device];
+    uint64_t reserved = 0, used = 0;
+    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used + kKeep)
+        cudaMemPoolTrimTo(pool, used + kKeep);
+    cudaGetLastError();
+}
+
 }  // namespace irr
