@@ -430,7 +430,7 @@ void free_pipe(irr_handle* h)
 // User map: positions for the partitioner (coordinates, else position-like
 // records, else none: the caller's order is kept), then the partition, the
 // node records in execution order, and the view's other arrays.
-int init_user(irr_handle* h)
+int init_user(irr_handle* h, const uint32_t* runs)
 {
     cudaStream_t s = h->stream;
     const int64_t n = h->n, e = h->e;
@@ -448,7 +448,7 @@ int init_user(irr_handle* h)
         reorder = 0;
     }
     PartitionOut p;
-    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, reorder, &p, s, h->cfg.order);
+    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, reorder, &p, s, h->cfg.order, runs);
     h->part = p;
     if (pe != cudaSuccess) {
         free_layout(h);
@@ -891,10 +891,16 @@ int irr_init(irr_handle* h)
     DeviceGuard dev_guard(h->device);
     cudaStream_t s = h->stream;
     const int64_t n = h->n, e = h->e;
-    H_CUDA(h, launch_validate_edges(h->d_edges, e, n, h->d_status, s), "validate edges");
-    int rc = check_status(h);
-    if (rc) return rc;
-    if (h->user_launch) return init_user(h);
+    // the list's runs of idx0, for the partitioner
+    uint32_t* runs = nullptr;
+    if (h->cfg.exec == IRR_EXEC_PARTITIONED) H_CUDA(h, dalloc(h, &runs, sizeof(uint32_t) * (size_t)(2 * n + 1)), "edge runs");
+    const cudaError_t ve = launch_validate_edges(h->d_edges, e, n, h->d_status, runs, s);
+    int rc = ve == cudaSuccess ? check_status(h) : cuda_fail(h, ve, "validate edges");
+    if (rc || h->user_launch) {
+        if (!rc) rc = init_user(h, runs);
+        dfree(h, runs);
+        return rc;
+    }
     const size_t nb = (size_t)(n > 0 ? n : 1) * sizeof(float4);
     H_CUDA(h, dalloc(h, &h->d_pos, nb), "allocate positions");
     H_CUDA(h, dalloc(h, &h->d_force, nb), "allocate results");
@@ -911,7 +917,8 @@ int irr_init(irr_handle* h)
     // partitioned: positions in the caller's order feed the partitioner
     H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, nullptr, n, h->d_pos, s), "load node data");
     PartitionOut p;
-    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, h->cfg.reorder, &p, s, h->cfg.order);
+    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, h->cfg.reorder, &p, s, h->cfg.order, runs);
+    dfree(h, runs);
     h->part = p;
     if (pe != cudaSuccess) {
         free_layout(h);

@@ -303,7 +303,9 @@ void* host_device_view(const void* p);
 // in order (out may be device memory or page-locked host memory).
 cudaError_t launch_store_result(const float4* force, const int32_t* inv, int64_t n,
                                 int elm_size, void* out, cudaStream_t s);
-cudaError_t launch_validate_edges(const int2* edges, int64_t e, int64_t n, int* d_status,
+// runs (or nullptr): 2n + 1 words; when the list is sorted by idx0, node i's
+// edges are [runs[i], runs[n + i]); runs[2n] != 0 when it is not.
+cudaError_t launch_validate_edges(const int2* edges, int64_t e, int64_t n, int* d_status, uint32_t* runs,
                                   cudaStream_t s);
 
 // -- user-map records (irr_user.cu) --
@@ -370,8 +372,10 @@ cudaError_t bbox_frame(const float4* pos, int64_t n, float lo[3], float scale[3]
 // Full partition of n nodes and e half edges.  Allocates out's arrays with
 // cudaMallocAsync on s (caller frees).  reorder == 0 keeps the identity order.
 // curve: 0 = Hilbert (IRR_ORDER_HILBERT), 1 = Morton.
+// runs: of the edges, from launch_validate_edges (nullptr: not known).
 cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges, int64_t e,
-                            int reorder, PartitionOut* out, cudaStream_t s, int curve = 0);
+                            int reorder, PartitionOut* out, cudaStream_t s, int curve = 0,
+                            const uint32_t* runs = nullptr);
 // A shard's partition: rows whose caller id is outside [lo, hi) lose their
 // entries (row_off and col rebuilt, order kept); *m_out = entries left.
 cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_t* m_out, cudaStream_t s);
@@ -397,7 +401,9 @@ cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cu
 // Sorts each row of a CSR (row_off[n + 1], col) ascending; every row must
 // hold at most kRowSortMax entries.
 constexpr int kRowSortMax = 1024;
-cudaError_t launch_row_sort(const uint32_t* row_off, int64_t n, int32_t* col, cudaStream_t s);
+// slots: the rows are read from slots[r * cap, ...) instead.
+cudaError_t launch_row_sort(const uint32_t* row_off, int64_t n, int32_t* col, cudaStream_t s,
+                            const int32_t* slots = nullptr, uint32_t cap = 0);
 // The longest row of a CSR (synchronises s).
 cudaError_t max_row_len(const uint32_t* row_off, int64_t n, uint32_t* result, cudaStream_t s);
 // Stable LSD radix sort of (key, value) pairs on key bits [0, key_bits).
