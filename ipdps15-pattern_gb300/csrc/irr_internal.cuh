@@ -404,6 +404,10 @@ constexpr int kRowSortMax = 1024;
 // slots: the rows are read from slots[r * cap, ...) instead.
 cudaError_t launch_row_sort(const uint32_t* row_off, int64_t n, int32_t* col, cudaStream_t s,
                             const int32_t* slots = nullptr, uint32_t cap = 0);
+// pairs[row_off[ids[t]], ...) = (ids[t], v) for the entries v of slots[t * cap, ...), ascending;
+// at most kRowSortMax of them.
+cudaError_t launch_slot_pairs(const uint32_t* row_off, const int32_t* ids, int64_t n, const int32_t* slots,
+                              uint32_t cap, int2* pairs, cudaStream_t s);
 // The longest row of a CSR (synchronises s).
 cudaError_t max_row_len(const uint32_t* row_off, int64_t n, uint32_t* result, cudaStream_t s);
 // Stable LSD radix sort of (key, value) pairs on key bits [0, key_bits).

@@ -27,6 +27,7 @@
 // written by one search over its 27 cells visited in curve order -- ascending
 // by construction, so the rows need neither the pair list, nor atomic row
 // cursors, nor a sort.
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -142,13 +143,18 @@ __global__ void cell_keys_kernel(const float4* pos, int64_t n, const __grid_cons
     }
 }
 
-// pos_c[q] = pos[sorted[q]]: positions in cell order
+// pos_c[q] = pos[sorted[q]]: positions in cell order, the node's id in w
 __global__ void cell_order_kernel(const float4* __restrict__ pos, const int32_t* __restrict__ sorted,
                                   int64_t n, float4* __restrict__ pos_c)
 {
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
          q += (int64_t)gridDim.x * blockDim.x)
-        pos_c[q] = pos[sorted[q]];
+    {
+        const int32_t i = sorted[q];
+        float4 p = pos[i];
+        p.w = __int_as_float(i);
+        pos_c[q] = p;
+    }
 }
 
 // WRITE == false: counts partners; WRITE == true: writes them from row_off[i],
@@ -236,6 +242,80 @@ __global__ void pairs_kernel(const float4* __restrict__ pos_c, const int32_t* __
         pairs_rows<WRITE, true>(pos_c, sorted, cell_start, n, g, count, row_off, nbr, pairs, sort_here);
     else
         pairs_rows<WRITE, false>(pos_c, sorted, cell_start, n, g, count, row_off, nbr, pairs, sort_here);
+}
+
+// The same partners j > i of every node in one pass, into slots of `cap` per
+// node (in cell order), where the cell decides the image (open boundaries, or
+// Grid::fast and every position in the box; else *over = 1 and nothing is
+// written).  cnt[i] = node i's partners; *over is raised when one has more than
+// cap.  The cells of a grid row are neighbours in cell order, so a node's 27
+// cells are 9 runs of candidates (at the wall of a periodic box up to 18), each
+// candidate one 16-byte load that brings its id.
+// What bounds it: issue, ~14 instructions a candidate and ~580 candidates a
+// node at 64 neighbours.  1,000,003 nodes, list radius 2.8: counting 556 +
+// writing 730 us with 27 runs and two loads a candidate -> 474 us.
+__global__ void __launch_bounds__(256) slot_partners_kernel(const float4* __restrict__ pos_c,
+                                                           const uint32_t* __restrict__ keys,
+                                                           const uint32_t* __restrict__ cell_start, int64_t n,
+                                                           const __grid_constant__ Grid g,
+                                                           const int* __restrict__ outside, uint32_t cap,
+                                                           uint32_t* __restrict__ cnt,
+                                                           int32_t* __restrict__ slots, int* over)
+{
+    if (g.periodic && (!g.fast || *outside)) {
+        if (threadIdx.x == 0) *over = 1;
+        return;
+    }
+    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < n; t0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t t = t0 + threadIdx.x;
+        if (t >= n) continue;
+        const float4 a = pos_c[t];
+        const int32_t i = __float_as_int(a.w);
+        const uint32_t c = keys[t];
+        const int cx = (int)(c % (uint32_t)g.nc[0]), cy = (int)(c / (uint32_t)g.nc[0] % (uint32_t)g.nc[1]),
+                  cz = (int)(c / ((uint32_t)g.nc[0] * (uint32_t)g.nc[1]));
+        // the block's slots, and the thread's next one and their end in them: 32-bit
+        // offsets from one base
+        char* const base = reinterpret_cast<char*>(slots + t0 * (int64_t)cap);
+        const uint32_t first = threadIdx.x * cap * 4u, end = first + cap * 4u;
+        uint32_t at = first;
+        auto run = [&](auto shift, uint32_t q, uint32_t q1, float sx, float sy, float sz) {
+#pragma unroll 8
+            for (; q < q1; q++) {
+                const float4 b = pos_c[q];
+                const int32_t j = __float_as_int(b.w);
+                // no branch: a hit every sixth candidate, so most warps have one
+                const bool hit = (j > i) & (decltype(shift)::value ? list_pair_shifted(a, b, sx, sy, sz, g.cut2)
+                                                                   : list_pair_unshifted(a, b, g.cut2));
+                if (hit & (at < end)) *reinterpret_cast<int32_t*>(base + at) = j;
+                at += hit ? 4u : 0u;
+            }
+        };
+        for (int k = 0; k < 9; k++) {
+            int z = cz + k / 3 - 1, y = cy + k % 3 - 1;
+            float sy = 0.f, sz = 0.f;
+            if (g.periodic) {
+                wrap_cell(z, g.nc[2], g.box, sz);
+                wrap_cell(y, g.nc[1], g.box, sy);
+            } else if (z < 0 || z >= g.nc[2] || y < 0 || y >= g.nc[1]) {
+                continue;
+            }
+            const uint32_t row = ((uint32_t)z * g.nc[1] + y) * g.nc[0];
+            const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.nc[0] - 1);
+            if (sy == 0.f && sz == 0.f)
+                run(std::false_type{}, cell_start[row + x0], cell_start[row + x1 + 1], 0.f, 0.f, 0.f);
+            else
+                run(std::true_type{}, cell_start[row + x0], cell_start[row + x1 + 1], 0.f, sy, sz);
+            if (g.periodic && (cx == 0 || cx == g.nc[0] - 1)) {
+                int x = cx == 0 ? -1 : g.nc[0];
+                float sx;
+                wrap_cell(x, g.nc[0], g.box, sx);
+                run(std::true_type{}, cell_start[row + x], cell_start[row + x + 1], sx, sy, sz);
+            }
+        }
+        cnt[i] = (at - first) / 4u;
+        if (at > end) *over = 1;
+    }
 }
 
 // The same pairs from a half stencil, for callers that take the pairs in any
@@ -615,6 +695,46 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
     IRR_CUDA_TRY(irr_malloc_async((void**)&pos_c, sizeof(float4) * n, s));
     cell_order_kernel<<<grid_of(n), 256, 0, s>>>(pos, sorted, n, pos_c);
     IRR_CUDA_TRY(cudaGetLastError());
+    // rows in order: one search pass into slots, where the cells decide the images
+    // and the slots (a third more than the mean sphere's nodes, and some) fit
+    double volume = 1.0;
+    for (int c = 0; c < 3; c++) volume *= g.periodic ? (double)box : std::max(g.nc[c] / g.inv[c], std::sqrt((double)cut2));
+    const double sphere = volume > 0 ? 4.18879 * cut2 * std::sqrt((double)cut2) * n / volume : (double)n;
+    const uint32_t cap = sphere < kRowSortMax ? ((uint32_t)(1.35 * sphere) + 31u) / 8u * 8u : 0u;
+    if (sort_rows && cap > 0 && cap <= (uint32_t)kRowSortMax && (g.fast || !g.periodic)) {
+        int32_t* slots = nullptr;
+        if (irr_malloc_async((void**)&slots, sizeof(int32_t) * cap * (size_t)n, s) != cudaSuccess) {
+            cudaGetLastError();  // no room: count first
+        } else {
+            uint32_t* aux = keys_tmp;  // reuse: the total, the flag that slots did not do
+            IRR_CUDA_TRY(cudaMemsetAsync(aux, 0, 2 * sizeof(uint32_t), s));
+            slot_partners_kernel<<<grid_of(n), 256, 0, s>>>(pos_c, keys, cell_start, n, g, outside, cap, cnt, slots,
+                                                            reinterpret_cast<int*>(aux + 1));
+            IRR_CUDA_TRY(cudaGetLastError());
+            IRR_CUDA_TRY(cudaMemsetAsync(cnt + n, 0, sizeof(uint32_t), s));
+            IRR_CUDA_TRY(scan_exclusive_u32(cnt, cnt, n + 1, aux, s));
+            uint32_t got[2] = {0, 0};
+            IRR_CUDA_TRY(cudaMemcpyAsync(got, aux, sizeof(got), cudaMemcpyDeviceToHost, s));
+            IRR_CUDA_TRY(cudaStreamSynchronize(s));
+            // (a total that does not fit 32 bits needs rows the slots do not hold, or more
+            // than 2^31 nodes' worth of memory: the counting path reports it)
+            const bool done = !got[1] && (double)cap * (double)n < 4294967296.0 && got[0] <= 0x7fffffffu;
+            int2* edges = nullptr;
+            if (done && got[0] > 0) {
+                IRR_CUDA_TRY(irr_malloc_async((void**)&edges, sizeof(int2) * got[0], s));
+                IRR_CUDA_TRY(launch_slot_pairs(cnt, sorted, n, slots, cap, edges, s));
+            }
+            void* tmp[] = {slots, keys, keys_tmp, sorted, vals_tmp, cell_start, cnt, pos_c};
+            for (void* q : tmp)
+                if (done || q == slots) IRR_CUDA_TRY(cudaFreeAsync(q, s));
+            if (done) {
+                IRR_CUDA_TRY(cudaStreamSynchronize(s));
+                *d_edges = edges;
+                *num_edges = got[0];
+                return cudaSuccess;
+            }
+        }
+    }
     // rows in any order are asked for: the half stencil, where the box allows it
     const bool half = !sort_rows && g.nc[0] >= 3 && g.nc[1] >= 3 && g.nc[2] >= 3;
     if (half)

@@ -167,9 +167,8 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
 // rows, up to kRowSortMax entries, go through a shared-memory buffer.
 constexpr int kRowSortWarps = 8;
 
-template <int E>
-__device__ __forceinline__ void sort_row_in_registers(const int32_t* src, int32_t* col, uint32_t beg,
-                                                      uint32_t len, int lane)
+template <int E, class Put>
+__device__ __forceinline__ void sort_row_in_registers(const int32_t* src, uint32_t len, int lane, Put put)
 {
     int32_t v[E];
 #pragma unroll
@@ -205,8 +204,39 @@ __device__ __forceinline__ void sort_row_in_registers(const int32_t* src, int32_
 #pragma unroll
     for (int r = 0; r < E; r++) {
         const uint32_t k = (uint32_t)(r * 32 + lane);
-        if (k < len) col[beg + k] = v[r];
+        if (k < len) put(k, v[r]);
     }
+}
+
+// One row by one warp: put(k, the row's k-th entry); b: kRowSortMax words.
+template <class Put>
+__device__ __forceinline__ void sort_row(const int32_t* src, uint32_t len, int lane, int32_t* b, Put put)
+{
+    if (len <= 32) return sort_row_in_registers<1>(src, len, lane, put);
+    if (len <= 64) return sort_row_in_registers<2>(src, len, lane, put);
+    if (len <= 128) return sort_row_in_registers<4>(src, len, lane, put);
+    if (len <= 256) return sort_row_in_registers<8>(src, len, lane, put);
+    uint32_t P = 2;
+    while (P < len) P <<= 1;  // len <= kRowSortMax, so P <= kRowSortMax
+    for (uint32_t k = lane; k < P; k += 32) b[k] = k < len ? src[k] : 0x7fffffff;
+    __syncwarp();
+    for (uint32_t size = 2; size <= P; size <<= 1) {
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t k = lane; k < P; k += 32) {
+                const uint32_t o = k ^ stride;
+                if (o > k) {
+                    const int32_t x = b[k], y = b[o];
+                    if ((x > y) == ((k & size) == 0)) {
+                        b[k] = y;
+                        b[o] = x;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    for (uint32_t k = lane; k < len; k += 32) put(k, b[k]);
+    __syncwarp();
 }
 
 // The row's entries are at its place in col, or, with slots, at slots[r * cap].
@@ -223,43 +253,26 @@ __global__ void __launch_bounds__(kRowSortWarps * 32) row_sort_kernel(const uint
         const uint32_t len = row_off[r + 1] - beg;
         const int32_t* src = slots ? slots + r * (int64_t)cap : col + beg;
         if (len < 2 && !slots) continue;
-        if (len <= 32) {
-            sort_row_in_registers<1>(src, col, beg, len, lane);
-            continue;
-        }
-        if (len <= 64) {
-            sort_row_in_registers<2>(src, col, beg, len, lane);
-            continue;
-        }
-        if (len <= 128) {
-            sort_row_in_registers<4>(src, col, beg, len, lane);
-            continue;
-        }
-        if (len <= 256) {
-            sort_row_in_registers<8>(src, col, beg, len, lane);
-            continue;
-        }
-        uint32_t P = 2;
-        while (P < len) P <<= 1;  // len <= kRowSortMax, so P <= kRowSortMax
-        for (uint32_t k = lane; k < P; k += 32) b[k] = k < len ? src[k] : 0x7fffffff;
-        __syncwarp();
-        for (uint32_t size = 2; size <= P; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t k = lane; k < P; k += 32) {
-                    const uint32_t o = k ^ stride;
-                    if (o > k) {
-                        const int32_t x = b[k], y = b[o];
-                        if ((x > y) == ((k & size) == 0)) {
-                            b[k] = y;
-                            b[o] = x;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        for (uint32_t k = lane; k < len; k += 32) col[beg + k] = b[k];
-        __syncwarp();
+        sort_row(src, len, lane, b, [&](uint32_t k, int32_t v) { col[beg + k] = v; });
+    }
+}
+
+// Row t of the slots holds the partners of node ids[t]: sorted, as pairs, at
+// the node's place.
+__global__ void __launch_bounds__(kRowSortWarps * 32) slot_pairs_kernel(const uint32_t* __restrict__ row_off,
+                                                                       const int32_t* __restrict__ ids,
+                                                                       int64_t n, const int32_t* slots,
+                                                                       uint32_t cap, int2* __restrict__ pairs)
+{
+    __shared__ int32_t buf[kRowSortWarps][kRowSortMax];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    for (int64_t t = (int64_t)blockIdx.x * kRowSortWarps + warp; t < n;
+         t += (int64_t)gridDim.x * kRowSortWarps) {
+        const int32_t i = ids[t];
+        const uint32_t beg = row_off[i], len = row_off[i + 1] - beg;
+        if (len == 0) continue;
+        sort_row(slots + t * (int64_t)cap, len, lane, buf[warp],
+                 [&](uint32_t k, int32_t v) { pairs[beg + k] = make_int2(i, v); });
     }
 }
 
@@ -812,6 +825,15 @@ cudaError_t launch_row_sort(const uint32_t* row_off, int64_t n, int32_t* col, cu
     int64_t blocks = (n + kRowSortWarps - 1) / kRowSortWarps;
     if (blocks > 65536) blocks = 65536;
     row_sort_kernel<<<(unsigned)blocks, kRowSortWarps * 32, 0, s>>>(row_off, n, col, slots, cap);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_slot_pairs(const uint32_t* row_off, const int32_t* ids, int64_t n, const int32_t* slots,
+                              uint32_t cap, int2* pairs, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    const int64_t blocks = std::min<int64_t>((n + kRowSortWarps - 1) / kRowSortWarps, 65536);
+    slot_pairs_kernel<<<(unsigned)blocks, kRowSortWarps * 32, 0, s>>>(row_off, ids, n, slots, cap, pairs);
     return cudaGetLastError();
 }
 
