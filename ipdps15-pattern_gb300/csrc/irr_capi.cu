@@ -85,6 +85,7 @@ void free_layout(irr_handle* h)
     dfree(h, h->part.inv);
     dfree(h, h->part.row_off);
     dfree(h, h->part.col);
+    dfree(h, h->part.slots);
     free_sliced(&h->sl, h->stream);
     free_staged(&h->st, h->stream);
     h->shape.staged = 0;
@@ -349,6 +350,7 @@ int apply_shard(irr_handle* h)
     if (h->own_lo < 0 || h->own_lo > h->own_hi || h->own_hi > h->n)
         return fail(h, IRR_ERR_STATE, "shard rows [%lld, %lld) outside the %lld nodes", (long long)h->own_lo,
                     (long long)h->own_hi, (long long)h->n);
+    H_CUDA(h, partition_rows(&h->part, h->n, 2 * h->e, h->stream), "partition rows");
     H_CUDA(h, keep_rows(&h->part, h->n, h->own_lo, h->own_hi, &h->m, h->stream), "shard rows");
     return IRR_OK;
 }
@@ -545,6 +547,28 @@ int irr_host_row_off(irr_handle* h)
     return IRR_OK;
 }
 
+namespace {
+
+// part.col of a handle whose entries are in the partitioner's slots or in the
+// staged layout alone.
+int ensure_rows(irr_handle* h)
+{
+    if (h->part.col) return IRR_OK;
+    if (!h->part.slots && (h->shape.staged || h->st.words)) {
+        H_CUDA(h, alloc_col(&h->part.col, h->m, h->stream), "allocate entries");
+        const cudaError_t e = rows_of_staged(h->st, h->st.items ? h->st.items : h->d_items, h->part.row_off, h->n,
+                                             h->part.col, h->stream);
+        if (e != cudaSuccess) {
+            dfree(h, h->part.col);
+            return cuda_fail(h, e, "rows of the staged layout");
+        }
+    }
+    H_CUDA(h, partition_rows(&h->part, h->n, h->m, h->stream), "partition rows");
+    return IRR_OK;
+}
+
+}  // namespace
+
 int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int staged_ok)
 {
     TraceRange trace_("irr_layout");
@@ -562,13 +586,14 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     if (want == IRR_LAYOUT_STAGED || (want == IRR_LAYOUT_AUTO && kAutoStaged && staged_ok)) {
         if (lanes_per_row == 4 && h->shape.stage_smem) {
             if (!h->st.words) {
-                cudaError_t se = build_staged(h->part.row_off, h->part.col, n, false, &h->st, h->stream);
+                const RowSource rows{h->part.row_off, h->part.col, h->part.slots, h->part.cap};
+                cudaError_t se = build_staged(rows, n, h->m, false, &h->st, h->stream);
                 // rows that touch more nodes than its tables hold: the wide limits
                 // (256,000 nodes with 248 neighbours each: 263 us sliced, 136 so).
                 // Where both apply they differ little (90 to 180 neighbours: 40
                 // to 84 us against 40 to 83) and the narrow ones are kept.
                 if (se == cudaErrorNotSupported && want == IRR_LAYOUT_AUTO)
-                    se = build_staged(h->part.row_off, h->part.col, n, true, &h->st, h->stream);
+                    se = build_staged(rows, n, h->m, true, &h->st, h->stream);
                 if (se != cudaSuccess) {
                     cudaGetLastError();
                     free_staged(&h->st);
@@ -590,7 +615,10 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     h->shape.staged = staged ? (h->st.wide ? 2 : 1) : 0;
     if (staged) {
         free_sliced(&h->sl);
+        dfree(h, h->part.slots);  // the layout holds the entries now
     } else {
+        const int rc = ensure_rows(h);
+        if (rc) return rc;
         free_staged(&h->st);
         if (want == IRR_LAYOUT_CSR) {
             free_sliced(&h->sl);
@@ -613,7 +641,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     rc = upload_items(h);
     if (rc) return rc;
     h->dev_bytes = 2 * (int64_t)(n > 0 ? n : 1) * (int64_t)sizeof(float4) + (int64_t)h->raw_cap +
-                   (int64_t)(2 * n + n + 1) * 4 + h->m * 4 +
+                   (int64_t)(2 * n + n + 1) * 4 + (h->part.col ? h->m * 4 : 0) +
                    (h->sl.lanes ? 4 * (h->sl.words + h->sl.slices + 1) : 0) +
                    (h->shape.staged ? 4 * (h->st.nwords + h->st.nids + h->st.slices + 1) : 0);
     return IRR_OK;
@@ -917,7 +945,7 @@ int irr_init(irr_handle* h)
     // partitioned: positions in the caller's order feed the partitioner
     H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, nullptr, n, h->d_pos, s), "load node data");
     PartitionOut p;
-    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, h->cfg.reorder, &p, s, h->cfg.order, runs);
+    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, h->cfg.reorder, &p, s, h->cfg.order, runs, true);
     dfree(h, runs);
     h->part = p;
     if (pe != cudaSuccess) {
@@ -1120,6 +1148,10 @@ int irr_get_partition(irr_handle* h, int32_t* perm, int64_t* row_off, int32_t* c
     if (!h->inited) return fail(h, IRR_ERR_STATE, "no partition before irr_init");
     DeviceGuard dev_guard(h->device);
     const int64_t n = h->n, m = h->m;
+    if (col && m > 0) {
+        const int rc = ensure_rows(h);
+        if (rc) return rc;
+    }
     if (perm && n > 0)
         H_CUDA(h, cudaMemcpyAsync(perm, h->part.perm, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, h->stream), "copy perm");
     std::vector<uint32_t> ro;

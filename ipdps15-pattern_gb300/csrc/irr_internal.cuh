@@ -178,13 +178,29 @@ struct Staged {
 // loads.
 constexpr int kHaloWideTabMax = 1008;
 constexpr int kHaloWideStreamMax = 9984;
-// Builds st from a CSR (rows in execution order, columns ascending) on the
-// device.  Synchronises s.  cudaErrorNotSupported (nothing allocated) when a
-// slice alone exceeds the limits above -- a row of more than ~440 entries
-// (wide: 1023), or 8 rows touching more than kHaloTabMax (wide:
-// kHaloWideTabMax) distinct nodes.
-cudaError_t build_staged(const uint32_t* row_off, const int32_t* col, int64_t n, bool wide, Staged* st,
-                         cudaStream_t s);
+// Where a graph's rows are, in execution order, each row's columns in any
+// order: packed in col at row_off, or, with slots, cap apart there.
+struct RowSource {
+    const uint32_t* row_off;
+    const int32_t* col;
+    const int32_t* slots;
+    int64_t cap;
+#ifdef __CUDACC__
+    __device__ __forceinline__ const int32_t* row(int64_t r, uint32_t beg) const
+    {
+        return slots ? slots + r * cap : col + beg;
+    }
+#endif
+};
+// Builds st from n rows of m entries in all on the device.  Synchronises s.
+// cudaErrorNotSupported (nothing allocated) when a slice alone exceeds the
+// limits above -- a row of more than ~440 entries (wide: 1023), or 8 rows
+// touching more than kHaloTabMax (wide: kHaloWideTabMax) distinct nodes.
+cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, Staged* st, cudaStream_t s);
+// The rows back from the layout (items: st's, wherever they are now): col, at
+// row_off, each row ascending.
+cudaError_t rows_of_staged(const Staged& st, const WorkItem* items, const uint32_t* row_off, int64_t n, int32_t* col,
+                           cudaStream_t s);
 void free_staged(Staged* st, cudaStream_t s = nullptr);
 // Items copied to the host; synchronises s.
 cudaError_t staged_items_to_host(const WorkItem* d_items, int64_t count, std::vector<WorkItem>* items, cudaStream_t s);
@@ -361,7 +377,9 @@ struct PartitionOut {
     int32_t* perm = nullptr;      // [n] new -> old
     int32_t* inv = nullptr;       // [n] old -> new
     uint32_t* row_off = nullptr;  // [n + 1]
-    int32_t* col = nullptr;       // [2e]
+    int32_t* col = nullptr;       // [2e], rows ascending; null while slots hold the entries
+    int32_t* slots = nullptr;     // row r's entries at slots[r * cap], in any order (or null)
+    int64_t cap = 0;
 };
 // Per-axis min and max of pos (synchronises s).
 cudaError_t bbox_minmax(const float4* pos, int64_t n, float lo[3], float hi[3], cudaStream_t s);
@@ -373,9 +391,16 @@ cudaError_t bbox_frame(const float4* pos, int64_t n, float lo[3], float scale[3]
 // cudaMallocAsync on s (caller frees).  reorder == 0 keeps the identity order.
 // curve: 0 = Hilbert (IRR_ORDER_HILBERT), 1 = Morton.
 // runs: of the edges, from launch_validate_edges (nullptr: not known).
+// keep_slots: where the rows were filled into slots they may stay there,
+// unsorted, out->col null (partition_rows packs them).
 cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges, int64_t e,
                             int reorder, PartitionOut* out, cudaStream_t s, int curve = 0,
-                            const uint32_t* runs = nullptr);
+                            const uint32_t* runs = nullptr, bool keep_slots = false);
+// out->col (m entries) from out->slots, which are freed; nothing where there
+// are none.
+cudaError_t partition_rows(PartitionOut* out, int64_t n, int64_t m, cudaStream_t s);
+// An array of m entries, and the padding that reads of col may touch, cleared.
+cudaError_t alloc_col(int32_t** col, int64_t m, cudaStream_t s);
 // A shard's partition: rows whose caller id is outside [lo, hi) lose their
 // entries (row_off and col rebuilt, order kept); *m_out = entries left.
 cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_t* m_out, cudaStream_t s);

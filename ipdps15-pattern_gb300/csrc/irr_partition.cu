@@ -851,19 +851,33 @@ cudaError_t max_row_len(const uint32_t* row_off, int64_t n, uint32_t* result, cu
     return cudaStreamSynchronize(s);
 }
 
+cudaError_t alloc_col(int32_t** col, int64_t m, cudaStream_t s)
+{
+    // + kColPad: bulk copies of an entry segment are widened to 16-byte
+    // boundaries and may read up to 3 entries past the last one
+    IRR_CUDA_TRY(alloc_async(col, m + kColPad, s));
+    return cudaMemsetAsync(*col + m, 0, sizeof(int32_t) * kColPad, s);
+}
+
+cudaError_t partition_rows(PartitionOut* out, int64_t n, int64_t m, cudaStream_t s)
+{
+    if (!out->slots) return cudaSuccess;
+    IRR_CUDA_TRY(alloc_col(&out->col, m, s));
+    IRR_CUDA_TRY(launch_row_sort(out->row_off, n, out->col, s, out->slots, (uint32_t)out->cap));
+    IRR_CUDA_TRY(cudaFreeAsync(out->slots, s));
+    out->slots = nullptr;
+    return cudaSuccess;
+}
+
 cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges, int64_t e,
                             int reorder, PartitionOut* out, cudaStream_t s, int curve,
-                            const uint32_t* runs)
+                            const uint32_t* runs, bool keep_slots)
 {
     if (n < 0 || e < 0 || n > 0x7fffffffLL || 2 * e > 0xffffffffLL) return cudaErrorInvalidValue;
     *out = PartitionOut{};
     IRR_CUDA_TRY(alloc_async(&out->perm, n, s));
     IRR_CUDA_TRY(alloc_async(&out->inv, n, s));
     IRR_CUDA_TRY(alloc_async(&out->row_off, n + 1, s));
-    // + kColPad: bulk copies of an entry segment are widened to 16-byte
-    // boundaries and may read up to 3 entries past the last one
-    IRR_CUDA_TRY(alloc_async(&out->col, 2 * e + kColPad, s));
-    IRR_CUDA_TRY(cudaMemsetAsync(out->col + 2 * e, 0, sizeof(int32_t) * kColPad, s));
     const int g = grid_for(n);
     if (reorder && n > 1) {
         float lo[3], scale[3];
@@ -896,30 +910,31 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
     // vary by a few standard deviations of a Poisson count
     const int64_t cap = n > 0 ? (3 * e / n + 24 + 7) / 8 * 8 : 0;
     if (runs && e > 0 && n > 0 && cap <= kRowSortMax) {
-        int32_t* slots = nullptr;
         int* over = nullptr;
-        if (alloc_async(&slots, n * cap, s) != cudaSuccess) {
+        if (alloc_async(&out->slots, n * cap, s) != cudaSuccess) {
             cudaGetLastError();  // no room: count first
+            out->slots = nullptr;
         } else {
+            out->cap = cap;
             IRR_CUDA_TRY(alloc_async(&over, 1, s));
             IRR_CUDA_TRY(cudaMemsetAsync(over, 0, sizeof(int), s));
             slot_rows_kernel<<<grid_for(32 * n), 256, 0, s>>>(edges, runs, out->perm, out->inv, n, (uint32_t)cap, deg,
-                                                             slots, over);
+                                                             out->slots, over);
             IRR_CUDA_TRY(cudaGetLastError());
             int was_over = 0;
             IRR_CUDA_TRY(cudaMemcpyAsync(&was_over, over, sizeof(int), cudaMemcpyDeviceToHost, s));
+            IRR_CUDA_TRY(cudaFreeAsync(over, s));
             IRR_CUDA_TRY(cudaStreamSynchronize(s));
             if (!was_over) {
                 IRR_CUDA_TRY(scan_exclusive_u32(deg, out->row_off, n + 1, nullptr, s));
-                IRR_CUDA_TRY(launch_row_sort(out->row_off, n, out->col, s, slots, (uint32_t)cap));
-            } else {
-                IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
+                return keep_slots ? cudaSuccess : partition_rows(out, n, 2 * e, s);
             }
-            IRR_CUDA_TRY(cudaFreeAsync(slots, s));
-            IRR_CUDA_TRY(cudaFreeAsync(over, s));
-            if (!was_over) return cudaSuccess;
+            IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
+            IRR_CUDA_TRY(cudaFreeAsync(out->slots, s));
+            out->slots = nullptr;
         }
     }
+    IRR_CUDA_TRY(alloc_col(&out->col, 2 * e, s));
     if (e > 0 && n > 0) {
         // rows of at most kRowSortMax entries (every MD list): count, scan,
         // fill at per-row cursors, sort each row -- the same (row, col) layout

@@ -38,16 +38,19 @@
 //                      map from the block a run enters it at to the next tile's;
 //   run_entries_kernel the entries of a greedy cut from block 0, by composing
 //   list_runs_kernel   those maps (8 states), and its runs;
-//   cut_runs_kernel    one CTA per run: the items' tables counted, their words;
+//   cut_runs_kernel    one CTA per run: its items, their tables and every
+//                      entry's place in its item's table (scratch);
 //   place_items_kernel the items' places in the words and tables;
 //   fill_items_kernel  one CTA per item: its table, words and slice offsets.
-// A table is gathered as a hash of 32-id groups with a bit per id: neighbours
-// on the curve share groups, so ~465 ids are ~120 groups to sort, and an id's
-// slot is its group's first slot plus a population count -- no search.
-// What bounds it: instruction issue (a hash probe and a bucket per entry).
-// 1,000,003 nodes at 64 neighbours: counting 228 -> 173 us, filling 1129 -> 722 us,
-// and the cut, the row offsets' copy to the host and the per-run counts' copies
-// (~1.6 ms on the host) are gone.
+// The rows come in any order (the partitioner's slots, unsorted): a table is
+// gathered as a hash of 32-id groups with a bit per id -- neighbours on the
+// curve share groups, so ~465 ids are ~120 groups to order, and an id's slot is
+// its group's first slot plus a population count -- and a row's places are
+// ordered as bits of a 1,024-bit map.
+// What bounds it: instruction issue (a hash probe, a bit and a pick per entry).
+// 1,000,003 nodes at 64 neighbours: sorting the rows, counting the tables and
+// filling, a table gathered in both, 353 + 172 + 721 us; now 443 + 343, and the
+// rows (4 bytes an entry) are made from the layout when they are asked for.
 #include <algorithm>
 #include <climits>
 #include <vector>
@@ -58,25 +61,29 @@ namespace irr {
 namespace {
 
 constexpr int kPick = 8;                         // slices of an item, blocks of a run: at most
-// The limits of the two variants.
+// The limits of the two variants.  kAhead: columns a thread has in flight while
+// it adds them to the table.
 struct NarrowItem {
     static constexpr int kTab = kHaloTabMax, kStream = kHaloStreamMax;
-    static constexpr int kHash = 1024, kThreads = 128, kCtas = 7, kHeld = 4, kCutAhead = 2;
+    static constexpr int kHash = 1024, kCutThreads = 128, kAhead = 2;
+    static constexpr int kFillWarps = 2, kFillCtas = 12;
 };
 struct WideItem {
     static constexpr int kTab = kHaloWideTabMax, kStream = kHaloWideStreamMax;
-    static constexpr int kHash = 2048, kThreads = 256, kCtas = 3, kHeld = 8, kCutAhead = 4;
+    static constexpr int kHash = 2048, kCutThreads = 256, kAhead = 4;
+    static constexpr int kFillWarps = 4, kFillCtas = 5;
 };
-static_assert(kHaloTabMax < 1024 - 4 && kHaloWideTabMax < 2048 - 4, "groups and their padding fit the hash");
+// add_rows' ids past the limit (8 rows' own ids, then what is in flight) fit the hash
 template <class V>
-constexpr bool holds_overshoot = V::kTab + V::kCutAhead * V::kThreads < V::kHash;
+constexpr bool holds_overshoot = V::kTab + 8 + V::kAhead * V::kCutThreads < V::kHash;
 static_assert(holds_overshoot<NarrowItem> && holds_overshoot<WideItem>, "add_rows' ids past the limit fit the hash");
+static_assert(kHaloTabMax <= 1024 && kHaloWideTabMax <= 1024, "a row's places fit its bit map");
 static_assert(kHaloSlicesPerItem == kPick, "the cut's maps have 8 states");
 
 static_assert(kHaloWideTabMax * 16 <= 0x3fff + 1, "a row's own offset fits the header's 14 bits");
 
 // What the kernels report.
-enum : uint32_t { kDoesNotFit = 1, kDisagree = 2 };
+enum : uint32_t { kDoesNotFit = 1 };
 struct BuildTotals {
     unsigned long long words;
     unsigned long long ids;
@@ -265,138 +272,218 @@ struct GroupSet {
         const uint2 g = group[at];
         return g.y + (uint32_t)__popc(g.x & ((1u << (id & 31u)) - 1u));
     }
-    __device__ __forceinline__ uint32_t find(int32_t group) const  // held
-    {
-        uint32_t h = bucket(group);
-        for (int probes = 0; probes < HASH / 2; probes++) {
-            const int2 k = key[h];
-            if (k.x == group) return 2 * h;
-            if (k.y == group) return 2 * h + 1;
-            h = (h + 1) & (HASH / 2 - 1);
-        }
-        return 0;  // not held: not reached
-    }
     __device__ __forceinline__ int32_t key_at(int k) const { return k & 1 ? key[k / 2].y : key[k / 2].x; }
     __device__ __forceinline__ void clear()
     {
-        for (int k = threadIdx.x; k < HASH; k += blockDim.x) {
-            if (!(k & 1)) key[k / 2] = make_int2(-1, -1);
-            group[k] = make_uint2(0, 0);
-        }
+        for (int k = threadIdx.x; k < HASH / 4; k += blockDim.x)
+            reinterpret_cast<int4*>(key)[k] = make_int4(-1, -1, -1, -1);
+        for (int k = threadIdx.x; k < HASH / 2; k += blockDim.x)
+            reinterpret_cast<uint4*>(group)[k] = make_uint4(0, 0, 0, 0);
     }
 };
 
-// Adds the ids of rows [r0, r1) -- the rows and their columns -- and counts
-// the new ones in *count, giving up once it is above `most`.  loc, if given,
-// gets for each entry its group's place | (id mod 32) << 11.  Whole CTA; each
-// thread has kAhead columns in flight, so up to kAhead ids per thread are added
-// past `most`: the hash holds them.
-template <int kAhead, int HASH>
-__device__ __forceinline__ void add_rows(GroupSet<HASH>& set, const uint32_t* __restrict__ row_off,
-                                         const int32_t* __restrict__ col, int64_t r0, int64_t r1, int* count,
-                                         int most, uint16_t* loc)
+// An item's rows by two at a time, a half-warp each: f(entry, column) for each
+// entry of rows [r0, r0 + rows), kAhead columns of a thread read ahead of its
+// calls, and after each such stretch the whole warp calls go_on(), which may
+// end it.  The same thread gets the same entries each time.
+template <int kAhead, class Each, class GoOn>
+__device__ __forceinline__ void each_entry(const RowSource& src, int64_t r0, int rows, Each f, GoOn go_on)
 {
-    const uint32_t e0 = row_off[r0], m = row_off[r1] - e0;
-    const uint32_t rows = (uint32_t)(r1 - r0), step = blockDim.x;
-    const int lane = threadIdx.x & 31;
-    uint32_t at;
-    for (uint32_t k0 = threadIdx.x & ~31u; k0 < rows; k0 += step) {
-        const bool fresh = k0 + lane < rows && set.add((int32_t)(r0 + k0 + lane), at);
-        const uint32_t b = __ballot_sync(0xffffffffu, fresh);
-        if (lane == 0 && b) atomicAdd(count, __popc(b));
-    }
-    for (uint32_t k0 = threadIdx.x & ~31u; k0 < m; k0 += kAhead * step) {
-        if (__any_sync(0xffffffffu, *(volatile int*)count > most)) return;
-        int32_t id[kAhead];
-#pragma unroll
-        for (int x = 0; x < kAhead; x++) {
-            const uint32_t k = k0 + x * step + lane;
-            id[x] = k < m ? col[e0 + k] : -1;
+    const int lane = threadIdx.x & 31, l = lane & 15;
+    for (int p = (threadIdx.x >> 5) * 2; p < rows; p += (blockDim.x >> 5) * 2) {
+        const int k = p + (lane >> 4);
+        const int64_t r = r0 + k;
+        uint32_t beg = 0, len = 0;
+        if (k < rows) {
+            beg = src.row_off[r];
+            len = src.row_off[r + 1] - beg;
         }
-        int news = 0;
+        const int32_t* __restrict__ row = src.row(r, beg);
+        const uint32_t longest = max(len, __shfl_xor_sync(0xffffffffu, len, 16));
+        for (uint32_t x0 = l; x0 < longest + l; x0 += 16 * kAhead) {
+            int32_t id[kAhead];
 #pragma unroll
-        for (int x = 0; x < kAhead; x++) {
-            if (id[x] >= 0) {
-                news += set.add(id[x], at) ? 1 : 0;
-                if (loc) loc[k0 + x * step + lane] = (uint16_t)(at | ((uint32_t)(id[x] & 31) << 11));
-            }
+            for (int x = 0; x < kAhead; x++) id[x] = x0 + 16 * x < len ? row[x0 + 16 * x] : -1;
+#pragma unroll
+            for (int x = 0; x < kAhead; x++)
+                if (id[x] >= 0) f(beg + x0 + 16 * x, id[x]);
+            if (!go_on()) return;
         }
-        news = __reduce_add_sync(0xffffffffu, news);
-        if (lane == 0 && news) atomicAdd(count, news);
     }
 }
 
-// Row lengths of an item ordered longest first, ties by row: rank of row k of m.
-__device__ __forceinline__ int length_rank(const uint32_t* len, int m, int k)
+// place[e] = f(place[e]), each thread for the entries that each_entry gives it.
+template <class F>
+__device__ __forceinline__ void place_slots(const uint32_t* __restrict__ row_off, int64_t r0, int rows,
+                                            uint16_t* place, F f)
 {
-    const uint32_t mine = len[k];
+    const int lane = threadIdx.x & 31, l = lane & 15;
+    for (int p = (threadIdx.x >> 5) * 2; p < rows; p += (blockDim.x >> 5) * 2) {
+        const int k = p + (lane >> 4);
+        if (k >= rows) continue;
+        const uint32_t beg = row_off[r0 + k], end = row_off[r0 + k + 1];
+        uint32_t e = beg + l;
+        for (; e + 48 < end; e += 64) {
+            uint32_t u[4];
+#pragma unroll
+            for (int x = 0; x < 4; x++) u[x] = place[e + 16 * x];
+#pragma unroll
+            for (int x = 0; x < 4; x++) place[e + 16 * x] = f(u[x]);
+        }
+        for (; e < end; e += 16) place[e] = f(place[e]);
+    }
+}
+
+// Adds the ids of rows [r0, r0 + rows) -- the rows and their columns -- and
+// counts the new ones in *count, giving up once it is above `most`.  own and
+// place get for each row and entry its group's place | (id mod 32) << 11.
+// Whole CTA.
+template <int kAhead, int HASH>
+__device__ __forceinline__ void add_rows(GroupSet<HASH>& set, const RowSource& src, int64_t r0, int rows, int* count,
+                                         int most, uint16_t* own, uint16_t* place)
+{
+    static_assert(HASH <= 2048, "a group's place fits 11 bits");
+    const int lane = threadIdx.x & 31;
+    uint32_t at;
+    if ((int)(threadIdx.x & ~31u) < rows) {  // at most 64 rows
+        const bool is = (int)threadIdx.x < rows;
+        const int32_t id = (int32_t)(r0 + threadIdx.x);
+        const bool fresh = is && set.add(id, at);
+        if (is) own[id] = (uint16_t)(at | ((uint32_t)(id & 31) << 11));
+        const uint32_t b = __ballot_sync(0xffffffffu, fresh);
+        if (lane == 0 && b) atomicAdd(count, __popc(b));
+    }
+    int news = 0;
+    each_entry<kAhead>(
+        src, r0, rows,
+        [&](uint32_t e, int32_t id) {
+            news += set.add(id, at) ? 1 : 0;
+            place[e] = (uint16_t)(at | ((uint32_t)(id & 31) << 11));
+        },
+        [&]() {
+            const int sum = __reduce_add_sync(0xffffffffu, news);
+            news = 0;
+            if (lane == 0 && sum) atomicAdd(count, sum);
+            return !__any_sync(0xffffffffu, *(volatile int*)count > most);
+        });
+}
+
+// Row lengths of an item ordered longest first, ties by row: rank of row k of
+// m.  key[x] = len << 6 | 63 - x, 0 past m, in whole fours.
+__device__ __forceinline__ uint32_t length_key(uint32_t len, int k) { return (len << 6) | (63u - (uint32_t)k); }
+__device__ __forceinline__ int length_rank(const uint32_t* key, int m, int k)
+{
+    const uint32_t mine = key[k];
     int rank = 0;
-    for (int x = 0; x < m; x++) rank += (len[x] > mine || (len[x] == mine && x < k)) ? 1 : 0;
+    for (int x = 0; x < m; x += 4) {
+        const uint4 y = *reinterpret_cast<const uint4*>(key + x);
+        rank += (y.x > mine) + (y.y > mine) + (y.z > mine) + (y.w > mine);
+    }
     return rank;
 }
 
 // One CTA per run: its items.  A run whose table fits is one item; else the
-// longest prefixes that fit, block by block.
+// longest prefixes that fit, block by block.  For an item from row r0 with
+// entries from e0: tab[e0 + r0 + k] the k-th id of its table, place[e] (of the
+// items' entries) and own[r] (of its rows) their places in it.
 template <class V>
-__global__ void __launch_bounds__(V::kThreads) cut_runs_kernel(const uint32_t* __restrict__ row_off,
-                                                              const int32_t* __restrict__ col, int64_t n,
-                                                              const int32_t* __restrict__ list,
-                                                              const uint8_t* __restrict__ run,
-                                                              CutItem* __restrict__ cut,
-                                                              uint8_t* __restrict__ cuts, BuildTotals* out)
+__global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src, int64_t n,
+                                                                 const int32_t* __restrict__ list,
+                                                                 const uint8_t* __restrict__ run,
+                                                                 CutItem* __restrict__ cut,
+                                                                 uint8_t* __restrict__ cuts, uint16_t* own,
+                                                                 uint16_t* place, int32_t* __restrict__ tab,
+                                                                 BuildTotals* out)
 {
-    __shared__ GroupSet<V::kHash> set;
-    __shared__ uint32_t len[8 * kPick];
-    __shared__ int count;
+    __shared__ __align__(16) GroupSet<V::kHash> set;
+    __shared__ __align__(16) uint32_t gkey[V::kTab + 4];  // the groups: id / 32 << 6 | ids in the set
+    __shared__ uint16_t gat[V::kTab];                     // their places in the hash
+    __shared__ __align__(16) uint32_t key[8 * kPick];
+    __shared__ int count, ngroups;
     __shared__ uint32_t words;
     if (out->flags) return;
     const uint32_t runs = out->runs;
+    const int tid = threadIdx.x;
+    auto add = [&](int64_t b0, int64_t b1) {
+        const int64_t r0 = 8 * b0;
+        add_rows<V::kAhead>(set, src, r0, (int)(min(8 * b1, n) - r0), &count, V::kTab, own, place);
+        __syncthreads();
+        return count;
+    };
+    auto reset = [&]() {
+        __syncthreads();
+        set.clear();
+        if (tid == 0) {
+            count = 0;
+            ngroups = 0;
+            words = 0;
+        }
+        __syncthreads();
+    };
     for (uint32_t r = blockIdx.x; r < runs; r += gridDim.x) {
         const int64_t b0 = list[r];
         const int nb = run[b0];
-        const int64_t b1 = b0 + nb;
         int from = 0;
         while (from < nb) {
             // all that is left at once; if that does not fit, block by block
-            int to = nb, ntab = 0;
-            for (int whole = 1; whole >= 0; whole--) {
-                __syncthreads();
-                set.clear();
-                if (threadIdx.x == 0) count = 0;
-                __syncthreads();
-                if (whole) {
-                    add_rows<V::kCutAhead>(set, row_off, col, 8 * (b0 + from), min(8 * b1, n), &count, V::kTab, nullptr);
+            int to = nb;
+            reset();
+            int ntab = add(b0 + from, b0 + nb);
+            if (ntab > V::kTab) {
+                reset();
+                for (to = from; to < nb; to++) {
+                    const int c = add(b0 + to, b0 + to + 1);
                     __syncthreads();
-                    ntab = count;
-                    if (ntab <= V::kTab) break;
-                } else {
-                    for (to = from; to < nb; to++) {
-                        add_rows<V::kCutAhead>(set, row_off, col, 8 * (b0 + to), min(8 * (b0 + to + 1), n), &count, V::kTab, nullptr);
-                        __syncthreads();
-                        const int c = count;
-                        __syncthreads();
-                        if (c > V::kTab) break;
-                        ntab = c;
-                    }
+                    if (c > V::kTab) break;
                 }
+                if (to == from) {  // one block's table is too large
+                    if (tid == 0) atomicOr(&out->flags, kDoesNotFit);
+                    return;
+                }
+                reset();
+                ntab = add(b0 + from, b0 + to);
             }
-            if (to == from) {  // one block's table is too large
-                if (threadIdx.x == 0) atomicOr(&out->flags, kDoesNotFit);
-                return;
-            }
-            // the item's words: slice j is as long as the row of rank 8 j
             const int64_t r0 = 8 * (b0 + from);
             const int m = (int)(min(8 * (b0 + to), n) - r0);
+            // the groups, and each one's first slot: the ids of those before it
+            for (int k = tid; k < V::kHash; k += V::kCutThreads) {
+                const int32_t g = set.key_at(k);
+                if (g != -1) {
+                    const int x = atomicAdd(&ngroups, 1);
+                    gkey[x] = ((uint32_t)g << 6) | (uint32_t)__popc(set.group[k].x);
+                    gat[x] = (uint16_t)k;
+                }
+            }
+            if (tid < 8 * kPick) key[tid] = tid < m ? length_key(src.row_off[r0 + tid + 1] - src.row_off[r0 + tid], tid) : 0u;
             __syncthreads();
-            if ((int)threadIdx.x < m) len[threadIdx.x] = row_off[r0 + threadIdx.x + 1] - row_off[r0 + threadIdx.x];
-            if (threadIdx.x == 0) words = 0;
+            const int groups = ngroups;
+            if (tid < 4) gkey[groups + tid] = 0xffffffffu;  // whole reads of four
+            // the item's words: slice j is as long as the row of rank 8 j
+            if (tid < m && (length_rank(key, m, tid) & 7) == 0) atomicAdd(&words, 32u * (((key[tid] >> 6) + 7u) / 8u + 1u));
             __syncthreads();
-            if ((int)threadIdx.x < m && (length_rank(len, m, threadIdx.x) & 7) == 0)
-                atomicAdd(&words, 32u * ((len[threadIdx.x] + 7u) / 8u + 1u));
+            const int64_t t0 = r0 + src.row_off[r0];
+            for (int k = tid; k < groups; k += V::kCutThreads) {
+                const uint32_t mine = gkey[k];
+                uint32_t slot = 0;
+                for (int x = 0; x < groups; x += 4) {
+                    const uint4 y = *reinterpret_cast<const uint4*>(gkey + x);
+                    slot += (y.x < mine ? y.x & 63u : 0u) + (y.y < mine ? y.y & 63u : 0u) +
+                            (y.z < mine ? y.z & 63u : 0u) + (y.w < mine ? y.w & 63u : 0u);
+                }
+                const uint32_t at = gat[k];
+                set.group[at].y = slot;
+                const int32_t id0 = (int32_t)(mine >> 6) << 5;
+                for (uint32_t b = set.group[at].x; b; b &= b - 1) tab[t0 + slot++] = id0 + __ffs(b) - 1;
+            }
             __syncthreads();
-            if (threadIdx.x == 0)
+            // places: each thread those that it wrote
+            auto slot_of = [&](uint32_t u) { return (uint16_t)set.slot(u & 2047u, u >> 11); };
+            if (tid < m) own[r0 + tid] = slot_of(own[r0 + tid]);
+            place_slots(src.row_off, r0, m, place, slot_of);
+            if (tid == 0) {
                 cut[b0 + from] = CutItem{(uint32_t)(to - from), (uint32_t)ntab, words};
-            if (threadIdx.x == 0) cuts[b0 + from] = 1;
+                cuts[b0 + from] = 1;
+            }
             from = to;
         }
     }
@@ -485,69 +572,119 @@ __global__ void __launch_bounds__(kPlaceThreads) place_items_kernel(int64_t n, i
     }
 }
 
-// One CTA per item: its sorted table into ids[tab0, tab0 + ntab), its slices'
-// offsets, and the words of its slices.
-template <class V>
-__global__ void __launch_bounds__(V::kThreads, V::kCtas) fill_items_kernel(
-    const uint32_t* __restrict__ row_off, const int32_t* __restrict__ col, int num_items,
-    const WorkItem* __restrict__ items, uint32_t* __restrict__ slice_off, int32_t* __restrict__ ids,
-    uint32_t* __restrict__ words, BuildTotals* out)
+// One warp: the row's places row[0, l) ordered by bank group (place mod 8),
+// each group ascending, and each group's first index into first[8].  A place is
+// a bit of a map, 32 words of up to 32 bits: 4 words per group, of 2^shift
+// places each.  bits: the warp's map, all zero before and after.  Rows that
+// name a node twice are sorted by a bitonic network (of exchanges in one
+// direction, so that any length can be padded with what is never moved).
+__device__ __forceinline__ void order_by_bank(uint16_t* row, uint32_t l, int shift, uint32_t* bits, uint16_t* first,
+                                              int lane)
 {
-    constexpr int kWarps = V::kThreads / 32;
-    constexpr int kEntries = 2 * V::kStream;  // every word of a step holds two entries
+    bool twice = false;
+    for (uint32_t k = lane; k < l; k += 32) {
+        const uint32_t sl = row[k], q = sl >> 3;
+        const uint32_t bit = 1u << (q & ((1u << shift) - 1u));
+        twice |= (atomicOr(bits + (((sl & 7u) << 2) | (q >> shift)), bit) & bit) != 0;
+    }
+    twice = __any_sync(0xffffffffu, twice);
+    __syncwarp();
+    const uint32_t mine = bits[lane];
+    bits[lane] = 0;
+    if (!twice) {
+        uint32_t sum = __popc(mine);
+#pragma unroll
+        for (int x = 1; x < 32; x <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, sum, x);
+            if (lane >= x) sum += y;
+        }
+        uint16_t* to = row + (sum - __popc(mine));
+        if (!(lane & 3)) first[lane >> 2] = (uint16_t)(sum - __popc(mine));
+        const uint32_t base = ((uint32_t)(lane & 3) << (shift + 3)) | ((uint32_t)lane >> 2);
+        for (uint32_t b = mine; b; b &= b - 1) *to++ = (uint16_t)(base + 8u * (uint32_t)(__ffs(b) - 1));
+        __syncwarp();
+        return;
+    }
+    auto order = [](uint32_t sl) { return ((sl & 7u) << 13) | (sl >> 3); };
+    auto exchange = [&](uint32_t a, uint32_t b) {  // a < b
+        const uint32_t x = row[a], y = row[b];
+        if (order(x) > order(y)) {
+            row[a] = (uint16_t)y;
+            row[b] = (uint16_t)x;
+        }
+    };
+    for (uint32_t size = 2; size < 2 * l; size <<= 1) {
+        for (uint32_t k = lane; k < l; k += 32) {
+            const uint32_t o = k ^ (size - 1);
+            if (o > k && o < l) exchange(k, o);
+        }
+        __syncwarp();
+        for (uint32_t stride = size >> 2; stride > 0; stride >>= 1) {
+            for (uint32_t k = lane; k < l; k += 32) {
+                const uint32_t o = k ^ stride;
+                if (o > k && o < l) exchange(k, o);
+            }
+            __syncwarp();
+        }
+    }
+    if (lane < 8) {
+        uint32_t lo = 0, hi = l;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if ((row[mid] & 7u) < (uint32_t)lane) lo = mid + 1;
+            else hi = mid;
+        }
+        first[lane] = (uint16_t)lo;
+    }
+    __syncwarp();
+}
+
+// One CTA per item: its table into ids[tab0, tab0 + ntab), its slices' offsets,
+// and the words of its slices.  A warp orders the places of its rows, then
+// picks for them, a thread per row, without waiting for the other warps; the
+// longest rows go to the first.
+template <class V>
+__global__ void __launch_bounds__(V::kFillWarps * 32, V::kFillCtas) fill_items_kernel(
+    const uint32_t* __restrict__ row_off, const uint16_t* __restrict__ own_place, const uint16_t* __restrict__ place,
+    const int32_t* __restrict__ tab, int num_items, const WorkItem* __restrict__ items,
+    uint32_t* __restrict__ slice_off, int32_t* __restrict__ ids, uint32_t* __restrict__ words)
+{
+    constexpr int kWarps = V::kFillWarps, kThreads = 32 * kWarps, kRows = 8 * kPick / kWarps;
+    static_assert(kRows <= 32, "a thread per row of the warp");
     extern __shared__ __align__(16) unsigned char dyn[];
-    // [kEntries] per row: its entries' groups (add_rows), then, in place, their
-    // slots bucketed by bank group
+    // the entries' places, 16-byte aligned as in memory (every word of a step
+    // holds two entries: at most 2 kStream of them), then ordered in place
     uint16_t* const rs = reinterpret_cast<uint16_t*>(dyn);
-    __shared__ GroupSet<V::kHash> set;
-    __shared__ __align__(16) int32_t gid[V::kHash];  // the groups, as collected
-    __shared__ uint16_t gat[V::kHash];          // their places
-    __shared__ uint16_t sorted[V::kHash];       // collected index of the k-th group
-    __shared__ uint32_t off[8 * kPick + 1];     // the rows' first entries, from the item's
-    __shared__ uint32_t len[8 * kPick];
+    __shared__ uint32_t off[8 * kPick + 1];     // the rows' first entries in rs
+    __shared__ __align__(16) uint32_t key[8 * kPick];
     __shared__ int order[8 * kPick];            // the item's rows, longest first
     __shared__ uint32_t at[kPick + 1];          // the slices' first words, from the item's
-    __shared__ uint16_t bucket[8 * kPick][8];   // a row's buckets: first places in rs
-    __shared__ uint32_t part[kWarps];
-    __shared__ int count;
+    __shared__ uint16_t bucket[8 * kPick][8];   // a row's bank groups: first places in its part of rs
+    __shared__ uint32_t bits[kWarps][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    bits[warp][lane] = 0;
     for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
         const WorkItem w = items[item];
         const int m = w.nrows, ns = (m + 7) / 8;
+        const int64_t e0 = row_off[w.row0], base = e0 & ~7ll;
         __syncthreads();
-        set.clear();
-        if (tid == 0) count = 0;
-        const uint32_t e0 = row_off[w.row0];
-        if (tid <= m) off[tid] = row_off[w.row0 + tid] - e0;
-        __syncthreads();
-        if (tid < m) len[tid] = off[tid + 1] - off[tid];
-        const bool fits = off[m] <= (uint32_t)kEntries;
-        if (fits) add_rows<4>(set, row_off, col, w.row0, (int64_t)w.row0 + m, &count, V::kTab, rs);
-        __syncthreads();
-        if (count != (int)w.ntab || !fits) {  // the cut and the fill disagree
-            if (tid == 0) atomicOr(&out->flags, kDisagree);
-            continue;
+        {
+            const int chunks = (int)((row_off[w.row0 + m] - base + 7) / 8);
+            const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(rs));
+            for (int k = tid; k < chunks; k += kThreads)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * k), "l"(place + base + 8 * k)
+                             : "memory");
         }
+        for (int k = tid; k <= m; k += kThreads) off[k] = (uint32_t)(row_off[w.row0 + k] - base);
+        for (int k = tid; k < 8 * kPick; k += kThreads)
+            key[k] = k < m ? length_key(row_off[w.row0 + k + 1] - row_off[w.row0 + k], k) : 0u;
+        for (uint32_t k = tid; k < w.ntab; k += kThreads) ids[(int64_t)w.tab0 + k] = tab[e0 + w.row0 + k];
         __syncthreads();
-        if (tid == 0) count = 0;
+        for (int k = tid; k < m; k += kThreads) order[length_rank(key, m, k)] = k;
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        // the groups, then in order (each counts the smaller ones), and each
-        // one's first slot
-        for (int k = tid; k < V::kHash; k += V::kThreads) {
-            const int32_t g = set.key_at(k);
-            if (g != -1) {
-                const int x = atomicAdd(&count, 1);
-                gid[x] = g;
-                gat[x] = (uint16_t)k;
-            }
-        }
-        if (tid < m) order[length_rank(len, m, tid)] = tid;
-        __syncthreads();
-        const int groups = count;
-        if (tid < 4) gid[groups + tid] = INT_MAX;  // whole reads of four (groups < kHash - 4: kTab is)
-        if (warp == kWarps - 1 && lane < 8) {
-            const uint32_t words_j = lane < ns ? 32u * ((len[order[8 * lane]] + 7u) / 8u + 1u) : 0u;
-            uint32_t sum = words_j;
+        if (lane < 8) {  // each warp for itself: the same values
+            uint32_t sum = lane < ns ? 32u * (((key[order[8 * lane]] >> 6) + 7u) / 8u + 1u) : 0u;
             for (int x = 1; x < 8; x <<= 1) {
                 const uint32_t y = __shfl_up_sync(0xffu, sum, x);
                 if (lane >= x) sum += y;
@@ -555,112 +692,18 @@ __global__ void __launch_bounds__(V::kThreads, V::kCtas) fill_items_kernel(
             if (lane == 0) at[0] = 0;
             if (lane < ns) at[lane + 1] = sum;
         }
-        __syncthreads();
-        for (int k = tid; k < groups; k += V::kThreads) {
-            const int32_t g = gid[k];
-            int rank = 0;
-            for (int x = 0; x < groups; x += 4) {
-                const int4 y = *reinterpret_cast<const int4*>(gid + x);
-                rank += (y.x < g) + (y.y < g) + (y.z < g) + (y.w < g);
-            }
-            sorted[rank] = (uint16_t)k;
+        const int shift = w.ntab <= 256 ? 3 : (w.ntab <= 512 ? 4 : 5);
+        for (int p = kRows * warp; p < min(m, kRows * (warp + 1)); p++) {
+            const int r = order[p];
+            order_by_bank(rs + off[r], off[r + 1] - off[r], shift, bits[warp], bucket[r], lane);
         }
-        __syncthreads();
-        uint32_t base = 0;
-        for (int k0 = 0; k0 < groups; k0 += V::kThreads) {
-            const int k = k0 + tid;
-            const int x0 = k < groups ? sorted[k] : 0;
-            const uint32_t place = gat[x0];
-            const uint32_t mask = k < groups ? set.group[place].x : 0u;
-            const uint32_t mine = __popc(mask);
-            uint32_t sum = mine;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, sum, o);
-                if (lane >= o) sum += y;
-            }
-            if (lane == 31) part[warp] = sum;
-            __syncthreads();
-            uint32_t slot = base + sum - mine;
-            for (int x = 0; x < warp; x++) slot += part[x];
-            for (int x = 0; x < kWarps; x++) base += part[x];
-            if (k < groups) {
-                set.group[place].y = slot;
-                const int32_t id0 = gid[x0] << 5;
-                for (uint32_t b = mask; b; b &= b - 1) ids[(int64_t)w.tab0 + slot++] = id0 + __ffs(b) - 1;
-            }
-            __syncthreads();
-        }
-        auto slot_of = [&](int32_t id) { return set.slot(set.find(id >> 5), (uint32_t)id); };
-        // one warp per row: its entries' slots bucketed by bank group, each
-        // bucket ascending (the row's columns are).  Lane g (mod 8) counts
-        // group g.  A row of up to kHeld * 32 entries stays in registers, each
-        // entry with its rank in its bucket, between counting and placing; a
-        // longer one reads its columns again.
-        for (int r = warp; r < m; r += kWarps) {
-            const uint32_t o = off[r], l = len[r];
-            uint32_t total = 0;
-            // rank of the lane's slot in its bucket; counts the buckets on
-            auto rank_of = [&](uint32_t sl, bool v) {
-                const uint32_t bv = __ballot_sync(0xffffffffu, v), b0 = __ballot_sync(0xffffffffu, sl & 1u),
-                               b1 = __ballot_sync(0xffffffffu, sl & 2u), b2 = __ballot_sync(0xffffffffu, sl & 4u);
-                const uint32_t peers = bv & (sl & 1u ? b0 : ~b0) & (sl & 2u ? b1 : ~b1) & (sl & 4u ? b2 : ~b2);
-                const uint32_t mine = bv & (lane & 1 ? b0 : ~b0) & (lane & 2 ? b1 : ~b1) & (lane & 4 ? b2 : ~b2);
-                const uint32_t before = __shfl_sync(0xffffffffu, total, sl & 7u);
-                total += __popc(mine);
-                return before + __popc(peers & ((1u << lane) - 1u));
-            };
-            auto starts_of = [&]() {  // of group (lane mod 8)
-                uint32_t sum = total;
-                for (int x = 1; x < 8; x <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, sum, x, 8);
-                    if ((lane & 7) >= x) sum += y;
-                }
-                const uint32_t start = o + sum - total;
-                if (lane < 8) bucket[r][lane] = (uint16_t)start;
-                return start;
-            };
-            if (l <= 32u * V::kHeld) {
-                uint32_t held[V::kHeld];  // slot | rank << 16
-#pragma unroll
-                for (int x = 0; x < V::kHeld; x++)
-                    if (32u * x < l) {
-                        const bool v = 32u * x + lane < l;
-                        const uint32_t e = v ? rs[o + 32 * x + lane] : 0u;
-                        const uint32_t sl = set.slot(e & 2047u, e >> 11);
-                        held[x] = sl | (rank_of(sl, v) << 16);
-                    }
-                const uint32_t start = starts_of();
-                __syncwarp();
-#pragma unroll
-                for (int x = 0; x < V::kHeld; x++)
-                    if (32u * x < l) {
-                        const uint32_t to = __shfl_sync(0xffffffffu, start, held[x] & 7u);
-                        if (32u * x + lane < l) rs[to + (held[x] >> 16)] = (uint16_t)held[x];
-                    }
-            } else {
-                const int32_t* __restrict__ row = col + e0 + o;
-                for (uint32_t k0 = 0; k0 < l; k0 += 32) {
-                    const bool v = k0 + lane < l;
-                    rank_of(v ? slot_of(row[k0 + lane]) : 0u, v);
-                }
-                const uint32_t start = starts_of();
-                total = 0;
-                __syncwarp();
-                for (uint32_t k0 = 0; k0 < l; k0 += 32) {
-                    const bool v = k0 + lane < l;
-                    const uint32_t sl = v ? slot_of(row[k0 + lane]) : 0u;
-                    const uint32_t rank = rank_of(sl, v);
-                    const uint32_t to = __shfl_sync(0xffffffffu, start, sl & 7u);
-                    if (v) rs[to + rank] = (uint16_t)sl;
-                }
-            }
-        }
-        __syncthreads();
-        if (tid < ns) slice_off[w.row0 / 8 + tid + 1] = w.ent0 + at[tid + 1];
+        __syncwarp();
+        for (int k = tid; k < ns; k += kThreads) slice_off[w.row0 / 8 + k + 1] = w.ent0 + at[k + 1];
         if (tid == 0 && w.row0 == 0) slice_off[0] = 0;
         // one thread per row position: the picks
-        if (tid < 8 * ns) {
-            const int j = tid / 8, i = tid & 7;
+        const int pos = kRows * warp + lane;
+        if (lane < kRows && pos < 8 * ns) {
+            const int j = pos / 8, i = pos & 7;
             const int T = (int)((at[j + 1] - at[j]) / 32) - 1;
             uint32_t* sw = words + w.ent0 + at[j];
             uint32_t own = 0;
@@ -676,17 +719,17 @@ __global__ void __launch_bounds__(V::kThreads, V::kCtas) fill_items_kernel(
             uint32_t o = 0;
 #pragma unroll
             for (int c = 0; c < 8; c++) st[c] = 0;
-            if (tid < m) {
-                const int lrow = order[tid];
-                const uint32_t l = len[lrow];
+            if (pos < m) {
+                const int lrow = order[pos];
+                const uint32_t l = key[lrow] >> 6;
                 o = off[lrow];
-                own = slot_of(w.row0 + lrow) * 16u;
+                own = own_place[w.row0 + lrow] * 16u;
                 hdr = own | (l << 14) | ((uint32_t)lrow << 24);
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
                     const uint32_t g = (c + p4) & 7u;
-                    const uint32_t a = bucket[lrow][g], b = g == 7u ? o + l : bucket[lrow][g + 1];
-                    st[c] = ((b - a) << 19) | ((7u - g) << 16) | (a - o);
+                    const uint32_t a = bucket[lrow][g], b = g == 7u ? l : bucket[lrow][g + 1];
+                    st[c] = ((b - a) << 19) | ((7u - g) << 16) | a;
                 }
             }
             const uint16_t* row = rs + o;
@@ -731,8 +774,9 @@ cudaError_t alloc_n(T** p, int64_t count, cudaStream_t s)
 }
 
 template <class V>
-cudaError_t build(const uint32_t* row_off, const int32_t* col, int64_t n, Staged* st, cudaStream_t s)
+cudaError_t build(const RowSource& src, int64_t n, int64_t m, Staged* st, cudaStream_t s)
 {
+    const uint32_t* row_off = src.row_off;
     const int64_t S = (n + 7) / 8;
     int dev = 0, sms = 0;
     IRR_CUDA_TRY(cudaGetDevice(&dev));
@@ -740,7 +784,8 @@ cudaError_t build(const uint32_t* row_off, const int32_t* col, int64_t n, Staged
     const int64_t tiles = (S + kRunTile - 1) / kRunTile;
     uint8_t *run = nullptr, *cuts = nullptr, *enter = nullptr;
     uint32_t* map = nullptr;
-    int32_t* list = nullptr;
+    int32_t *list = nullptr, *tab = nullptr;
+    uint16_t *own = nullptr, *place = nullptr;
     CutItem* cut = nullptr;
     Places* sums = nullptr;
     WorkItem* items = nullptr;
@@ -760,6 +805,9 @@ cudaError_t build(const uint32_t* row_off, const int32_t* col, int64_t n, Staged
         IRR_CUDA_TRY(alloc_n(&sums, kPlaceCtas, s));
         IRR_CUDA_TRY(alloc_n(&items, S, s));
         IRR_CUDA_TRY(alloc_n(&d_out, 1, s));
+        IRR_CUDA_TRY(alloc_n(&own, n, s));
+        IRR_CUDA_TRY(alloc_n(&place, m + 8, s));  // read in whole eights
+        IRR_CUDA_TRY(alloc_n(&tab, n + m, s));    // a table is at most its item's rows and entries
         IRR_CUDA_TRY(cudaMemsetAsync(d_out, 0, sizeof(BuildTotals), s));
         IRR_CUDA_TRY(cudaMemsetAsync(cuts, 0, (size_t)(S > 0 ? S : 1), s));
         if (S > 0) {
@@ -768,8 +816,8 @@ cudaError_t build(const uint32_t* row_off, const int32_t* col, int64_t n, Staged
             run_entries_kernel<<<1, 1024, 0, s>>>(map, tiles, enter);
             list_runs_kernel<<<(unsigned)std::min<int64_t>((tiles + 7) / 8, 8192), kRunTile, 0, s>>>(run, enter, S,
                                                                                                     list, d_out);
-            cut_runs_kernel<V><<<(unsigned)std::min<int64_t>(S, (int64_t)sms * 128), V::kThreads, 0, s>>>(
-                row_off, col, n, list, run, cut, cuts, d_out);
+            cut_runs_kernel<V><<<(unsigned)std::min<int64_t>(S, (int64_t)sms * 128), V::kCutThreads, 0, s>>>(
+                src, n, list, run, cut, cuts, own, place, tab, d_out);
             place_items_kernel<false><<<kPlaceCtas, kPlaceThreads, 0, s>>>(n, S, cut, cuts, sums, items, d_out);
             place_items_kernel<true><<<kPlaceCtas, kPlaceThreads, 0, s>>>(n, S, cut, cuts, sums, items, d_out);
             IRR_CUDA_TRY(cudaGetLastError());
@@ -787,20 +835,17 @@ cudaError_t build(const uint32_t* row_off, const int32_t* col, int64_t n, Staged
         IRR_CUDA_TRY(alloc_n(&out.items, out.nitems, s));
         if (S == 0) IRR_CUDA_TRY(cudaMemsetAsync(out.slice_off, 0, sizeof(uint32_t), s));
         if (got.items > 0) {
-            const int smem = 2 * V::kStream * (int)sizeof(uint16_t);
+            const int smem = (2 * V::kStream + 16) * (int)sizeof(uint16_t);
             IRR_CUDA_TRY(cudaMemcpyAsync(out.items, items, sizeof(WorkItem) * got.items, cudaMemcpyDeviceToDevice, s));
             IRR_CUDA_TRY(cudaFuncSetAttribute(fill_items_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            fill_items_kernel<V><<<(unsigned)std::min<int64_t>(got.items, (int64_t)sms * 128), V::kThreads, smem, s>>>(
-                row_off, col, (int)got.items, out.items, out.slice_off, out.ids, out.words, d_out);
+            fill_items_kernel<V><<<(unsigned)std::min<int64_t>(got.items, (int64_t)sms * 128), 32 * V::kFillWarps, smem, s>>>(
+                row_off, own, place, tab, (int)got.items, out.items, out.slice_off, out.ids, out.words);
             IRR_CUDA_TRY(cudaGetLastError());
-            IRR_CUDA_TRY(cudaMemcpyAsync(&got, d_out, sizeof(got), cudaMemcpyDeviceToHost, s));
-            IRR_CUDA_TRY(cudaStreamSynchronize(s));
-            if (got.flags) return cudaErrorInvalidValue;
         }
         return cudaSuccess;
     };
     const cudaError_t e = go();
-    void* tmp[] = {run, cuts, enter, map, list, cut, sums, items, d_out};
+    void* tmp[] = {run, cuts, enter, map, list, cut, sums, items, d_out, own, place, tab};
     for (void* p : tmp)
         if (p) cudaFreeAsync(p, s);
     if (e != cudaSuccess) {
@@ -824,11 +869,52 @@ void free_staged(Staged* st, cudaStream_t s)
     *st = Staged{};
 }
 
-cudaError_t build_staged(const uint32_t* row_off, const int32_t* col, int64_t n, bool wide, Staged* st,
-                         cudaStream_t s)
+cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, Staged* st, cudaStream_t s)
 {
     free_staged(st, s);
-    return wide ? build<WideItem>(row_off, col, n, st, s) : build<NarrowItem>(row_off, col, n, st, s);
+    return wide ? build<WideItem>(src, n, m, st, s) : build<NarrowItem>(src, n, m, st, s);
+}
+
+namespace {
+
+// One warp per slice of an item: its rows' ids to their places in col, in the
+// slice's order.  A row's picks come before its padding, so pick k of a row is
+// an entry for k < its length.
+__global__ void __launch_bounds__(32 * kPick) rows_of_items_kernel(const WorkItem* __restrict__ items, int num_items,
+                                                                  const uint32_t* __restrict__ slice_off,
+                                                                  const uint32_t* __restrict__ words,
+                                                                  const int32_t* __restrict__ ids,
+                                                                  const uint32_t* __restrict__ row_off,
+                                                                  int32_t* __restrict__ col)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+        const WorkItem w = items[item];
+        if (8 * warp >= w.nrows) continue;
+        const uint32_t o = slice_off[w.row0 / 8 + warp];
+        const uint32_t hdr = words[o + lane];
+        if (hdr >> 31) continue;  // a padding row
+        const uint32_t len = (hdr >> 14) & 1023u;
+        const int32_t* tab = ids + w.tab0;
+        int32_t* row = col + row_off[w.row0 + ((hdr >> 24) & 127u)];
+        for (uint32_t k = lane & 3; k < len; k += 8) {
+            const uint32_t pair = words[o + 32 * (k / 8 + 1) + lane];
+            row[k] = tab[(pair & 0xffffu) / 16];
+            if (k + 4 < len) row[k + 4] = tab[(pair >> 16) / 16];
+        }
+    }
+}
+
+}  // namespace
+
+cudaError_t rows_of_staged(const Staged& st, const WorkItem* items, const uint32_t* row_off, int64_t n, int32_t* col,
+                           cudaStream_t s)
+{
+    if (st.nitems <= 0) return cudaSuccess;
+    rows_of_items_kernel<<<(unsigned)std::min<int64_t>(st.nitems, 65536), 32 * kPick, 0, s>>>(
+        items, (int)st.nitems, st.slice_off, st.words, st.ids, row_off, col);
+    IRR_CUDA_TRY(cudaGetLastError());
+    return launch_row_sort(row_off, n, col, s);
 }
 
 cudaError_t staged_items_to_host(const WorkItem* d_items, int64_t count, std::vector<WorkItem>* items, cudaStream_t s)
