@@ -465,13 +465,17 @@ __global__ void fill_rows_kernel(const int2* edges, int64_t e, const int32_t* in
     }
 }
 
-// Directed entries of a list sorted by idx0 into slots of `cap` per row, one
-// warp per row in execution order: row a = execution id of node i takes i's
-// pairs as one stretch, and each partner b's row one entry.  In that order the
-// rows a warp writes are its curve neighbours', so the slots and counters stay
-// in L2 where edge-order writes went to memory (1M nodes, 64 neighbours: counting
-// 254 + filling 645 -> 539 us), and one pass counts and fills.  A row longer than
-// cap raises *over and the caller starts again the other way.
+// Directed entries of a list sorted by idx0 into slots of `cap` per row, in
+// execution order: row a = execution id of node i takes i's pairs as one stretch,
+// and each partner b's row one entry.  In that order the rows a warp writes are
+// its curve neighbours', so the slots and counters stay in L2 where edge-order
+// writes went to memory (1M nodes, 64 neighbours: counting 254 + filling 645 ->
+// 539 us), and one pass counts and fills.  What bounds it is the latency of its
+// chain (partner, its row, an atomic, the write): a warp takes 8 nodes' pairs as
+// one run, 4 per lane at a time (539 -> 363 us); more nodes at once would
+// spread the GPU's rows beyond L2.  A row longer than cap raises *over and the
+// caller starts again the other way.
+constexpr int kSlotNodes = 8, kSlotAhead = 4;
 __global__ void __launch_bounds__(256) slot_rows_kernel(const int2* __restrict__ edges,
                                                        const uint32_t* __restrict__ runs,
                                                        const int32_t* __restrict__ perm,
@@ -483,23 +487,55 @@ __global__ void __launch_bounds__(256) slot_rows_kernel(const int2* __restrict__
         return;
     }
     const int lane = threadIdx.x & 31;
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t a = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < n; a += warps) {
+    const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * kSlotNodes;
+    for (int64_t a0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSlotNodes; a0 < n; a0 += stride) {
         if (*(volatile int*)over) return;
-        const int32_t i = perm[a];
-        const uint32_t r0 = runs[i], r1 = runs[n + i];
-        if (r0 == r1) continue;
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(count + a, r1 - r0);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        bool full = r1 - r0 > cap || at > cap - (r1 - r0);
-        for (uint32_t k = r0 + lane; k < r1; k += 32) {
-            const int32_t b = inv[edges[k].y];
-            const uint32_t mine = at + (k - r0);
-            if (mine < cap) slots[a * (int64_t)cap + mine] = b;
-            const uint32_t theirs = atomicAdd(count + b, 1u);
-            if (theirs < cap) slots[b * (int64_t)cap + theirs] = (int32_t)a;
-            else full = true;
+        // lane t: node a0 + t, its pairs and the place of its stretch
+        uint32_t r0 = 0, len = 0, at = 0;
+        if (lane < kSlotNodes && a0 + lane < n) {
+            const int32_t i = perm[a0 + lane];
+            r0 = runs[i];
+            len = runs[n + i] - r0;
+            if (len) at = atomicAdd(count + a0 + lane, len);
+        }
+        bool full = len > cap || at > cap - len;
+        uint32_t end = len;  // of its pairs among the warp's
+#pragma unroll
+        for (int x = 1; x < kSlotNodes; x <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, end, x);
+            if (lane >= x) end += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, end, kSlotNodes - 1);
+        for (uint32_t f0 = 0; f0 < total; f0 += 32 * kSlotAhead) {
+            int32_t b[kSlotAhead], a[kSlotAhead];
+            uint32_t mine[kSlotAhead];
+#pragma unroll
+            for (int x = 0; x < kSlotAhead; x++) {
+                const uint32_t f = f0 + 32 * x + lane;
+                int t = 0;  // the nodes whose pairs end at or before f
+#pragma unroll
+                for (int half = kSlotNodes / 2; half > 0; half >>= 1)
+                    if (__shfl_sync(0xffffffffu, end, t + half - 1) <= f) t += half;
+                const uint32_t k = f - __shfl_sync(0xffffffffu, end - len, t);
+                mine[x] = __shfl_sync(0xffffffffu, at, t) + k;
+                const uint32_t src = __shfl_sync(0xffffffffu, r0, t) + k;
+                a[x] = t;
+                b[x] = f < total ? edges[src].y : -1;
+            }
+#pragma unroll
+            for (int x = 0; x < kSlotAhead; x++)
+                if (b[x] >= 0) b[x] = inv[b[x]];
+            uint32_t theirs[kSlotAhead];
+#pragma unroll
+            for (int x = 0; x < kSlotAhead; x++)
+                if (b[x] >= 0) theirs[x] = atomicAdd(count + b[x], 1u);
+#pragma unroll
+            for (int x = 0; x < kSlotAhead; x++)
+                if (b[x] >= 0) {
+                    if (mine[x] < cap) slots[(a0 + a[x]) * cap + mine[x]] = b[x];
+                    if (theirs[x] < cap) slots[b[x] * (int64_t)cap + theirs[x]] = (int32_t)(a0 + a[x]);
+                    else full = true;
+                }
         }
         if (full) *over = 1;
     }
@@ -918,7 +954,7 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
             out->cap = cap;
             IRR_CUDA_TRY(alloc_async(&over, 1, s));
             IRR_CUDA_TRY(cudaMemsetAsync(over, 0, sizeof(int), s));
-            slot_rows_kernel<<<grid_for(32 * n), 256, 0, s>>>(edges, runs, out->perm, out->inv, n, (uint32_t)cap, deg,
+            slot_rows_kernel<<<grid_for(32 * ((n + kSlotNodes - 1) / kSlotNodes)), 256, 0, s>>>(edges, runs, out->perm, out->inv, n, (uint32_t)cap, deg,
                                                              out->slots, over);
             IRR_CUDA_TRY(cudaGetLastError());
             int was_over = 0;
