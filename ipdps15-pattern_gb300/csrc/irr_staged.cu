@@ -49,7 +49,7 @@
 // ordered as bits of a 1,024-bit map.
 // What bounds it: instruction issue (a hash probe, a bit and a pick per entry).
 // 1,000,003 nodes at 64 neighbours: sorting the rows, counting the tables and
-// filling, a table gathered in both, 353 + 172 + 721 us; now 443 + 343, and the
+// filling, a table gathered in both, 353 + 172 + 721 us; now 350 + 343, and the
 // rows (4 bytes an entry) are made from the layout when they are asked for.
 #include <algorithm>
 #include <climits>
@@ -61,8 +61,8 @@ namespace irr {
 namespace {
 
 constexpr int kPick = 8;                         // slices of an item, blocks of a run: at most
-// The limits of the two variants.  kAhead: columns a thread has in flight while
-// it adds them to the table.
+// The limits of the two variants.  kAhead: columns that a thread adds to a table
+// between two looks at whether it is full (1, 2 or 4).
 struct NarrowItem {
     static constexpr int kTab = kHaloTabMax, kStream = kHaloStreamMax;
     static constexpr int kHash = 1024, kCutThreads = 128, kAhead = 2;
@@ -232,38 +232,51 @@ struct GroupSet {
     {
         return ((uint32_t)group * 2654435761u) >> (HASH == 1024 ? 23 : 22);
     }
-    // Adds id; true if it was new; at: the group's place.  At most HASH - 1
-    // groups may ever be held.
-    __device__ __forceinline__ bool add(int32_t id, uint32_t& at)
+    // Adds id; returns its group's place.  A new group is counted in *groups;
+    // at most HASH - 1 may ever be held.
+    __device__ __forceinline__ uint32_t add(int32_t id, int* groups)
     {
         const int32_t group = id >> 5;
+        const uint32_t h = bucket(group);
+        const int2 k = read(h);
+        uint32_t at = 2 * h + (k.x != group);
+        if (k.x != group && k.y != group) at = insert(group, h, groups);
+        uint32_t* const mask = &this->group[at].x;
         const uint32_t bit = 1u << (id & 31);
-        uint32_t h = bucket(group);
-        for (int probes = 0;; probes++) {
-            if (probes == HASH / 2) return false;  // full: not reached, see add_rows
-            int2 k;
-            asm volatile("ld.volatile.shared.v2.s32 {%0, %1}, [%2];"
-                         : "=r"(k.x), "=r"(k.y)
-                         : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&key[h]))));
-            at = 2 * h;
-            if (k.x == group) break;
-            at++;
-            if (k.y == group) break;
+        if (!(*(volatile uint32_t*)mask & bit)) atomicOr(mask, bit);
+        return at;
+    }
+    __device__ __forceinline__ int2 read(uint32_t h)
+    {
+        int2 k;
+        asm volatile("ld.volatile.shared.v2.s32 {%0, %1}, [%2];"
+                     : "=r"(k.x), "=r"(k.y)
+                     : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&key[h]))));
+        return k;
+    }
+    __device__ __forceinline__ uint32_t insert(int32_t group, uint32_t h, int* groups)
+    {
+        for (int probes = 0; probes < HASH / 2; probes++) {
+            int2 k = read(h);
             if (k.x == -1) {
                 k.x = atomicCAS(&key[h].x, -1, group);
-                at--;
-                if (k.x == -1 || k.x == group) break;
-                at++;
+                if (k.x == -1) {
+                    atomicAdd(groups, 1);
+                    return 2 * h;
+                }
             }
+            if (k.x == group) return 2 * h;
             if (k.y == -1) {
                 k.y = atomicCAS(&key[h].y, -1, group);
-                if (k.y == -1 || k.y == group) break;
+                if (k.y == -1) {
+                    atomicAdd(groups, 1);
+                    return 2 * h + 1;
+                }
             }
+            if (k.y == group) return 2 * h + 1;
             h = (h + 1) & (HASH / 2 - 1);
         }
-        uint32_t* const mask = &this->group[at].x;
-        if (*(volatile uint32_t*)mask & bit) return false;
-        return !(atomicOr(mask, bit) & bit);
+        return 0;  // full: not reached, see add_rows
     }
     // The slot of an id of the group at `at`: the group's first slot plus the
     // ids before it.
@@ -283,10 +296,9 @@ struct GroupSet {
 };
 
 // An item's rows by two at a time, a half-warp each: f(entry, column) for each
-// entry of rows [r0, r0 + rows), kAhead columns of a thread read ahead of its
-// calls, and after each such stretch the whole warp calls go_on(), which may
-// end it.  The same thread gets the same entries each time.
-template <int kAhead, class Each, class GoOn>
+// entry of rows [r0, r0 + rows), 4 columns of a thread read ahead, and after
+// each kStep of them the whole warp calls go_on(), which may end it.
+template <int kStep, class Each, class GoOn>
 __device__ __forceinline__ void each_entry(const RowSource& src, int64_t r0, int rows, Each f, GoOn go_on)
 {
     const int lane = threadIdx.x & 31, l = lane & 15;
@@ -300,14 +312,15 @@ __device__ __forceinline__ void each_entry(const RowSource& src, int64_t r0, int
         }
         const int32_t* __restrict__ row = src.row(r, beg);
         const uint32_t longest = max(len, __shfl_xor_sync(0xffffffffu, len, 16));
-        for (uint32_t x0 = l; x0 < longest + l; x0 += 16 * kAhead) {
-            int32_t id[kAhead];
+        for (uint32_t x0 = l; x0 < longest + l; x0 += 64) {
+            int32_t id[4];
 #pragma unroll
-            for (int x = 0; x < kAhead; x++) id[x] = x0 + 16 * x < len ? row[x0 + 16 * x] : -1;
+            for (int x = 0; x < 4; x++) id[x] = x0 + 16 * x < len ? row[x0 + 16 * x] : -1;
 #pragma unroll
-            for (int x = 0; x < kAhead; x++)
+            for (int x = 0; x < 4; x++) {
                 if (id[x] >= 0) f(beg + x0 + 16 * x, id[x]);
-            if (!go_on()) return;
+                if (x % kStep == kStep - 1 && !go_on()) return;
+            }
         }
     }
 }
@@ -334,38 +347,20 @@ __device__ __forceinline__ void place_slots(const uint32_t* __restrict__ row_off
     }
 }
 
-// Adds the ids of rows [r0, r0 + rows) -- the rows and their columns -- and
-// counts the new ones in *count, giving up once it is above `most`.  own and
-// place get for each row and entry its group's place | (id mod 32) << 11.
+// Adds the ids of rows [r0, r0 + rows) -- the rows and their columns --,
+// giving up once their groups (*groups) are more than `most` ids can be in.
+// own and place get for each row and entry its group's place | (id mod 32) << 11.
 // Whole CTA.
 template <int kAhead, int HASH>
-__device__ __forceinline__ void add_rows(GroupSet<HASH>& set, const RowSource& src, int64_t r0, int rows, int* count,
+__device__ __forceinline__ void add_rows(GroupSet<HASH>& set, const RowSource& src, int64_t r0, int rows, int* groups,
                                          int most, uint16_t* own, uint16_t* place)
 {
     static_assert(HASH <= 2048, "a group's place fits 11 bits");
-    const int lane = threadIdx.x & 31;
-    uint32_t at;
-    if ((int)(threadIdx.x & ~31u) < rows) {  // at most 64 rows
-        const bool is = (int)threadIdx.x < rows;
-        const int32_t id = (int32_t)(r0 + threadIdx.x);
-        const bool fresh = is && set.add(id, at);
-        if (is) own[id] = (uint16_t)(at | ((uint32_t)(id & 31) << 11));
-        const uint32_t b = __ballot_sync(0xffffffffu, fresh);
-        if (lane == 0 && b) atomicAdd(count, __popc(b));
-    }
-    int news = 0;
+    auto add = [&](int32_t id) { return (uint16_t)(set.add(id, groups) | ((uint32_t)(id & 31) << 11)); };
+    if ((int)threadIdx.x < rows) own[r0 + threadIdx.x] = add((int32_t)(r0 + threadIdx.x));  // at most 64 rows
     each_entry<kAhead>(
-        src, r0, rows,
-        [&](uint32_t e, int32_t id) {
-            news += set.add(id, at) ? 1 : 0;
-            place[e] = (uint16_t)(at | ((uint32_t)(id & 31) << 11));
-        },
-        [&]() {
-            const int sum = __reduce_add_sync(0xffffffffu, news);
-            news = 0;
-            if (lane == 0 && sum) atomicAdd(count, sum);
-            return !__any_sync(0xffffffffu, *(volatile int*)count > most);
-        });
+        src, r0, rows, [&](uint32_t e, int32_t id) { place[e] = add(id); },
+        [&]() { return !__any_sync(0xffffffffu, *(volatile int*)groups > most); });
 }
 
 // Row lengths of an item ordered longest first, ties by row: rank of row k of
@@ -399,26 +394,35 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
     __shared__ __align__(16) uint32_t gkey[V::kTab + 4];  // the groups: id / 32 << 6 | ids in the set
     __shared__ uint16_t gat[V::kTab];                     // their places in the hash
     __shared__ __align__(16) uint32_t key[8 * kPick];
-    __shared__ int count, ngroups;
+    __shared__ int held, ngroups;  // groups in the hash, and collected
+    __shared__ int count;          // ids
     __shared__ uint32_t words;
     if (out->flags) return;
     const uint32_t runs = out->runs;
     const int tid = threadIdx.x;
-    auto add = [&](int64_t b0, int64_t b1) {
-        const int64_t r0 = 8 * b0;
-        add_rows<V::kAhead>(set, src, r0, (int)(min(8 * b1, n) - r0), &count, V::kTab, own, place);
-        __syncthreads();
-        return count;
-    };
     auto reset = [&]() {
         __syncthreads();
         set.clear();
         if (tid == 0) {
-            count = 0;
+            held = 0;
             ngroups = 0;
+            count = 0;
             words = 0;
         }
         __syncthreads();
+    };
+    // blocks [b0, b1) added: the ids in the set now, kTab + 1 if more than kTab
+    auto add = [&](int64_t b0, int64_t b1) {
+        const int64_t r0 = 8 * b0;
+        add_rows<V::kAhead>(set, src, r0, (int)(min(8 * b1, n) - r0), &held, V::kTab, own, place);
+        __syncthreads();
+        if (held > V::kTab) return V::kTab + 1;
+        int ids = 0;
+        for (int k = tid; k < V::kHash; k += V::kCutThreads) ids += __popc(set.group[k].x);
+        ids = __reduce_add_sync(0xffffffffu, ids);
+        if ((tid & 31) == 0) atomicAdd(&count, ids);
+        __syncthreads();
+        return min(count, V::kTab + 1);
     };
     for (uint32_t r = blockIdx.x; r < runs; r += gridDim.x) {
         const int64_t b0 = list[r];
@@ -432,9 +436,9 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
             if (ntab > V::kTab) {
                 reset();
                 for (to = from; to < nb; to++) {
-                    const int c = add(b0 + to, b0 + to + 1);
+                    if (add(b0 + to, b0 + to + 1) > V::kTab) break;
                     __syncthreads();
-                    if (c > V::kTab) break;
+                    if (tid == 0) count = 0;  // counted whole after each block
                 }
                 if (to == from) {  // one block's table is too large
                     if (tid == 0) atomicOr(&out->flags, kDoesNotFit);
