@@ -54,14 +54,14 @@ int grid_of(int64_t n)
 // KICKS = 1: kick + drift of a step; KICKS = 2: also the closing kick of
 // the step before (the same forces).
 template <int KICKS>
-__global__ void kick_drift_kernel(double* __restrict__ x, double* __restrict__ v,
-                                  const float4* __restrict__ f, int64_t n, double dt, double L,
-                                  float4* __restrict__ pos4)
+__global__ void __launch_bounds__(256, 5)
+    kick_drift_kernel(double* __restrict__ x, double* __restrict__ v, const float4* __restrict__ f, int64_t n,
+                      double dt, double hk, double L, float Lf, float4* __restrict__ pos4)
 {
     grid_begin();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-        md_kick_drift_atom<KICKS>(x, v, f, i, dt, L, pos4);
+        md_kick_drift_atom<KICKS>(x, v, f, i, dt, hk, L, Lf, pos4);
 }
 
 // cnt[t] = entries of row t with a column above t (rows ascending: a suffix).
@@ -90,11 +90,11 @@ __global__ void half_write_kernel(const uint32_t* __restrict__ row_off, const in
 }
 
 __global__ void kick_kernel(double* __restrict__ v, const float4* __restrict__ f, int64_t n,
-                            double dt)
+                            double hk)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-        md_kick_atom(v, f, i, dt);
+        md_kick_atom(v, f, i, hk);
 }
 
 __global__ void to_float4_kernel(const double* __restrict__ x, int64_t n, double L,
@@ -401,7 +401,7 @@ int md_forces(irr_md* m)
 int md_kick_drift(irr_md* m)
 {
     MD_CUDA(m, launch_chained(kick_drift_kernel<1>, grid_of(m->n), 256, 0, m->stream, m->x, m->v, m->force,
-                              m->n, m->cfg.dt, m->cfg.side, m->pos4), "kick-drift");
+                              m->n, m->cfg.dt, md_half_kick(m->cfg.dt), m->cfg.side, (float)m->cfg.side, m->pos4), "kick-drift");
     m->since_rebuild++;
     return IRR_OK;
 }
@@ -410,7 +410,7 @@ int md_kick_drift(irr_md* m)
 int md_kick_kick_drift(irr_md* m)
 {
     MD_CUDA(m, launch_chained(kick_drift_kernel<2>, grid_of(m->n), 256, 0, m->stream, m->x, m->v, m->force,
-                              m->n, m->cfg.dt, m->cfg.side, m->pos4), "kick-drift");
+                              m->n, m->cfg.dt, md_half_kick(m->cfg.dt), m->cfg.side, (float)m->cfg.side, m->pos4), "kick-drift");
     m->steps++;
     m->since_rebuild++;
     return IRR_OK;
@@ -418,7 +418,7 @@ int md_kick_kick_drift(irr_md* m)
 
 int md_kick(irr_md* m)
 {
-    kick_kernel<<<grid_of(m->n), 256, 0, m->stream>>>(m->v, m->force, m->n, m->cfg.dt);
+    kick_kernel<<<grid_of(m->n), 256, 0, m->stream>>>(m->v, m->force, m->n, md_half_kick(m->cfg.dt));
     MD_CUDA(m, cudaGetLastError(), "kick");
     m->steps++;
     return IRR_OK;

@@ -133,25 +133,25 @@ __device__ __forceinline__ int find_job(int njobs, int64_t x, Start start)
 // Each job's kick-drift; a job that did not retire last tick had its closing
 // kick left to this pass (kicks == 2, the same roundings as a separate kick).
 __global__ void __launch_bounds__(kTickThreads) tick_kick_drift_kernel(const TickJob* __restrict__ jobs,
-                                                                       int njobs, double dt)
+                                                                       int njobs, double dt, double hk)
 {
     const int k = find_job(njobs, blockIdx.x, [&](int j) { return (int64_t)jobs[j].block0; });
     const TickJob& J = jobs[k];
     const int64_t i = (int64_t)(blockIdx.x - J.block0) * kTickThreads + threadIdx.x;
     if (i >= J.n) return;
     if (J.kicks == 2)
-        md_kick_drift_atom<2>(J.x, J.v, J.force, i, dt, J.side, J.pos4);
+        md_kick_drift_atom<2>(J.x, J.v, J.force, i, dt, hk, J.side, (float)J.side, J.pos4);
     else
-        md_kick_drift_atom<1>(J.x, J.v, J.force, i, dt, J.side, J.pos4);
+        md_kick_drift_atom<1>(J.x, J.v, J.force, i, dt, hk, J.side, (float)J.side, J.pos4);
 }
 
 __global__ void __launch_bounds__(kTickThreads) tick_kick_kernel(const TickJob* __restrict__ jobs,
-                                                                 int njobs, double dt)
+                                                                 int njobs, double hk)
 {
     const int k = find_job(njobs, blockIdx.x, [&](int j) { return (int64_t)jobs[j].block0; });
     const TickJob& J = jobs[k];
     const int64_t i = (int64_t)(blockIdx.x - J.block0) * kTickThreads + threadIdx.x;
-    if (i < J.n) md_kick_atom(J.v, J.force, i, dt);
+    if (i < J.n) md_kick_atom(J.v, J.force, i, hk);
 }
 
 // The batch's work items: job k's own items with the instance set to k.
@@ -294,7 +294,7 @@ int force_and_kick(const std::vector<irr_md*>& ms, const std::vector<irr_md*>& r
     int kblocks = 0;
     int64_t unused = 0;
     if (!upload_tick_jobs(retiring, B.closing, s, &kblocks, &unused)) return IRR_ERR_CUDA;
-    tick_kick_kernel<<<kblocks, kTickThreads, 0, s>>>(B.closing.d, (int)retiring.size(), dt);
+    tick_kick_kernel<<<kblocks, kTickThreads, 0, s>>>(B.closing.d, (int)retiring.size(), md_half_kick(dt));
     return cudaGetLastError() == cudaSuccess ? IRR_OK : IRR_ERR_CUDA;
 }
 
@@ -654,7 +654,7 @@ int irr_serve_run(const irr_serve_config* cfg, irr_serve_stats* st, irr_serve_jo
         int blocks = 0;
         int64_t nitems = 0;
         if (!upload_tick_jobs(all, tick_a, s, &blocks, &nitems, &kicks)) { rc = IRR_ERR_CUDA; break; }
-        tick_kick_drift_kernel<<<blocks, kTickThreads, 0, s>>>(tick_a.d, (int)all.size(), cfg->dt);
+        tick_kick_drift_kernel<<<blocks, kTickThreads, 0, s>>>(tick_a.d, (int)all.size(), cfg->dt, md_half_kick(cfg->dt));
         if (cudaGetLastError() != cudaSuccess) { rc = IRR_ERR_CUDA; break; }
         for (size_t k = 0; k < live.size(); k++) {
             irr_md* m = live[k].md;
