@@ -623,7 +623,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
         if (want == IRR_LAYOUT_CSR) {
             free_sliced(&h->sl);
         } else if (h->sl.lanes != lanes_per_row) {
-            const cudaError_t se = build_sliced(h->part.row_off, h->part.col, n, lanes_per_row, &h->sl, h->stream);
+            const cudaError_t se = build_sliced(RowSource{h->part.row_off, h->part.col, nullptr, 0}, n, lanes_per_row, &h->sl, h->stream);
             if (se != cudaSuccess) {
                 cudaGetLastError();
                 free_sliced(&h->sl);

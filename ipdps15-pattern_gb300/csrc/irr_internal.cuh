@@ -250,7 +250,7 @@ void make_instance_items(const uint32_t* host_row_off, const Sliced& sl, int64_t
 // Builds sl for G lanes per row from a CSR (row_off, col) of n rows on the
 // device; synchronises s (the host keeps the slice offsets).  Fails with
 // cudaErrorInvalidValue if the layout would exceed 2^32 - 1 words.
-cudaError_t build_sliced(const uint32_t* row_off, const int32_t* col, int64_t n, int G,
+cudaError_t build_sliced(const RowSource& rows, int64_t n, int G,
                          Sliced* sl, cudaStream_t s);
 // s != nullptr: stream-ordered frees on s (the arrays come from cudaMallocAsync).
 void free_sliced(Sliced* sl, cudaStream_t s = nullptr);
@@ -413,16 +413,18 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
                                 int2** d_edges, int64_t* num_edges, cudaStream_t s, bool sort_rows = true);
 // Full neighbour rows of a periodic box of at least 3 cells per axis (and no
 // more cells than nodes), for the MD rebuild: out->perm (new -> old) orders
-// the nodes by the Hilbert index of their cell, out->row_off / out->col hold
-// each node's partners j != i (rule of build_neighbor_list) in that order,
-// ascending; out->inv is not made.  *num_edges = pairs (entries / 2),
+// the nodes by the Hilbert index of their cell, out->row_off and out->col, or
+// out->slots, hold each node's partners j != i (rule of build_neighbor_list)
+// in that order, ascending; out->inv is not made.  *num_edges = pairs (entries / 2),
 // *longest = the longest row.  cap_hint > 0 (e.g. from the previous build's
 // longest row) lets one search pass write rows of up to cap_hint entries into
-// per-node slots, packed afterwards; 0, or a longer row, takes a counting and
-// a writing pass.  cudaErrorNotSupported, with nothing allocated, for other
+// per-node slots, where they stay; 0, or a longer row, takes a counting and a
+// writing pass, into out->col.  cudaErrorNotSupported, with nothing allocated, for other
 // boxes.
 cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cut2, PartitionOut* out,
                                int64_t* num_edges, uint32_t* longest, uint32_t cap_hint, cudaStream_t s);
+// p->col (m entries) from p->slots, in their order; the slots stay.
+cudaError_t pack_rows(PartitionOut* p, int64_t n, int64_t m, cudaStream_t s);
 // Sorts each row of a CSR (row_off[n + 1], col) ascending; every row must
 // hold at most kRowSortMax entries.
 constexpr int kRowSortMax = 1024;

@@ -65,27 +65,27 @@ __global__ void __launch_bounds__(256, 5)
 }
 
 // cnt[t] = entries of row t with a column above t (rows ascending: a suffix).
-__global__ void half_count_kernel(const uint32_t* __restrict__ row_off, const int32_t* __restrict__ col,
-                                  int64_t n, uint32_t* __restrict__ cnt)
+__global__ void half_count_kernel(const RowSource src, int64_t n, uint32_t* __restrict__ cnt)
 {
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = row_off[t], e = row_off[t + 1];
-        uint32_t k = b;
-        while (k < e && col[k] <= (int32_t)t) k++;
-        cnt[t] = e - k;
+        const uint32_t b = src.row_off[t], len = src.row_off[t + 1] - b;
+        const int32_t* row = src.row(t, b);
+        uint32_t k = 0;
+        while (k < len && row[k] <= (int32_t)t) k++;
+        cnt[t] = len - k;
     }
 }
 
 // half[off[t] ..] = (t, j) for the entries j > t of row t.
-__global__ void half_write_kernel(const uint32_t* __restrict__ row_off, const int32_t* __restrict__ col,
-                                  int64_t n, const uint32_t* __restrict__ off, int2* __restrict__ half)
+__global__ void half_write_kernel(const RowSource src, int64_t n, const uint32_t* __restrict__ off, int2* __restrict__ half)
 {
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t e = row_off[t + 1];
-        const uint32_t k0 = e - (off[t + 1] - off[t]);
-        for (uint32_t k = k0; k < e; k++) half[off[t] + (k - k0)] = make_int2((int)t, col[k]);
+        const uint32_t b = src.row_off[t], len = src.row_off[t + 1] - b;
+        const int32_t* row = src.row(t, b);
+        const uint32_t k0 = len - (off[t + 1] - off[t]);
+        for (uint32_t k = k0; k < len; k++) half[off[t] + (k - k0)] = make_int2((int)t, row[k]);
     }
 }
 
@@ -210,46 +210,35 @@ __global__ void kinetic_kernel(const double* __restrict__ v, int64_t n, double* 
     if (threadIdx.x == 0) part[3 * blockIdx.x] = 0.5 * s;
 }
 
+// One block: the partials' sums, each thread's share in order.
 __global__ void energy_final_kernel(const double* __restrict__ part, int blocks, double* acc)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double k = 0.0, p = 0.0, w = 0.0;
-    for (int b = 0; b < blocks; b++) {
-        k += part[3 * b];
-        p += part[3 * b + 1];
-        w += part[3 * b + 2];
+    __shared__ double red[32];
+    for (int c = 0; c < 3; c++) {
+        double sum = 0.0;
+        for (int b = threadIdx.x; b < blocks; b += blockDim.x) sum += part[3 * b + c];
+        sum = block_sum(sum, red);
+        if (threadIdx.x == 0) acc[c] = sum;
+        __syncthreads();
     }
-    acc[0] = k;
-    acc[1] = p;
-    acc[2] = w;
 }
 
-// Potential energy 4(r^-12 - r^-6) and virial r.F = 48 r^2 s over every
-// directed entry (each pair counted twice, halved), FP32 per entry, FP64 sums.
-__global__ void potential_kernel(const float4* __restrict__ pos, const uint32_t* __restrict__ row_off,
-                                 const int32_t* __restrict__ col, int64_t n, LawParams law,
-                                 double* part)
+// Potential energy 4(r^-12 - r^-6) and virial r.F = 48 r^2 s of one entry.
+__device__ __forceinline__ void add_entry(float4 a, float4 b, const LawParams& law, float& pe, float& vir)
+{
+    float dx, dy, dz;
+    const float s = lj_scalar<true>(a, b, law, dx, dy, dz);
+    if (s == 0.0f) return;
+    const float rd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    const float r = 1.0f / rd;
+    const float r6 = r * r * r;
+    pe += 4.0f * r6 * (r6 - 1.0f);
+    vir += 48.0f * s * rd;
+}
+
+__device__ __forceinline__ void energy_part(double pe, double vir, double* part)
 {
     __shared__ double red[32];
-    double pe = 0.0, vir = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 a = pos[i];
-        float pe_i = 0.f, vir_i = 0.f;
-        for (uint32_t k = row_off[i]; k < row_off[i + 1]; k++) {
-            const float4 b = pos[col[k]];
-            float dx, dy, dz;
-            const float s = lj_scalar<true>(a, b, law, dx, dy, dz);
-            if (s == 0.0f) continue;
-            const float rd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            const float r = 1.0f / rd;
-            const float r6 = r * r * r;
-            pe_i += 4.0f * r6 * (r6 - 1.0f);
-            vir_i += 48.0f * s * rd;
-        }
-        pe += 0.5 * (double)pe_i;
-        vir += 0.5 * (double)vir_i;
-    }
     pe = block_sum(pe, red);
     __syncthreads();
     vir = block_sum(vir, red);
@@ -257,6 +246,64 @@ __global__ void potential_kernel(const float4* __restrict__ pos, const uint32_t*
         part[3 * blockIdx.x + 1] = pe;
         part[3 * blockIdx.x + 2] = vir;
     }
+}
+
+// Over every directed entry (each pair counted twice, halved), FP32 per entry
+// and row, FP64 sums; the rows in CSR, one thread per row.
+__global__ void potential_kernel(const float4* __restrict__ pos, const uint32_t* __restrict__ row_off,
+                                 const int32_t* __restrict__ col, int64_t n, LawParams law,
+                                 double* part)
+{
+    double pe = 0.0, vir = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const float4 a = pos[i];
+        float pe_i = 0.f, vir_i = 0.f;
+        for (uint32_t k = row_off[i]; k < row_off[i + 1]; k++) add_entry(a, pos[col[k]], law, pe_i, vir_i);
+        pe += 0.5 * (double)pe_i;
+        vir += 0.5 * (double)vir_i;
+    }
+    energy_part(pe, vir, part);
+}
+
+// The same over slices of 8 rows, 4 lanes per row as the force kernel reads
+// them: whole 256-byte steps where a thread per row read lines of its own.  A
+// warp takes 4 slices, so that each lane has one row's FP32 sums to add in FP64
+// (whose rate would bound it else).
+__global__ void potential_slices_kernel(const float4* __restrict__ pos, const uint32_t* __restrict__ row_off,
+                                        const uint32_t* __restrict__ slice_off, const int32_t* __restrict__ scol,
+                                        int64_t n, int64_t slices, LawParams law, double* part)
+{
+    const int lane = threadIdx.x & 31, l = lane & 3;
+    double pe = 0.0, vir = 0.0;
+    const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * 4;
+    for (int64_t q0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; q0 < slices; q0 += stride) {
+        float pe_row = 0.f, vir_row = 0.f;
+        for (int j = 0; j < 4 && q0 + j < slices; j++) {
+            const int64_t r = 8 * (q0 + j) + (lane >> 2);
+            const uint32_t o = slice_off[q0 + j], steps = (slice_off[q0 + j + 1] - o) >> 6;
+            const uint32_t len = r < n ? row_off[r + 1] - row_off[r] : 0u;
+            const float4 a = pos[r < n ? r : 0];
+            const int2* line = reinterpret_cast<const int2*>(scol + o) + lane;
+            float pe_l = 0.f, vir_l = 0.f;
+            for (uint32_t t = 0; t < steps; t++) {
+                const int2 e = line[32 * t];
+                if (8 * t + l < len) add_entry(a, pos[e.x], law, pe_l, vir_l);
+                if (8 * t + 4 + l < len) add_entry(a, pos[e.y], law, pe_l, vir_l);
+            }
+            for (int x = 1; x < 4; x <<= 1) {
+                pe_l += __shfl_xor_sync(0xffffffffu, pe_l, x);
+                vir_l += __shfl_xor_sync(0xffffffffu, vir_l, x);
+            }
+            if (l == j) {
+                pe_row = pe_l;
+                vir_row = vir_l;
+            }
+        }
+        pe += 0.5 * (double)pe_row;
+        vir += 0.5 * (double)vir_row;
+    }
+    energy_part(pe, vir, part);
 }
 
 // Stream-ordered frees (on s): no device-wide synchronisation, so the set-up
@@ -268,6 +315,7 @@ void free_part(irr_md* m, cudaStream_t s)
     if (m->part.inv) cudaFreeAsync(m->part.inv, s);
     if (m->part.row_off) cudaFreeAsync(m->part.row_off, s);
     if (m->part.col) cudaFreeAsync(m->part.col, s);
+    if (m->part.slots) cudaFreeAsync(m->part.slots, s);
     m->part = PartitionOut{};
     free_sliced(&m->sl, s);
     if (m->d_items) cudaFreeAsync(m->d_items, s);
@@ -336,7 +384,8 @@ int md_rebuild(irr_md* m)
     // the sliced layout's work items are cut from its slice offsets (which
     // build_sliced brings to the host); only the CSR fallback needs the row
     // offsets on the host
-    if (build_sliced(m->part.row_off, m->part.col, m->n, m->shape.lanes_per_row, &m->sl, s) != cudaSuccess) {
+    const RowSource rows{m->part.row_off, m->part.col, m->part.slots, m->part.cap};
+    if (build_sliced(rows, m->n, m->shape.lanes_per_row, &m->sl, s) != cudaSuccess) {
         cudaGetLastError();
         free_sliced(&m->sl, s);  // CSR
     } else if (!sliced_pays(m->sl, 2 * e)) {
@@ -344,6 +393,7 @@ int md_rebuild(irr_md* m)
     }
     std::vector<uint32_t> ro;
     if (!m->sl.lanes) {
+        MD_CUDA(m, pack_rows(&m->part, m->n, 2 * e, s), "neighbour rows");
         ro.resize((size_t)m->n + 1);
         MD_CUDA(m, cudaMemcpyAsync(ro.data(), m->part.row_off, sizeof(uint32_t) * (m->n + 1),
                                    cudaMemcpyDeviceToHost, s), "row offsets");
@@ -373,13 +423,15 @@ int md_rebuild(irr_md* m)
         uint32_t* off = nullptr;
         MD_CUDA(m, irr_malloc_async(&off, sizeof(uint32_t) * (m->n + 1), s), "half list");
         MD_CUDA(m, irr_malloc_async(&m->half, sizeof(int2) * e, s), "half list");
-        half_count_kernel<<<grid_of(m->n), 256, 0, s>>>(m->part.row_off, m->part.col, m->n, off);
+        half_count_kernel<<<grid_of(m->n), 256, 0, s>>>(rows, m->n, off);
         MD_CUDA(m, cudaMemsetAsync(off + m->n, 0, sizeof(uint32_t), s), "half list");
         MD_CUDA(m, scan_exclusive_u32(off, off, m->n + 1, nullptr, s), "half list");
-        half_write_kernel<<<grid_of(m->n), 256, 0, s>>>(m->part.row_off, m->part.col, m->n, off, m->half);
+        half_write_kernel<<<grid_of(m->n), 256, 0, s>>>(rows, m->n, off, m->half);
         MD_CUDA(m, cudaGetLastError(), "half list");
         cudaFreeAsync(off, s);
     }
+    if (m->part.slots) cudaFreeAsync(m->part.slots, s);  // the slices, or col, hold the rows now
+    m->part.slots = nullptr;
     MD_CUDA(m, cudaStreamSynchronize(s), "rebuild");
     m->edges = e;
     m->rebuilds++;
@@ -607,9 +659,13 @@ int irr_md_energy(irr_md* m, double* kinetic, double* potential, double* virial)
     const int blocks = grid_of(m->n) < kEnergyBlocks ? grid_of(m->n) : kEnergyBlocks;
     double* part = m->d_acc + 4;
     kinetic_kernel<<<blocks, 256, 0, m->stream>>>(m->v, m->n, part);
-    potential_kernel<<<blocks, 256, 0, m->stream>>>(m->pos4, m->part.row_off, m->part.col, m->n,
-                                                    m->law, part);
-    energy_final_kernel<<<1, 32, 0, m->stream>>>(part, blocks, m->d_acc);
+    if (m->sl.lanes == 4)
+        potential_slices_kernel<<<blocks, 256, 0, m->stream>>>(m->pos4, m->part.row_off, m->sl.slice_off, m->sl.col, m->n,
+                                                               m->sl.slices, m->law, part);
+    else
+        potential_kernel<<<blocks, 256, 0, m->stream>>>(m->pos4, m->part.row_off, m->part.col, m->n,
+                                                        m->law, part);
+    energy_final_kernel<<<1, 256, 0, m->stream>>>(part, blocks, m->d_acc);
     MD_CUDA(m, cudaGetLastError(), "energy kernels");
     double h[4];
     int st = 0;

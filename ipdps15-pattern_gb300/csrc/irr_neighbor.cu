@@ -552,6 +552,54 @@ __device__ __forceinline__ void cell_rows_body(const float4* __restrict__ pos_c,
     }
 }
 
+// The same with L lanes per node: a run's candidates L at a time, the hits of
+// a step placed by a ballot, so in the same order.
+template <int MODE, bool FAST, int L>
+__device__ __forceinline__ void cell_rows_lanes(const float4* __restrict__ pos_c, int64_t n, const Grid& g,
+                                                const int4* __restrict__ table, uint32_t* deg,
+                                                const uint32_t* __restrict__ row_off, int32_t* col, uint32_t cap)
+{
+    const int lane = threadIdx.x & 31, l = lane % L, first = lane - l;
+    const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * (32 / L);
+    for (int64_t t0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 / L); t0 < n; t0 += stride) {
+        const bool is = t0 + lane / L < n;
+        const int64_t t = is ? t0 + lane / L : n - 1;
+        const float4 a = pos_c[t];
+        const int4* st = table + (int64_t)cell_of(a, g) * 27;
+        int32_t* out = MODE == kWrite ? col + row_off[t] : (MODE == kScratch ? col + t * (int64_t)cap : nullptr);
+        uint32_t m = 0;
+        int4 e = st[0];
+        for (int k = 0; k < 27; k++) {
+            const int4 next = st[k < 26 ? k + 1 : k];
+            const int count = is ? e.y - e.x : 0;
+            const int most = __reduce_max_sync(0xffffffffu, count);
+            const float sx = image_shift(e.z & 3, g.box), sy = image_shift((e.z >> 2) & 3, g.box),
+                        sz = image_shift((e.z >> 4) & 3, g.box);
+            for (int x0 = 0; x0 < most; x0 += 4 * L) {  // 4 of a lane's candidates in flight
+                float4 b[4];
+#pragma unroll
+                for (int y = 0; y < 4; y++) {
+                    const int x = x0 + y * L + l;
+                    b[y] = pos_c[x < count ? (int64_t)e.x + x : t];
+                }
+#pragma unroll
+                for (int y = 0; y < 4; y++) {
+                    if (x0 + y * L >= most) break;
+                    const int x = x0 + y * L + l;
+                    const int64_t q = x < count ? (int64_t)e.x + x : t;
+                    const bool hit = pair_hit<FAST>(a, b[y], g, sx, sy, sz) && q != t;
+                    const uint32_t hits = (__ballot_sync(0xffffffffu, hit) >> first) & ((1u << L) - 1u);
+                    const uint32_t at = m + (uint32_t)__popc(hits & ((1u << l) - 1u));
+                    if (MODE != kCount && hit && (MODE == kWrite || at < cap)) out[at] = (int32_t)q;
+                    m += (uint32_t)__popc(hits);
+                }
+            }
+            e = next;
+        }
+        if (MODE != kWrite && is && l == 0) deg[t] = m;
+    }
+}
+
 // Scratch rows (cap apart) packed into col at row_off: one warp per row.
 __global__ void compact_rows_kernel(const int32_t* __restrict__ scratch, uint32_t cap,
                                     const uint32_t* __restrict__ row_off, int64_t n, int32_t* __restrict__ col)
@@ -586,16 +634,20 @@ __global__ void sum_u32_kernel(const uint32_t* __restrict__ deg, int64_t n, unsi
     }
 }
 
-template <int MODE>
+template <int MODE, int L>
 __global__ void cell_rows_kernel(const float4* __restrict__ pos_c, int64_t n, const __grid_constant__ Grid g,
                                  const int* __restrict__ outside, const int4* __restrict__ table,
                                  uint32_t* deg, const uint32_t* __restrict__ row_off, int32_t* col,
                                  uint32_t cap)
 {
-    if (g.fast && *outside == 0)
-        cell_rows_body<MODE, true>(pos_c, n, g, table, deg, row_off, col, cap);
-    else
-        cell_rows_body<MODE, false>(pos_c, n, g, table, deg, row_off, col, cap);
+    const bool fast = g.fast && *outside == 0;
+    if constexpr (L > 1) {
+        if (fast) cell_rows_lanes<MODE, true, L>(pos_c, n, g, table, deg, row_off, col, cap);
+        else cell_rows_lanes<MODE, false, L>(pos_c, n, g, table, deg, row_off, col, cap);
+    } else {
+        if (fast) cell_rows_body<MODE, true>(pos_c, n, g, table, deg, row_off, col, cap);
+        else cell_rows_body<MODE, false>(pos_c, n, g, table, deg, row_off, col, cap);
+    }
 }
 
 int grid_of(int64_t n)
@@ -813,6 +865,21 @@ struct Temps {
     }
 };
 
+// Where the nodes are too few warps to hide the search's latency, 8 lanes share
+// a node's candidates: a search 189 -> 35 us at 2,048 nodes, 115 -> 65 at 32,000,
+// 106 -> 94 at 55,296; 120 -> 143 at 87,808, where instructions bound it.
+constexpr int64_t kLanesNodes = 65536;
+
+template <int MODE>
+void launch_cell_rows(const float4* pos_c, int64_t n, const Grid& g, const int* outside, const int4* table,
+                      uint32_t* deg, const uint32_t* row_off, int32_t* col, uint32_t cap, cudaStream_t s)
+{
+    if (n <= kLanesNodes)
+        cell_rows_kernel<MODE, 8><<<grid_of(8 * n), 256, 0, s>>>(pos_c, n, g, outside, table, deg, row_off, col, cap);
+    else
+        cell_rows_kernel<MODE, 1><<<grid_of(n), 256, 0, s>>>(pos_c, n, g, outside, table, deg, row_off, col, cap);
+}
+
 }  // namespace
 
 cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cut2, PartitionOut* out,
@@ -828,7 +895,7 @@ cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cu
     if (g.nc[0] < 3 || g.nc[1] < 3 || g.nc[2] < 3 || ncell > n) return cudaErrorNotSupported;
     Temps tmp{s, {}};
     uint32_t *keys = nullptr, *keys_tmp = nullptr;
-    int32_t *vals_tmp = nullptr, *scratch = nullptr;
+    int32_t* vals_tmp = nullptr;
     float4* pos_c = nullptr;
     uint2* span = nullptr;
     int4* table = nullptr;
@@ -848,8 +915,12 @@ cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cu
         // otherwise (and at the first build) a counting pass, then the writing one
         bool one_pass = false;
         if (cap_hint > 0 && cap_hint <= 4096) {
-            one_pass = tmp.get(&scratch, (size_t)n * cap_hint) == cudaSuccess;
-            if (!one_pass) cudaGetLastError();
+            one_pass = irr_malloc_async((void**)&p.slots, sizeof(int32_t) * (size_t)n * cap_hint, s) == cudaSuccess;
+            p.cap = cap_hint;
+            if (!one_pass) {
+                cudaGetLastError();
+                p.slots = nullptr;
+            }
         }
         IRR_CUDA_TRY(cudaMemsetAsync(span, 0, sizeof(uint2) * ncell, s));
         IRR_CUDA_TRY(cudaMemsetAsync(aux, 0, 3 * sizeof(unsigned long long), s));
@@ -857,16 +928,18 @@ cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cu
         const int gn = grid_of(n);
         cell_curve_keys_kernel<<<gn, 256, 0, s>>>(pos, n, g, keys, p.perm, outside);
         IRR_CUDA_TRY(cudaGetLastError());
-        IRR_CUDA_TRY(radix_sort_pairs(keys, p.perm, keys_tmp, vals_tmp, n, 30, s));
+        // coordinates below 2^b give curve indices below 8^b: the levels above
+        // only exchange axes
+        int bits = 0;
+        while ((1 << bits) < std::max(g.nc[0], std::max(g.nc[1], g.nc[2]))) bits++;
+        IRR_CUDA_TRY(radix_sort_pairs(keys, p.perm, keys_tmp, vals_tmp, n, 3 * bits, s));
         cell_order_kernel<<<gn, 256, 0, s>>>(pos, p.perm, n, pos_c);
         cell_spans_kernel<<<gn, 256, 0, s>>>(pos_c, keys, n, g, span);
         cell_stencil_kernel<<<grid_of(32 * ncell), 256, 0, s>>>(g, span, ncell, table);
         if (one_pass)
-            cell_rows_kernel<kScratch><<<gn, 256, 0, s>>>(pos_c, n, g, outside, table, p.row_off, nullptr,
-                                                          scratch, cap_hint);
+            launch_cell_rows<kScratch>(pos_c, n, g, outside, table, p.row_off, nullptr, p.slots, cap_hint, s);
         else
-            cell_rows_kernel<kCount><<<gn, 256, 0, s>>>(pos_c, n, g, outside, table, p.row_off, nullptr,
-                                                        nullptr, 0);
+            launch_cell_rows<kCount>(pos_c, n, g, outside, table, p.row_off, nullptr, nullptr, 0, s);
         sum_u32_kernel<<<gn < 256 ? gn : 256, 256, 0, s>>>(p.row_off, n, aux);  // few atomics
         IRR_CUDA_TRY(cudaGetLastError());
         unsigned long long host_aux[2] = {0, 0};
@@ -876,14 +949,13 @@ cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cu
         if (total > 0x7fffffffull) return cudaErrorInvalidValue;
         IRR_CUDA_TRY(cudaMemsetAsync(p.row_off + n, 0, sizeof(uint32_t), s));
         IRR_CUDA_TRY(scan_exclusive_u32(p.row_off, p.row_off, n + 1, nullptr, s));
-        // + kColPad: bulk copies of an entry segment may read past the last one
-        IRR_CUDA_TRY(irr_malloc_async((void**)&p.col, sizeof(int32_t) * (total + kColPad), s));
-        IRR_CUDA_TRY(cudaMemsetAsync(p.col + total, 0, sizeof(int32_t) * kColPad, s));
-        if (one_pass && host_aux[1] <= cap_hint)
-            compact_rows_kernel<<<grid_of(32 * n), 256, 0, s>>>(scratch, cap_hint, p.row_off, n, p.col);
-        else  // a row longer than the slots (or no scratch): search again, writing in place
-            cell_rows_kernel<kWrite><<<gn, 256, 0, s>>>(pos_c, n, g, outside, table, nullptr, p.row_off,
-                                                        p.col, 0);
+        if (!one_pass || host_aux[1] > cap_hint) {
+            // a row longer than the slots (or no scratch): search again, writing in place
+            if (p.slots) cudaFreeAsync(p.slots, s);
+            p.slots = nullptr;
+            IRR_CUDA_TRY(alloc_col(&p.col, (int64_t)total, s));
+            launch_cell_rows<kWrite>(pos_c, n, g, outside, table, nullptr, p.row_off, p.col, 0, s);
+        }
         IRR_CUDA_TRY(cudaGetLastError());
         *num_edges = (int64_t)(total / 2);
         *longest = (uint32_t)host_aux[1];
@@ -894,12 +966,21 @@ cudaError_t build_rows_by_cell(const float4* pos, int64_t n, float box, float cu
         if (p.perm) cudaFreeAsync(p.perm, s);
         if (p.row_off) cudaFreeAsync(p.row_off, s);
         if (p.col) cudaFreeAsync(p.col, s);
+        if (p.slots) cudaFreeAsync(p.slots, s);
         *num_edges = 0;
         *longest = 0;
         return e;
     }
     *out = p;
     return cudaSuccess;
+}
+
+cudaError_t pack_rows(PartitionOut* p, int64_t n, int64_t m, cudaStream_t s)
+{
+    if (!p->slots) return cudaSuccess;
+    IRR_CUDA_TRY(alloc_col(&p->col, m, s));
+    compact_rows_kernel<<<grid_of(32 * n), 256, 0, s>>>(p->slots, (uint32_t)p->cap, p->row_off, n, p->col);
+    return cudaGetLastError();
 }
 
 }  // namespace irr

@@ -734,7 +734,7 @@ __global__ void slice_words_kernel(const uint32_t* row_off, int64_t n, int G, in
 // power of two: lg = log2 G).  A padding word holds the row's own id (0 for a
 // row past n), so the kernel's gathers need no predicate: a padded slot reads
 // its own position, d = 0, and is masked to 0.
-__global__ void slice_fill_kernel(const uint32_t* row_off, const int32_t* col, int64_t n, int lg,
+__global__ void slice_fill_kernel(const RowSource src, int64_t n, int lg,
                                   int64_t slices, const uint32_t* slice_off, int32_t* out)
 {
     const int G = 1 << lg;
@@ -745,13 +745,14 @@ __global__ void slice_fill_kernel(const uint32_t* row_off, const int32_t* col, i
         const int64_t r = (q << (5 - lg)) + i;
         const uint32_t o = slice_off[q];
         const uint32_t steps = (slice_off[q + 1] - o) >> 6;
-        const uint32_t beg = r < n ? row_off[r] : 0u;
-        const uint32_t len = r < n ? row_off[r + 1] - beg : 0u;
+        const uint32_t beg = r < n ? src.row_off[r] : 0u;
+        const uint32_t len = r < n ? src.row_off[r + 1] - beg : 0u;
+        const int32_t* __restrict__ row = src.row(r, beg);
         const int32_t pad = r < n ? (int32_t)r : 0;
         int2* line = reinterpret_cast<int2*>(out + o) + lane;
         for (uint32_t t = 0; t < steps; t++) {
             const uint32_t k0 = (t << (lg + 1)) + l, k1 = k0 + G;
-            line[32 * t] = make_int2(k0 < len ? col[beg + k0] : pad, k1 < len ? col[beg + k1] : pad);
+            line[32 * t] = make_int2(k0 < len ? row[k0] : pad, k1 < len ? row[k1] : pad);
         }
     }
 }
@@ -1084,7 +1085,7 @@ cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_
     return cudaSuccess;
 }
 
-cudaError_t build_sliced(const uint32_t* row_off, const int32_t* col, int64_t n, int G,
+cudaError_t build_sliced(const RowSource& rows, int64_t n, int G,
                          Sliced* sl, cudaStream_t s)
 {
     free_sliced(sl);
@@ -1100,7 +1101,7 @@ cudaError_t build_sliced(const uint32_t* row_off, const int32_t* col, int64_t n,
     IRR_CUDA_TRY(cudaMemsetAsync(words, 0, sizeof(uint32_t) * (size_t)(slices + 1), s));
     IRR_CUDA_TRY(cudaMemsetAsync(d_total, 0, sizeof(unsigned long long), s));
     if (slices > 0) {
-        slice_words_kernel<<<grid_for(slices), 256, 0, s>>>(row_off, n, G, slices, words, d_total);
+        slice_words_kernel<<<grid_for(slices), 256, 0, s>>>(rows.row_off, n, G, slices, words, d_total);
         IRR_CUDA_TRY(cudaGetLastError());
     }
     unsigned long long total = 0;
@@ -1113,7 +1114,7 @@ cudaError_t build_sliced(const uint32_t* row_off, const int32_t* col, int64_t n,
     if (err == cudaSuccess && slices > 0) {
         int lg = 0;
         while ((1 << lg) < G) lg++;
-        slice_fill_kernel<<<grid_for(slices * 32), 256, 0, s>>>(row_off, col, n, lg, slices,
+        slice_fill_kernel<<<grid_for(slices * 32), 256, 0, s>>>(rows, n, lg, slices,
                                                                 sl->slice_off, sl->col);
         err = cudaGetLastError();
     }
