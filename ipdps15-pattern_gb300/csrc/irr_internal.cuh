@@ -450,14 +450,15 @@ cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uin
 constexpr int kScanThreads = 256;
 constexpr int kScanBlock = kScanThreads * 4;
 constexpr int kSortThreads = 256;
-constexpr int kSortTile = kSortThreads * 16;
+constexpr int kSortRounds = 16;                         // of a tile whose places are scanned
+constexpr int kSortTile = kSortThreads * kSortRounds;
 __global__ void scan_blocks_kernel(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* block_sums);
 __global__ void add_offsets_kernel(uint32_t* out, int64_t n, const uint32_t* block_off);
-__global__ void radix_hist_kernel(const uint32_t* keys, int64_t n, int shift, uint32_t* hist,
-                                  int64_t ntiles);
-__global__ void radix_scatter_kernel(const uint32_t* kin, const int32_t* vin, uint32_t* kout,
-                                     int32_t* vout, int64_t n, int shift, const uint32_t* offs,
-                                     int64_t ntiles);
+// One pass's kernels where the caller scans the counts, hist[digit][tile] of
+// tiles of kSortTile, in between.
+cudaError_t launch_radix_hist(const uint32_t* keys, int64_t n, int shift, uint32_t* hist, cudaStream_t s);
+cudaError_t launch_radix_scatter(const uint32_t* kin, const int32_t* vin, uint32_t* kout, int32_t* vout, int64_t n,
+                                 int shift, const uint32_t* hist, cudaStream_t s);
 
 // Morton key of one position in a frame (shared with the oracle bit for bit).
 __host__ __device__ __forceinline__ uint32_t spread3(uint32_t v)

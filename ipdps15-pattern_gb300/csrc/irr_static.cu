@@ -222,14 +222,9 @@ extern "C" int irr_morton_order_static(int device, void* stream, const void* d_p
     uint32_t *ka = keys, *kb = keys_tmp;
     int32_t *va = d_perm, *vb = vals_tmp;
     for (int shift = 0; shift < 32 && e == cudaSuccess; shift += 8) {
-        radix_hist_kernel<<<(unsigned)ntiles, kSortThreads, 0, s>>>(ka, n, shift, hist, ntiles);
-        e = cudaGetLastError();
+        e = launch_radix_hist(ka, n, shift, hist, s);
         if (e == cudaSuccess) e = scan_ws(hist, hist, 256 * ntiles, scan, kScanWords, s);
-        if (e == cudaSuccess) {
-            radix_scatter_kernel<<<(unsigned)ntiles, kSortThreads, 0, s>>>(ka, va, kb, vb, n, shift,
-                                                                          hist, ntiles);
-            e = cudaGetLastError();
-        }
+        if (e == cudaSuccess) e = launch_radix_scatter(ka, va, kb, vb, n, shift, hist, s);
         uint32_t* tk = ka;
         ka = kb;
         kb = tk;
