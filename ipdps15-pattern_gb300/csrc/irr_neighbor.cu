@@ -497,7 +497,10 @@ __device__ __forceinline__ float image_shift(int code, float box)
 // MODE kCount: deg[t] = row length.  kWrite: the row's columns from
 // row_off[t], ascending.  kScratch: both in one pass, the columns into a
 // fixed-capacity slot scratch[t * cap, +cap) (the count goes on past cap, so
-// an overflowing row is known and its entries are not stored).
+// an overflowing row is known and its entries are not stored).  864,000 atoms,
+// list radius 2.8, ~500 candidates and 78 partners each: one pass 550 us with a
+// branch per hit and 64-bit addresses, 475 without.  What bounds it: issue, and
+// the scattered 4-byte writes (counting alone takes 360).
 enum RowsMode { kCount = 0, kWrite = 1, kScratch = 2 };
 
 template <int MODE, bool FAST>
@@ -506,19 +509,24 @@ __device__ __forceinline__ void cell_rows_body(const float4* __restrict__ pos_c,
                                                const uint32_t* __restrict__ row_off, int32_t* col,
                                                uint32_t cap)
 {
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-         t += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < n; t0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t t = t0 + threadIdx.x;
+        if (t >= n) continue;
         const float4 a = pos_c[t];
         const int4* st = table + (int64_t)cell_of(a, g) * 27;
-        uint32_t m = 0;
-        int32_t* out = MODE == kWrite ? col + row_off[t] : (MODE == kScratch ? col + t * (int64_t)cap : nullptr);
+        // bytes: the row's next entry and, of slots, their end, from one base for
+        // the block (a row written in place has its own)
+        char* const base = reinterpret_cast<char*>(MODE == kWrite ? col + row_off[t]
+                                                   : MODE == kScratch ? col + t0 * (int64_t)cap : nullptr);
+        const uint32_t first = MODE == kScratch ? threadIdx.x * cap * 4u : 0u, end = first + cap * 4u;
+        uint32_t at = first;
         // one run of candidates; SELF: the node's own run (skip q == t),
         // SHIFT: a run across the box boundary (FAST only: elsewhere the cell
         // decides no shift, and the rule's own test runs when !FAST)
-        auto run = [&](auto self, auto shift, uint32_t q0, uint32_t q1, float sx, float sy, float sz) {
+        auto run = [&](auto self, auto shift, uint32_t q, uint32_t q1, float sx, float sy, float sz) {
             constexpr bool SELF = decltype(self)::value, SHIFT = decltype(shift)::value;
-#pragma unroll 4
-            for (uint32_t q = q0; q < q1; q++) {
+#pragma unroll 8
+            for (; q < q1; q++) {
                 const float4 b = pos_c[q];
                 bool hit;
                 if (!FAST)
@@ -527,11 +535,11 @@ __device__ __forceinline__ void cell_rows_body(const float4* __restrict__ pos_c,
                     hit = list_pair_shifted(a, b, sx, sy, sz, g.cut2);
                 else
                     hit = list_pair_unshifted(a, b, g.cut2);
-                if (SELF) hit = hit && q != (uint32_t)t;
-                if (hit) {
-                    if (MODE == kWrite || (MODE == kScratch && m < cap)) out[m] = (int32_t)q;
-                    m++;
-                }
+                if (SELF) hit = hit & (q != (uint32_t)t);
+                // no branch: most warps have a hit
+                if (MODE != kCount && (hit & (MODE == kWrite || at < end)))
+                    *reinterpret_cast<int32_t*>(base + at) = (int32_t)q;
+                at += hit ? 4u : 0u;
             }
         };
         using T = std::true_type;
@@ -548,7 +556,7 @@ __device__ __forceinline__ void cell_rows_body(const float4* __restrict__ pos_c,
                 run(F{}, F{}, q0, q1, 0.f, 0.f, 0.f);
             }
         }
-        if (MODE != kWrite) deg[t] = m;
+        if (MODE != kWrite) deg[t] = (at - first) / 4u;
     }
 }
 
@@ -866,9 +874,10 @@ struct Temps {
 };
 
 // Where the nodes are too few warps to hide the search's latency, 8 lanes share
-// a node's candidates: a search 189 -> 35 us at 2,048 nodes, 115 -> 65 at 32,000,
-// 106 -> 94 at 55,296; 120 -> 143 at 87,808, where instructions bound it.
-constexpr int64_t kLanesNodes = 65536;
+// a node's candidates: a search 35 us at 2,048 nodes (with a lane each 189 before
+// its loop lost its branches), 28 against 53 at 6,912, 39 against 55 at 16,384;
+// 65 against 58 at 32,000, 94 against 66 at 55,296.
+constexpr int64_t kLanesNodes = 24000;
 
 template <int MODE>
 void launch_cell_rows(const float4* pos_c, int64_t n, const Grid& g, const int* outside, const int4* table,
