@@ -274,7 +274,13 @@ inline cudaError_t irr_malloc_async(T** p, size_t bytes, cudaStream_t s)
     return irr_malloc_async(reinterpret_cast<void**>(p), bytes, s);
 }
 
-// Gives back to the driver what the pool of `device` holds unused above 8 GB.
+// The same from a second pool, for arrays that are handed to the caller (edge
+// lists).  In one pool a list that is freed while the next one's temporaries
+// are live let both wander over three places, and a neighbour list of 1,000,003
+// nodes, made again and again, took 975 or 1320 us from one process to the next.
+cudaError_t irr_malloc_result(void** p, size_t bytes, cudaStream_t s);
+
+// Gives back to the driver what the pools of `device` hold unused above 8 GB.
 void irr_pool_trim(int device);
 
 // How long a kernel's device-side waits may last before it gives up

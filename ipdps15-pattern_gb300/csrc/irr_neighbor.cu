@@ -781,7 +781,7 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
             const bool done = !got[1] && (double)cap * (double)n < 4294967296.0 && got[0] <= 0x7fffffffu;
             int2* edges = nullptr;
             if (done && got[0] > 0) {
-                IRR_CUDA_TRY(irr_malloc_async((void**)&edges, sizeof(int2) * got[0], s));
+                IRR_CUDA_TRY(irr_malloc_result((void**)&edges, sizeof(int2) * got[0], s));
                 IRR_CUDA_TRY(launch_slot_pairs(cnt, sorted, n, slots, cap, edges, s));
             }
             void* tmp[] = {slots, keys, keys_tmp, sorted, vals_tmp, cell_start, cnt, pos_c};
@@ -817,7 +817,8 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
     }
     int2* edges = nullptr;
     if (total > 0) {
-        IRR_CUDA_TRY(irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
+        IRR_CUDA_TRY(sort_rows ? irr_malloc_result((void**)&edges, sizeof(int2) * total, s)
+                               : irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
         if (sort_rows) {
             uint32_t longest = 0;
             IRR_CUDA_TRY(max_row_len(cnt, n, &longest, s));

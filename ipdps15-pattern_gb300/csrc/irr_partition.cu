@@ -1352,49 +1352,69 @@ cudaError_t launch_validate_edges(const int2* edges, int64_t e, int64_t n, int* 
 }
 
 namespace {
-constexpr int kMaxPoolDevices = 64;
+constexpr int kMaxPoolDevices = 64, kPools = 2;
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pools[kMaxPoolDevices] = {};
-}  // namespace
+cudaMemPool_t g_pools[kMaxPoolDevices][kPools] = {};
 
-cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s)
+cudaMemPool_t pool_of(int dev, int which)  // null: none could be made
+{
+    if (dev < 0 || dev >= kMaxPoolDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    cudaMemPool_t& pool = g_pools[dev][which];
+    if (!pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t made = nullptr;
+        if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
+            uint64_t keep = ~0ull;
+            cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+            pool = made;
+        } else {
+            cudaGetLastError();
+        }
+    }
+    return pool;
+}
+
+cudaError_t malloc_from(int which, void** p, size_t bytes, cudaStream_t s)
 {
     int dev = 0;
     IRR_CUDA_TRY(cudaGetDevice(&dev));
-    cudaMemPool_t pool = nullptr;
-    if (dev >= 0 && dev < kMaxPoolDevices) {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        if (!g_pools[dev]) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.handleTypes = cudaMemHandleTypeNone;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            cudaMemPool_t made = nullptr;
-            if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
-                uint64_t keep = ~0ull;
-                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
-                g_pools[dev] = made;
-            } else {
-                cudaGetLastError();
-            }
-        }
-        pool = g_pools[dev];
-    }
+    const cudaMemPool_t pool = pool_of(dev, which);
     if (!pool) return cudaMallocAsync(p, bytes, s);  // the device's default pool
-    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation) {  // what the other pool holds unused
+        const cudaMemPool_t other = pool_of(dev, 1 - which);
+        if (other && cudaMemPoolTrimTo(other, 0) == cudaSuccess) {
+            cudaGetLastError();
+            e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+        }
+    }
+    return e;
 }
+}  // namespace
+
+cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s) { return malloc_from(0, p, bytes, s); }
+cudaError_t irr_malloc_result(void** p, size_t bytes, cudaStream_t s) { return malloc_from(1, p, bytes, s); }
 
 void irr_pool_trim(int device)
 {
     constexpr uint64_t kKeep = 8ull << 30;
     if (device < 0 || device >= kMaxPoolDevices) return;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    cudaMemPool_t pool = g_pools[device];
-    uint64_t reserved = 0, used = 0;
-    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used + kKeep)
-        cudaMemPoolTrimTo(pool, used + kKeep);
+    uint64_t left = kKeep;  // unused, of both pools
+    for (cudaMemPool_t pool : g_pools[device]) {
+        uint64_t reserved = 0, used = 0;
+        if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+            continue;
+        const uint64_t unused = reserved - std::min(used, reserved);
+        if (unused > left) cudaMemPoolTrimTo(pool, used + left);
+        left -= std::min(unused, left);
+    }
     cudaGetLastError();
 }
 
