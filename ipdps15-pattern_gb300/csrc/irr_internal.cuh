@@ -173,11 +173,13 @@ struct Staged {
     int64_t nitems = 0;
     bool wide = false;               // built to the wide limits
 };
-// The wide limits, for rows that touch more nodes: an item takes up to the
-// whole ring of the halo kernel, whose other CTAs on the SM compute while one
-// loads.
+// The wide limits, for rows that touch more nodes.  An item of 6,400 words and
+// its table take about two thirds of the halo kernel's ring, so that much of the
+// next one loads beside it: 1,048,576 nodes with ~248 neighbours 489 us a step
+// at 9,984 words (64 rows an item, the whole ring) -> 450, 473 at 6,000 (fewer
+// rows share a table); with 300 neighbours 195 -> 187 (262,144 nodes).
 constexpr int kHaloWideTabMax = 1008;
-constexpr int kHaloWideStreamMax = 9984;
+constexpr int kHaloWideStreamMax = 6400;
 // Where a graph's rows are, in execution order, each row's columns in any
 // order: packed in col at row_off, or, with slots, cap apart there.
 struct RowSource {

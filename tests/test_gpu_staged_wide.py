@@ -9,7 +9,7 @@ from helpers import TOL_NORMWISE_F64, TOL_PERNODE_F64, normwise_error, random_bo
 
 pytestmark = pytest.mark.gpu
 
-WIDE = dict(slices_per_item=8, tab_max=1008, stream_max=9984)
+WIDE = dict(slices_per_item=8, tab_max=1008, stream_max=6400)
 
 
 def system(O, n, neighbours, seed):
