@@ -876,9 +876,9 @@ struct Temps {
 
 // Where the nodes are too few warps to hide the search's latency, 8 lanes share
 // a node's candidates: a search 35 us at 2,048 nodes (with a lane each 189 before
-// its loop lost its branches), 28 against 53 at 6,912, 39 against 55 at 16,384;
-// 65 against 58 at 32,000, 94 against 66 at 55,296.
-constexpr int64_t kLanesNodes = 24000;
+// its loop lost its branches), 28 against 53 at 6,912, 39 against 55 at 16,384; at
+// 32,000 100 MD steps with 5 rebuilds 2.54 against 2.63 ms; 94 against 66 at 55,296.
+constexpr int64_t kLanesNodes = 40000;
 
 template <int MODE>
 void launch_cell_rows(const float4* pos_c, int64_t n, const Grid& g, const int* outside, const int4* table,

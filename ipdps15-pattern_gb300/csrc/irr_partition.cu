@@ -1405,14 +1405,20 @@ void irr_pool_trim(int device)
     constexpr uint64_t kKeep = 8ull << 30;
     if (device < 0 || device >= kMaxPoolDevices) return;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
+    // (a query takes ~20 us: what is used matters only above kKeep)
+    uint64_t reserved[kPools] = {}, sum = 0;
+    for (int k = 0; k < kPools; k++) {
+        if (g_pools[device][k])
+            cudaMemPoolGetAttribute(g_pools[device][k], cudaMemPoolAttrReservedMemCurrent, &reserved[k]);
+        sum += reserved[k];
+    }
     uint64_t left = kKeep;  // unused, of both pools
-    for (cudaMemPool_t pool : g_pools[device]) {
-        uint64_t reserved = 0, used = 0;
-        if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    for (int k = 0; k < kPools && sum > kKeep; k++) {
+        uint64_t used = 0;
+        if (!reserved[k] || cudaMemPoolGetAttribute(g_pools[device][k], cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
             continue;
-        const uint64_t unused = reserved - std::min(used, reserved);
-        if (unused > left) cudaMemPoolTrimTo(pool, used + left);
+        const uint64_t unused = reserved[k] - std::min(used, reserved[k]);
+        if (unused > left) cudaMemPoolTrimTo(g_pools[device][k], used + left);
         left -= std::min(unused, left);
     }
     cudaGetLastError();

@@ -1,5 +1,5 @@
 """The MD rebuild's rows (GPU) against the oracle's list, with 8 lanes per node
-and with one (24,000 nodes and below, above), for cells of few and of many
+and with one (40,000 nodes and below, above), for cells of few and of many
 nodes: the pair count, and the forces of the rows."""
 import numpy as np
 import pytest
@@ -9,8 +9,8 @@ from helpers import TOL_PERNODE_F64, random_box, scaled_error
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,neighbours", [(1500, 40), (1501, 250), (5003, 100), (23999, 60), (24000, 60), (24001, 60),
-                                          (30011, 200)])
+@pytest.mark.parametrize("n,neighbours", [(1500, 40), (1501, 250), (5003, 100), (39999, 60), (40000, 60), (40001, 60),
+                                          (40005, 200)])
 def test_pairs_and_forces(built_lib, oracle_lib, n, neighbours):
     import irregular_gb300 as irr
     O = oracle_lib
