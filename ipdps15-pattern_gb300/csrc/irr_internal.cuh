@@ -391,10 +391,6 @@ struct PartitionOut {
 };
 // Per-axis min and max of pos (synchronises s).
 cudaError_t bbox_minmax(const float4* pos, int64_t n, float lo[3], float hi[3], cudaStream_t s);
-// Computes the curve frame (per-axis min and 1024 / extent) of pos: the
-// 10-bit grid both node orders quantise on.
-cudaError_t bbox_frame(const float4* pos, int64_t n, float lo[3], float scale[3],
-                       cudaStream_t s);
 // Full partition of n nodes and e half edges.  Allocates out's arrays with
 // cudaMallocAsync on s (caller frees).  reorder == 0 keeps the identity order.
 // curve: 0 = Hilbert (IRR_ORDER_HILBERT), 1 = Morton.

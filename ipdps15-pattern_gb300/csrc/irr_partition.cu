@@ -506,9 +506,19 @@ __device__ __forceinline__ uint32_t quant10(float x, float lo, float scale)
 }
 
 // Curve key of each node (curve 0: Hilbert, 1: Morton) on the 10-bit grid.
-__global__ void curve_key_kernel(const float4* pos, int64_t n, float3 lo, float3 scale, int curve,
+// box: the positions' least and greatest coordinates per axis; the curve's grid
+// divides that by 1024.
+__global__ void curve_key_kernel(const float4* pos, int64_t n, const float* __restrict__ box, int curve,
                                  uint32_t* keys, int32_t* vals)
 {
+    float lo_c[3], scale_c[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        lo_c[c] = box[c];
+        const float ext = __fsub_rn(box[3 + c], lo_c[c]);
+        scale_c[c] = ext > 0.0f ? __fdiv_rn(1024.0f, ext) : 0.0f;
+    }
+    const float3 lo = make_float3(lo_c[0], lo_c[1], lo_c[2]), scale = make_float3(scale_c[0], scale_c[1], scale_c[2]);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const float4 p = pos[i];
@@ -964,6 +974,19 @@ cudaError_t radix_sort_pairs(uint32_t* keys, int32_t* vals, uint32_t* keys_tmp,
     return err != cudaSuccess ? err : ferr;
 }
 
+namespace {
+constexpr int kBboxParts = 1024;
+
+// box[0, 6): the least and the greatest coordinates; box[6, 6 + 6 kBboxParts) is scratch.
+cudaError_t launch_bbox(const float4* pos, int64_t n, float* box, cudaStream_t s)
+{
+    const int nparts = (int)std::min<int64_t>((n + 255) / 256, kBboxParts);
+    bbox_partial_kernel<<<nparts, 256, 0, s>>>(pos, n, box + 6);
+    bbox_final_kernel<<<1, 32, 0, s>>>(box + 6, nparts, box);
+    return cudaGetLastError();
+}
+}  // namespace
+
 cudaError_t bbox_minmax(const float4* pos, int64_t n, float lo[3], float hi[3], cudaStream_t s)
 {
     for (int c = 0; c < 3; c++) {
@@ -971,34 +994,19 @@ cudaError_t bbox_minmax(const float4* pos, int64_t n, float lo[3], float hi[3], 
         hi[c] = 0.f;
     }
     if (n <= 0) return cudaSuccess;
-    const int nparts = (int)std::min<int64_t>((n + 255) / 256, 1024);
-    float* part = nullptr;
-    IRR_CUDA_TRY(alloc_async(&part, 6 * (int64_t)nparts + 6, s));
-    bbox_partial_kernel<<<nparts, 256, 0, s>>>(pos, n, part);
-    bbox_final_kernel<<<1, 32, 0, s>>>(part, nparts, part + 6 * nparts);
+    float* box = nullptr;
+    IRR_CUDA_TRY(alloc_async(&box, 6 + 6 * kBboxParts, s));
     float h[6];
-    cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(h, part + 6 * nparts, sizeof(h), cudaMemcpyDeviceToHost, s);
+    cudaError_t err = launch_bbox(pos, n, box, s);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(h, box, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-    cudaError_t ferr = cudaFreeAsync(part, s);
+    cudaError_t ferr = cudaFreeAsync(box, s);
     if (err != cudaSuccess) return err;
     for (int c = 0; c < 3; c++) {
         lo[c] = h[c];
         hi[c] = h[3 + c];
     }
     return ferr;
-}
-
-cudaError_t bbox_frame(const float4* pos, int64_t n, float lo[3], float scale[3], cudaStream_t s)
-{
-    float hi[3];
-    IRR_CUDA_TRY(bbox_minmax(pos, n, lo, hi, s));
-    for (int c = 0; c < 3; c++) {
-        const float ext = hi[c] - lo[c];
-        scale[c] = ext > 0.0f ? 1024.0f / ext : 0.0f;
-    }
-    return cudaSuccess;
 }
 
 cudaError_t launch_row_sort(const uint32_t* row_off, int64_t n, int32_t* col, cudaStream_t s,
@@ -1065,16 +1073,17 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
     IRR_CUDA_TRY(alloc_async(&out->row_off, n + 1, s));
     const int g = grid_for(n);
     if (reorder && n > 1) {
-        float lo[3], scale[3];
-        IRR_CUDA_TRY(bbox_frame(pos_user, n, lo, scale, s));
+        // the box stays on the device: the host has no use for it
+        float* box = nullptr;
+        IRR_CUDA_TRY(alloc_async(&box, 6 + 6 * kBboxParts, s));
+        IRR_CUDA_TRY(launch_bbox(pos_user, n, box, s));
         uint32_t *keys = nullptr, *keys_tmp = nullptr;
         int32_t* vals_tmp = nullptr;
         IRR_CUDA_TRY(alloc_async(&keys, n, s));
         IRR_CUDA_TRY(alloc_async(&keys_tmp, n, s));
         IRR_CUDA_TRY(alloc_async(&vals_tmp, n, s));
-        curve_key_kernel<<<g, 256, 0, s>>>(pos_user, n, make_float3(lo[0], lo[1], lo[2]),
-                                           make_float3(scale[0], scale[1], scale[2]), curve, keys,
-                                           out->perm);
+        curve_key_kernel<<<g, 256, 0, s>>>(pos_user, n, box, curve, keys, out->perm);
+        IRR_CUDA_TRY(cudaFreeAsync(box, s));
         IRR_CUDA_TRY(cudaGetLastError());
         IRR_CUDA_TRY(radix_sort_pairs(keys, out->perm, keys_tmp, vals_tmp, n, 30, s));
         IRR_CUDA_TRY(cudaFreeAsync(keys, s));

@@ -836,11 +836,11 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, Staged* st, cudaSt
         IRR_CUDA_TRY(alloc_n(&out.slice_off, S + 1, s));
         IRR_CUDA_TRY(alloc_n(&out.words, out.nwords, s));
         IRR_CUDA_TRY(alloc_n(&out.ids, out.nids, s));
-        IRR_CUDA_TRY(alloc_n(&out.items, out.nitems, s));
+        out.items = items;  // with room for an item per block
+        items = nullptr;
         if (S == 0) IRR_CUDA_TRY(cudaMemsetAsync(out.slice_off, 0, sizeof(uint32_t), s));
         if (got.items > 0) {
             const int smem = (2 * V::kStream + 16) * (int)sizeof(uint16_t);
-            IRR_CUDA_TRY(cudaMemcpyAsync(out.items, items, sizeof(WorkItem) * got.items, cudaMemcpyDeviceToDevice, s));
             IRR_CUDA_TRY(cudaFuncSetAttribute(fill_items_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             fill_items_kernel<V><<<(unsigned)std::min<int64_t>(got.items, (int64_t)sms * 128), 32 * V::kFillWarps, smem, s>>>(
                 row_off, own, place, tab, (int)got.items, out.items, out.slice_off, out.ids, out.words);
