@@ -49,7 +49,7 @@
 // ordered as bits of a 1,024-bit map.
 // What bounds it: instruction issue (a hash probe, a bit and a pick per entry).
 // 1,000,003 nodes at 64 neighbours: sorting the rows, counting the tables and
-// filling, a table gathered in both, 353 + 172 + 721 us; now 350 + 343, and the
+// filling, a table gathered in both, 353 + 172 + 721 us; now 350 + 288, and the
 // rows (4 bytes an entry) are made from the layout when they are asked for.
 #include <algorithm>
 #include <climits>
@@ -66,12 +66,12 @@ constexpr int kPick = 8;                         // slices of an item, blocks of
 struct NarrowItem {
     static constexpr int kTab = kHaloTabMax, kStream = kHaloStreamMax;
     static constexpr int kHash = 1024, kCutThreads = 128, kAhead = 2;
-    static constexpr int kFillWarps = 2, kFillCtas = 12;
+    static constexpr int kFillWarps = 2, kFillCtas = 18;
 };
 struct WideItem {
     static constexpr int kTab = kHaloWideTabMax, kStream = kHaloWideStreamMax;
     static constexpr int kHash = 2048, kCutThreads = 256, kAhead = 4;
-    static constexpr int kFillWarps = 4, kFillCtas = 5;
+    static constexpr int kFillWarps = 4, kFillCtas = 8;
 };
 // add_rows' ids past the limit (8 rows' own ids, then what is in flight) fit the hash
 template <class V>
@@ -90,7 +90,7 @@ struct BuildTotals {
     uint32_t items;
     uint32_t runs;
     uint32_t flags;
-    uint32_t pad_;
+    uint32_t entries;  // of the largest item
 };
 
 // One item as cut_runs_kernel finds it, at its first block.
@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
             if (tid == 0) {
                 cut[b0 + from] = CutItem{(uint32_t)(to - from), (uint32_t)ntab, words};
                 cuts[b0 + from] = 1;
+                atomicMax(&out->entries, src.row_off[r0 + m] - src.row_off[r0]);
             }
             from = to;
         }
@@ -656,8 +657,8 @@ __global__ void __launch_bounds__(V::kFillWarps * 32, V::kFillCtas) fill_items_k
     constexpr int kWarps = V::kFillWarps, kThreads = 32 * kWarps, kRows = 8 * kPick / kWarps;
     static_assert(kRows <= 32, "a thread per row of the warp");
     extern __shared__ __align__(16) unsigned char dyn[];
-    // the entries' places, 16-byte aligned as in memory (every word of a step
-    // holds two entries: at most 2 kStream of them), then ordered in place
+    // the entries' places, 16-byte aligned as in memory (of the largest item:
+    // every word of a step holds two, so at most 2 kStream), then ordered in place
     uint16_t* const rs = reinterpret_cast<uint16_t*>(dyn);
     __shared__ uint32_t off[8 * kPick + 1];     // the rows' first entries in rs
     __shared__ __align__(16) uint32_t key[8 * kPick];
@@ -840,7 +841,8 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, Staged* st, cudaSt
         items = nullptr;
         if (S == 0) IRR_CUDA_TRY(cudaMemsetAsync(out.slice_off, 0, sizeof(uint32_t), s));
         if (got.items > 0) {
-            const int smem = (2 * V::kStream + 16) * (int)sizeof(uint16_t);
+            // the largest item's entries and 7 on either side, in whole eights
+            const int smem = (int)((std::min<uint32_t>(got.entries, 2 * V::kStream) + 7 + 15) / 8 * 8 * sizeof(uint16_t));
             IRR_CUDA_TRY(cudaFuncSetAttribute(fill_items_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             fill_items_kernel<V><<<(unsigned)std::min<int64_t>(got.items, (int64_t)sms * 128), 32 * V::kFillWarps, smem, s>>>(
                 row_off, own, place, tab, (int)got.items, out.items, out.slice_off, out.ids, out.words);
