@@ -49,7 +49,7 @@
 // ordered as bits of a 1,024-bit map.
 // What bounds it: instruction issue (a hash probe, a bit and a pick per entry).
 // 1,000,003 nodes at 64 neighbours: sorting the rows, counting the tables and
-// filling, a table gathered in both, 353 + 172 + 721 us; now 350 + 288, and the
+// filling, a table gathered in both, 353 + 172 + 721 us; now 323 + 288, and the
 // rows (4 bytes an entry) are made from the layout when they are asked for.
 #include <algorithm>
 #include <climits>
@@ -65,7 +65,7 @@ constexpr int kPick = 8;                         // slices of an item, blocks of
 // between two looks at whether it is full (1, 2 or 4).
 struct NarrowItem {
     static constexpr int kTab = kHaloTabMax, kStream = kHaloStreamMax;
-    static constexpr int kHash = 1024, kCutThreads = 128, kAhead = 2;
+    static constexpr int kHash = 1024, kCutThreads = 160, kAhead = 2;
     static constexpr int kFillWarps = 2, kFillCtas = 18;
 };
 struct WideItem {
