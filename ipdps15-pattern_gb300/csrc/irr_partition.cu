@@ -635,7 +635,8 @@ __global__ void __launch_bounds__(256) slot_rows_kernel(const int2* __restrict__
     const int lane = threadIdx.x & 31;
     const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * kSlotNodes;
     for (int64_t a0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSlotNodes; a0 < n; a0 += stride) {
-        if (*(volatile int*)over) return;
+        // other warps may raise it now: all lanes leave or none
+        if (__any_sync(0xffffffffu, *(volatile int*)over)) return;
         // lane t: node a0 + t, its pairs and the place of its stretch
         uint32_t r0 = 0, len = 0, at = 0;
         if (lane < kSlotNodes && a0 + lane < n) {
