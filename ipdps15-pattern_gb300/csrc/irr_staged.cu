@@ -397,9 +397,13 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
     __shared__ int held, ngroups;  // groups in the hash, and collected
     __shared__ int count;          // ids
     __shared__ uint32_t words;
-    if (out->flags) return;
-    const uint32_t runs = out->runs;
+    __shared__ uint32_t refused;
     const int tid = threadIdx.x;
+    // other CTAs may raise the flag now: one thread looks, for all to leave or none
+    if (tid == 0) refused = *(volatile uint32_t*)&out->flags;
+    __syncthreads();
+    if (refused) return;
+    const uint32_t runs = out->runs;
     auto reset = [&]() {
         __syncthreads();
         set.clear();
