@@ -9,8 +9,10 @@
 #include <cstring>
 #include <string>
 #include <vector>
+#include <cuda.h>
 
 #include "irr_handle.cuh"
+#include "irr_records.h"
 #include "irr_trace.cuh"
 
 using namespace irr;
@@ -100,19 +102,48 @@ void free_layout(irr_handle* h)
     h->inited = false;
 }
 
-// Whether the load kernels can read records of elm bytes at p in place: memory
-// the device addresses as its own, at the alignment their loads want.  Other
-// pointers go through the staging copy, whose checks are the runtime's.
-bool device_records(const void* p, int elm)
+// The driver's pointer query (it knows the allocation's range, the runtime's
+// does not), found at run time so that the library links the runtime alone.
+// Null where there is none.
+using PointerQuery = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+PointerQuery pointer_query()
 {
-    const uintptr_t align = elm == 12 ? 4 : (elm == 16 ? 16 : 8);
-    if (reinterpret_cast<uintptr_t>(p) % align) return false;
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) && a.devicePointer == p;
+    static const PointerQuery query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<PointerQuery>(f);
+    }();
+    return query;
+}
+
+// records_in_place for n records of elm bytes at p.
+bool device_records(const irr_handle* h, const void* p, int elm, int64_t n)
+{
+    const PointerQuery query = pointer_query();
+    if (!query) return false;
+    unsigned type = 0, managed = 0;
+    int ordinal = -1;
+    CUdeviceptr address = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,    CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* to[] = {&type, &managed, &ordinal, &address, &start, &size};
+    if (query(6, what, to, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    PointerFacts f;
+    f.managed = managed != 0;
+    f.device = type == CU_MEMORYTYPE_DEVICE || f.managed;
+    f.ordinal = ordinal;
+    f.address = address;
+    f.range_start = start;
+    f.range_size = size;
+    return records_in_place((uint64_t)(uintptr_t)p, elm, (uint64_t)n * (uint64_t)elm, h->device, f);
 }
 
 // Node records: positions (12/16/24 bytes) for the built-in laws; any
@@ -273,7 +304,7 @@ int set_nodes_common(irr_handle* h, const void* src, int elm, int64_t n, cudaMem
             return IRR_OK;
         }
     }
-    if (kind == cudaMemcpyDeviceToDevice && h->inited && n > 0 && !h->user_launch && device_records(src, elm)) {
+    if (kind == cudaMemcpyDeviceToDevice && h->inited && n > 0 && !h->user_launch && device_records(h, src, elm, n)) {
         // device records straight into execution order, without the staging
         // copy (14 us of 446 at 4M nodes, 2.8 of 16.5 at 65,536).  Gathered by
         // the execution order; read in order and scattered, as host records
