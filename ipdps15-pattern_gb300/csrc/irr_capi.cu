@@ -606,7 +606,8 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     if (!h || !h->inited || h->cfg.exec != IRR_EXEC_PARTITIONED) return IRR_ERR_STATE;
     if (h->user_launch) return fail(h, IRR_ERR_STATE, "a handle with a user map runs its own kernel");
     DeviceGuard dev_guard(h->device);
-    H_CUDA(h, cudaStreamSynchronize(h->stream), "layout");  // no launch may use the old layout
+    // no launch may use the old layout: a batch's steps read it on the batch's stream
+    H_CUDA(h, h->d_items ? cudaDeviceSynchronize() : cudaStreamSynchronize(h->stream), "layout");
     const int64_t n = h->n, e = h->e;
     h->shape.lanes_per_row = lanes_per_row;
     h->shape.block_nodes = block_nodes;
@@ -627,7 +628,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
                     se = build_staged(rows, n, h->m, true, &h->st, h->stream);
                 if (se != cudaSuccess) {
                     cudaGetLastError();
-                    free_staged(&h->st);
+                    free_staged(&h->st, h->stream);
                     if (want == IRR_LAYOUT_STAGED)
                         return se == cudaErrorNotSupported
                                    ? fail(h, IRR_ERR_CAPACITY,
@@ -637,7 +638,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
                 }
             }
             if (want == IRR_LAYOUT_AUTO && h->st.words && h->m < kStagedMinReuse * h->st.nids)
-                free_staged(&h->st);  // too little reuse to pay for staging
+                free_staged(&h->st, h->stream);  // too little reuse to pay for staging
             staged = h->st.words != nullptr || (n == 0 && want == IRR_LAYOUT_STAGED);
         } else if (want == IRR_LAYOUT_STAGED) {
             return fail(h, IRR_ERR_ARG, "the staged layout needs 4 lanes per row and stage_smem");
@@ -645,25 +646,25 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     }
     h->shape.staged = staged ? (h->st.wide ? 2 : 1) : 0;
     if (staged) {
-        free_sliced(&h->sl);
+        free_sliced(&h->sl, h->stream);
         dfree(h, h->part.slots);  // the layout holds the entries now
     } else {
         const int rc = ensure_rows(h);
         if (rc) return rc;
-        free_staged(&h->st);
+        free_staged(&h->st, h->stream);
         if (want == IRR_LAYOUT_CSR) {
-            free_sliced(&h->sl);
+            free_sliced(&h->sl, h->stream);
         } else if (h->sl.lanes != lanes_per_row) {
             const cudaError_t se = build_sliced(RowSource{h->part.row_off, h->part.col, nullptr, 0}, n, lanes_per_row, &h->sl, h->stream);
             if (se != cudaSuccess) {
                 cudaGetLastError();
-                free_sliced(&h->sl);
+                free_sliced(&h->sl, h->stream);
                 if (want == IRR_LAYOUT_SLICED)
                     return se == cudaErrorInvalidValue
                                ? fail(h, IRR_ERR_CAPACITY, "sliced layout above 2^32 words")
                                : cuda_fail(h, se, "build sliced layout");
             } else if (want != IRR_LAYOUT_SLICED && !sliced_pays(h->sl, h->m)) {
-                free_sliced(&h->sl);
+                free_sliced(&h->sl, h->stream);
             }
         }
     }

@@ -194,7 +194,9 @@ struct RowSource {
     }
 #endif
 };
-// Builds st from n rows of m entries in all on the device.  Synchronises s.
+// Builds st from n rows of m entries in all on the device.  Waits for s while it
+// learns the sizes; the layout's words are still being written on s when it
+// returns, and may read src until then.
 // cudaErrorNotSupported (nothing allocated) when a slice alone exceeds the
 // limits above -- a row of more than ~440 entries (wide: 1023), or 8 rows
 // touching more than kHaloTabMax (wide: kHaloWideTabMax) distinct nodes.
@@ -203,7 +205,8 @@ cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, 
 // row_off, each row ascending.
 cudaError_t rows_of_staged(const Staged& st, const WorkItem* items, const uint32_t* row_off, int64_t n, int32_t* col,
                            cudaStream_t s);
-void free_staged(Staged* st, cudaStream_t s = nullptr);
+// Freed behind the work on s (0: the default stream), which is all that uses it.
+void free_staged(Staged* st, cudaStream_t s);
 // Items copied to the host; synchronises s.
 cudaError_t staged_items_to_host(const WorkItem* d_items, int64_t count, std::vector<WorkItem>* items, cudaStream_t s);
 
@@ -254,8 +257,8 @@ void make_instance_items(const uint32_t* host_row_off, const Sliced& sl, int64_t
 // cudaErrorInvalidValue if the layout would exceed 2^32 - 1 words.
 cudaError_t build_sliced(const RowSource& rows, int64_t n, int G,
                          Sliced* sl, cudaStream_t s);
-// s != nullptr: stream-ordered frees on s (the arrays come from cudaMallocAsync).
-void free_sliced(Sliced* sl, cudaStream_t s = nullptr);
+// As free_staged.
+void free_sliced(Sliced* sl, cudaStream_t s);
 // The automatic choice: sliced when padding adds at most half the entries.
 inline bool sliced_pays(const Sliced& sl, int64_t entries)
 {

@@ -1268,7 +1268,7 @@ cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_
 cudaError_t build_sliced(const RowSource& rows, int64_t n, int G,
                          Sliced* sl, cudaStream_t s)
 {
-    free_sliced(sl);
+    free_sliced(sl, s);
     if (n < 0 || (G != 1 && G != 2 && G != 4 && G != 8 && G != 16 && G != 32))
         return cudaErrorInvalidValue;
     const int R = 32 / G;
@@ -1307,7 +1307,7 @@ cudaError_t build_sliced(const RowSource& rows, int64_t n, int G,
     cudaFreeAsync(d_total, s);
     if (err == cudaSuccess) err = cudaStreamSynchronize(s);
     if (err != cudaSuccess) {
-        free_sliced(sl);
+        free_sliced(sl, s);
         return err;
     }
     sl->slices = slices;
@@ -1318,13 +1318,8 @@ cudaError_t build_sliced(const RowSource& rows, int64_t n, int G,
 
 void free_sliced(Sliced* sl, cudaStream_t s)
 {
-    if (s) {
-        if (sl->slice_off) cudaFreeAsync(sl->slice_off, s);
-        if (sl->col) cudaFreeAsync(sl->col, s);
-    } else {
-        if (sl->slice_off) cudaFree(sl->slice_off);
-        if (sl->col) cudaFree(sl->col);
-    }
+    if (sl->slice_off) cudaFreeAsync(sl->slice_off, s);
+    if (sl->col) cudaFreeAsync(sl->col, s);
     sl->slice_off = nullptr;
     sl->col = nullptr;
     sl->slices = sl->words = 0;

@@ -872,10 +872,7 @@ void free_staged(Staged* st, cudaStream_t s)
 {
     void* ps[4] = {st->slice_off, st->words, st->ids, st->items};
     for (void* p : ps)
-        if (p) {
-            if (s) cudaFreeAsync(p, s);
-            else cudaFree(p);
-        }
+        if (p) cudaFreeAsync(p, s);
     *st = Staged{};
 }
 
