@@ -845,9 +845,11 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, Staged* st, cudaSt
         items = nullptr;
         if (S == 0) IRR_CUDA_TRY(cudaMemsetAsync(out.slice_off, 0, sizeof(uint32_t), s));
         if (got.items > 0) {
-            // the largest item's entries and 7 on either side, in whole eights
+            // the largest item's entries and 7 on either side, in whole eights (a
+            // launch's own argument: the kernel's limit, which all threads share, stays)
             const int smem = (int)((std::min<uint32_t>(got.entries, 2 * V::kStream) + 7 + 15) / 8 * 8 * sizeof(uint16_t));
-            IRR_CUDA_TRY(cudaFuncSetAttribute(fill_items_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            static_assert((2 * V::kStream + 22) * sizeof(uint16_t) + 4096 <= 48 * 1024,
+                          "with the kernel's own arrays inside the shared memory a launch may have unasked");
             fill_items_kernel<V><<<(unsigned)std::min<int64_t>(got.items, (int64_t)sms * 128), 32 * V::kFillWarps, smem, s>>>(
                 row_off, own, place, tab, (int)got.items, out.items, out.slice_off, out.ids, out.words);
             IRR_CUDA_TRY(cudaGetLastError());

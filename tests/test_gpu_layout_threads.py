@@ -93,3 +93,27 @@ def test_dropped_layouts(built_lib):
             h.close()
 
     in_threads(len(inputs), work)
+
+
+def test_setups_of_different_sizes(built_lib):
+    """Items of few and of many entries: a set-up's launch takes the shared memory
+    of its own largest item, whatever another thread's takes at that moment."""
+    import irregular_gb300 as irr
+    inputs = [graph(600 + 9 * k, 8 if k % 2 else 40, 60, k) for k in range(16)]
+    alone = []
+    for e, pos in inputs:
+        h = handle(irr, e, pos)
+        assert h.info().layout == irr.IRR_LAYOUT_STAGED
+        alone.append(facts(irr, h))
+        h.close()
+
+    def work(k):
+        e, pos = inputs[k]
+        for _ in range(250):
+            h = handle(irr, e, pos)
+            h.step()
+            got = h.get_result(elm_size=12).view(np.uint32)
+            h.close()
+            assert np.array_equal(got, alone[k][-1])
+
+    in_threads(len(inputs), work)
