@@ -70,10 +70,14 @@ cudaError_t dalloc(irr_handle* h, T** p, size_t bytes)
     return e == cudaSuccess ? cudaStreamSynchronize(h->own_stream) : e;
 }
 
-// Freed behind the work on the handle's stream, the only one that uses it.
+// Freed behind the work on the handle's stream and on those it had before.
 template <class T>
 void dfree(irr_handle* h, T*& p)
 {
+    if (p && h->switched) {
+        cudaDeviceSynchronize();
+        h->switched = false;
+    }
     if (p) cudaFreeAsync((void*)p, h->stream);
     p = nullptr;
 }
@@ -837,6 +841,9 @@ const char* irr_last_error(const irr_handle* h) { return h ? h->err.c_str() : "n
 int irr_set_stream(irr_handle* h, void* stream)
 {
     if (!h) return IRR_ERR_ARG;
+    // the old stream is not asked: it may be gone already
+    const bool used = h->n >= 0 || h->e >= 0 || h->coord_n >= 0;
+    if (used && (cudaStream_t)stream != h->stream) h->switched = true;
     h->stream = (cudaStream_t)stream;  // used as given: NULL is the default stream
     return IRR_OK;
 }

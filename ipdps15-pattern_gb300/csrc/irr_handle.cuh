@@ -18,6 +18,7 @@ struct irr_handle {
     int sms = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
+    bool switched = false;       // work may be in flight on a stream it had before
     std::string err;
 
     int map_idx = IRR_MAP_LJ_MOLDYN;
