@@ -271,7 +271,8 @@ inline bool sliced_pays(const Sliced& sl, int64_t entries)
 // cudaFreeAsync stay in the pool for the next allocation instead of going back
 // to the driver at every synchronisation (the default pool's behaviour), so a
 // rebuild that frees and re-allocates ~300 MB of layout does not re-map it.
-// The pool keeps what is freed until a handle is destroyed (irr_pool_trim).
+// What is freed stays in the pool, up to 8 GB of it after a handle, a list or a
+// system is freed (irr_pool_trim).
 cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s);
 template <class T>
 inline cudaError_t irr_malloc_async(T** p, size_t bytes, cudaStream_t s)
@@ -279,13 +280,16 @@ inline cudaError_t irr_malloc_async(T** p, size_t bytes, cudaStream_t s)
     return irr_malloc_async(reinterpret_cast<void**>(p), bytes, s);
 }
 
-// The same from a second pool, for arrays that are handed to the caller (edge
-// lists).  In one pool a list that is freed while the next one's temporaries
-// are live let both wander over three places, and a neighbour list of 1,000,003
-// nodes, made again and again, took 975 or 1320 us from one process to the next.
-cudaError_t irr_malloc_result(void** p, size_t bytes, cudaStream_t s);
+// Edge lists, which are the caller's: cudaMalloc'd, so that peers and other
+// processes reach them as any device memory.  irr_free_list, after the last use
+// of p by the device, keeps up to 1 GB of freed ones per device for the next
+// list: of 370 MB, 1,000,003 nodes' list, the cudaMalloc takes 140 to 200 us and the
+// cudaFree 180 to 200, the search 960.  Memory that the library did not give out
+// as a list is cudaFree'd.
+cudaError_t irr_malloc_list(void** p, size_t bytes);
+cudaError_t irr_free_list(void* p);
 
-// Gives back to the driver what the pools of `device` hold unused above 8 GB.
+// Gives back to the driver what the pool of `device` holds unused above 8 GB.
 void irr_pool_trim(int device);
 
 // How long a kernel's device-side waits may last before it gives up
@@ -411,8 +415,8 @@ cudaError_t alloc_col(int32_t** col, int64_t m, cudaStream_t s);
 // A shard's partition: rows whose caller id is outside [lo, hi) lose their
 // entries (row_off and col rebuilt, order kept); *m_out = entries left.
 cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_t* m_out, cudaStream_t s);
-// Half neighbour list (irr_neighbor.cu); *d_edges is from the pool, allocated
-// on s, which is synchronised.
+// Half neighbour list (irr_neighbor.cu); *d_edges is from irr_malloc_list
+// (unsorted: from the pool, on s); s is synchronised.
 // sort_rows == false returns the same pairs (i < j) in no particular order,
 // for a caller that re-sorts them anyway, like the partitioner (found by a
 // half-stencil search when the box has at least 3 cells per axis).

@@ -439,6 +439,22 @@ int md_rebuild(irr_md* m)
     return IRR_OK;
 }
 
+void md_free(irr_md* m)
+{
+    DeviceGuard dev_guard(m->device);
+    if (m->stream) cudaStreamSynchronize(m->stream);
+    if (m->own_stream) {
+        free_part(m, m->own_stream);
+        void* ptrs[] = {m->x, m->v, m->tmp, m->pos4, m->force, m->ids, m->ids_tmp,
+                        m->d_inst, m->d_queue, m->d_status, m->d_acc};
+        for (void* p : ptrs)
+            if (p) cudaFreeAsync(p, m->own_stream);
+        cudaStreamSynchronize(m->own_stream);
+        cudaStreamDestroy(m->own_stream);
+    }
+    delete m;
+}
+
 int md_forces(irr_md* m)
 {
     if (m->cfg.exec_plain) {
@@ -613,18 +629,10 @@ int irr_md_create(const irr_md_config* cfg, const double* pos, const double* vel
 int irr_md_destroy(irr_md* m)
 {
     if (!m) return IRR_ERR_ARG;
-    DeviceGuard dev_guard(m->device);
-    if (m->stream) cudaStreamSynchronize(m->stream);
-    if (m->own_stream) {
-        free_part(m, m->own_stream);
-        void* ptrs[] = {m->x, m->v, m->tmp, m->pos4, m->force, m->ids, m->ids_tmp,
-                        m->d_inst, m->d_queue, m->d_status, m->d_acc};
-        for (void* p : ptrs)
-            if (p) cudaFreeAsync(p, m->own_stream);
-        cudaStreamSynchronize(m->own_stream);
-        cudaStreamDestroy(m->own_stream);
-    }
-    delete m;
+    const int device = m->device;
+    md_free(m);
+    DeviceGuard dev_guard(device);
+    irr_pool_trim(device);
     return IRR_OK;
 }
 

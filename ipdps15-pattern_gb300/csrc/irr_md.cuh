@@ -214,6 +214,9 @@ int md_forces(irr_md* m);
 int md_kick_drift(irr_md* m);
 int md_kick(irr_md* m);
 InstDesc md_instance(const irr_md* m);
+// irr_md_destroy, what the pool holds unused left there (a serving loop's next
+// system takes it).
+void md_free(irr_md* m);
 // Digest of the final positions by atom id (a sum of per-atom 64-bit mixes).
 int md_state_digest(irr_md* m, uint64_t* digest);
 }  // namespace irr

@@ -781,7 +781,7 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
             const bool done = !got[1] && (double)cap * (double)n < 4294967296.0 && got[0] <= 0x7fffffffu;
             int2* edges = nullptr;
             if (done && got[0] > 0) {
-                IRR_CUDA_TRY(irr_malloc_result((void**)&edges, sizeof(int2) * got[0], s));
+                IRR_CUDA_TRY(irr_malloc_list((void**)&edges, sizeof(int2) * got[0]));
                 IRR_CUDA_TRY(launch_slot_pairs(cnt, sorted, n, slots, cap, edges, s));
             }
             void* tmp[] = {slots, keys, keys_tmp, sorted, vals_tmp, cell_start, cnt, pos_c};
@@ -817,7 +817,7 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
     }
     int2* edges = nullptr;
     if (total > 0) {
-        IRR_CUDA_TRY(sort_rows ? irr_malloc_result((void**)&edges, sizeof(int2) * total, s)
+        IRR_CUDA_TRY(sort_rows ? irr_malloc_list((void**)&edges, sizeof(int2) * total)
                                : irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
         if (sort_rows) {
             uint32_t longest = 0;
@@ -1031,7 +1031,10 @@ int irr_neighbor_build(int device, void* stream, const void* pos, int pos_elm, i
     if (e != cudaSuccess) {
         cudaGetLastError();
         rc = (e == cudaErrorMemoryAllocation) ? IRR_ERR_NOMEM : (e == cudaErrorInvalidValue ? IRR_ERR_CAPACITY : IRR_ERR_CUDA);
-        if (edges) cudaFreeAsync(edges, s);
+        if (edges) {
+            cudaStreamSynchronize(s);
+            irr::irr_free_list(edges);
+        }
         edges = nullptr;
         cnt = 0;
     }
@@ -1046,11 +1049,11 @@ int irr_device_free(int device, void* d_ptr)
 {
     if (!d_ptr) return IRR_OK;
     irr::DeviceGuard dev_guard(device);
-    // pool memory is freed without waiting for its last use
-    if (!dev_guard.ok() || cudaDeviceSynchronize() != cudaSuccess || cudaFree(d_ptr) != cudaSuccess) {
+    if (!dev_guard.ok() || cudaDeviceSynchronize() != cudaSuccess || irr::irr_free_list(d_ptr) != cudaSuccess) {
         cudaGetLastError();
         return IRR_ERR_CUDA;
     }
+    irr::irr_pool_trim(device);
     return IRR_OK;
 }
 

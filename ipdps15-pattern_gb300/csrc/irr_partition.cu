@@ -23,6 +23,7 @@
 //    so that one warp reads one contiguous line per step.
 #include <algorithm>
 #include <mutex>
+#include <vector>
 
 #include "irr_internal.cuh"
 
@@ -1379,15 +1380,15 @@ cudaError_t launch_validate_edges(const int2* edges, int64_t e, int64_t n, int* 
 }
 
 namespace {
-constexpr int kMaxPoolDevices = 64, kPools = 2;
+constexpr int kMaxPoolDevices = 64;
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pools[kMaxPoolDevices][kPools] = {};
+cudaMemPool_t g_pools[kMaxPoolDevices] = {};
 
-cudaMemPool_t pool_of(int dev, int which)  // null: none could be made
+cudaMemPool_t pool_of(int dev)  // null: none could be made
 {
     if (dev < 0 || dev >= kMaxPoolDevices) return nullptr;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    cudaMemPool_t& pool = g_pools[dev][which];
+    cudaMemPool_t& pool = g_pools[dev];
     if (!pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
@@ -1406,48 +1407,127 @@ cudaMemPool_t pool_of(int dev, int which)  // null: none could be made
     return pool;
 }
 
-cudaError_t malloc_from(int which, void** p, size_t bytes, cudaStream_t s)
+// Lists in the caller's hands, and freed ones kept for the next list (the
+// longest kept first).
+struct ListBlock {
+    void* p;
+    size_t bytes;
+    int device;
+};
+constexpr size_t kSpareBytes = 1ull << 30;
+std::mutex g_list_mutex;
+std::vector<ListBlock> g_lists, g_spares;
+
+// Frees the device's oldest spares until they take at most `keep` bytes.
+bool drop_spares(int dev, size_t keep)
 {
-    int dev = 0;
-    IRR_CUDA_TRY(cudaGetDevice(&dev));
-    const cudaMemPool_t pool = pool_of(dev, which);
-    if (!pool) return cudaMallocAsync(p, bytes, s);  // the device's default pool
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
-    if (e == cudaErrorMemoryAllocation) {  // what the other pool holds unused
-        const cudaMemPool_t other = pool_of(dev, 1 - which);
-        if (other && cudaMemPoolTrimTo(other, 0) == cudaSuccess) {
-            cudaGetLastError();
-            e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    std::vector<void*> drop;
+    {
+        std::lock_guard<std::mutex> lock(g_list_mutex);
+        size_t held = 0;
+        for (const ListBlock& b : g_spares) held += b.device == dev ? b.bytes : 0;
+        for (size_t k = 0; k < g_spares.size() && held > keep;) {
+            if (g_spares[k].device != dev) {
+                k++;
+                continue;
+            }
+            held -= g_spares[k].bytes;
+            drop.push_back(g_spares[k].p);
+            g_spares.erase(g_spares.begin() + (ptrdiff_t)k);
         }
     }
-    return e;
+    for (void* p : drop) cudaFree(p);
+    return !drop.empty();
 }
 }  // namespace
 
-cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s) { return malloc_from(0, p, bytes, s); }
-cudaError_t irr_malloc_result(void** p, size_t bytes, cudaStream_t s) { return malloc_from(1, p, bytes, s); }
+cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s)
+{
+    int dev = 0;
+    IRR_CUDA_TRY(cudaGetDevice(&dev));
+    const cudaMemPool_t pool = pool_of(dev);
+    auto get = [&]() { return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s); };
+    cudaError_t e = get();
+    if (e == cudaErrorMemoryAllocation && drop_spares(dev, 0)) {
+        cudaGetLastError();
+        e = get();
+    }
+    return e;
+}
+
+cudaError_t irr_malloc_list(void** p, size_t bytes)
+{
+    int dev = 0;
+    IRR_CUDA_TRY(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lock(g_list_mutex);
+        size_t best = g_spares.size();
+        for (size_t k = 0; k < g_spares.size(); k++) {
+            const ListBlock& b = g_spares[k];
+            if (b.device == dev && b.bytes >= bytes && b.bytes / 4 * 3 <= bytes &&
+                (best == g_spares.size() || b.bytes < g_spares[best].bytes))
+                best = k;
+        }
+        if (best < g_spares.size()) {
+            *p = g_spares[best].p;
+            g_lists.push_back(g_spares[best]);
+            g_spares.erase(g_spares.begin() + (ptrdiff_t)best);
+            return cudaSuccess;
+        }
+    }
+    // whole 2 MB pages, and a 64th more: the next list is seldom just as long
+    constexpr size_t kPage = 2ull << 20;
+    const size_t more = (bytes + bytes / 64 + kPage - 1) / kPage * kPage;
+    size_t got = more;
+    cudaError_t e = cudaMalloc(p, got);
+    if (e == cudaErrorMemoryAllocation) {  // what is kept unused, and no more than the list
+        cudaGetLastError();
+        drop_spares(dev, 0);
+        if (const cudaMemPool_t pool = pool_of(dev)) cudaMemPoolTrimTo(pool, 0);
+        cudaGetLastError();
+        got = bytes;
+        e = cudaMalloc(p, got);
+    }
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(g_list_mutex);
+    for (size_t k = 0; k < g_lists.size();) {  // of a list that the caller gave to cudaFree
+        if (g_lists[k].p == *p) g_lists.erase(g_lists.begin() + (ptrdiff_t)k);
+        else k++;
+    }
+    g_lists.push_back(ListBlock{*p, got, dev});
+    return cudaSuccess;
+}
+
+cudaError_t irr_free_list(void* p)
+{
+    ListBlock b{p, 0, -1};
+    {
+        std::lock_guard<std::mutex> lock(g_list_mutex);
+        for (size_t k = 0; k < g_lists.size(); k++) {
+            if (g_lists[k].p != p) continue;
+            b = g_lists[k];
+            g_lists.erase(g_lists.begin() + (ptrdiff_t)k);
+            break;
+        }
+        if (b.device >= 0 && b.bytes <= kSpareBytes) g_spares.push_back(b);
+    }
+    if (b.device < 0 || b.bytes > kSpareBytes) return cudaFree(p);
+    drop_spares(b.device, kSpareBytes);
+    return cudaSuccess;
+}
 
 void irr_pool_trim(int device)
 {
     constexpr uint64_t kKeep = 8ull << 30;
     if (device < 0 || device >= kMaxPoolDevices) return;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
+    const cudaMemPool_t pool = g_pools[device];
     // (a query takes ~20 us: what is used matters only above kKeep)
-    uint64_t reserved[kPools] = {}, sum = 0;
-    for (int k = 0; k < kPools; k++) {
-        if (g_pools[device][k])
-            cudaMemPoolGetAttribute(g_pools[device][k], cudaMemPoolAttrReservedMemCurrent, &reserved[k]);
-        sum += reserved[k];
-    }
-    uint64_t left = kKeep;  // unused, of both pools
-    for (int k = 0; k < kPools && sum > kKeep; k++) {
-        uint64_t used = 0;
-        if (!reserved[k] || cudaMemPoolGetAttribute(g_pools[device][k], cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-            continue;
-        const uint64_t unused = reserved[k] - std::min(used, reserved[k]);
-        if (unused > left) cudaMemPoolTrimTo(g_pools[device][k], used + left);
-        left -= std::min(unused, left);
-    }
+    uint64_t reserved = 0, used = 0;
+    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        reserved > kKeep && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        reserved - std::min(used, reserved) > kKeep)
+        cudaMemPoolTrimTo(pool, used + kKeep);
     cudaGetLastError();
 }
 

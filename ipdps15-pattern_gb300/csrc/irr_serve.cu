@@ -720,7 +720,7 @@ int irr_serve_run(const irr_serve_config* cfg, irr_serve_stats* st, irr_serve_jo
                     r.status = IRR_OK;
                     out[L.id] = r;
                 }
-                irr_md_destroy(L.md);
+                md_free(L.md);
             });
             for (size_t i = fin.size(); i-- > 0;) {
                 const Live& L = live[fin[i]];
@@ -736,10 +736,10 @@ int irr_serve_run(const irr_serve_config* cfg, irr_serve_stats* st, irr_serve_jo
     const double makespan = now();
     for (auto& a : creating) {  // set-ups still running after an error
         if (a->worker.joinable()) a->worker.join();
-        if (a->made) irr_md_destroy(a->made);
+        if (a->made) md_free(a->made);
     }
     for (auto& r : req) r.release();
-    for (auto& L : live) irr_md_destroy(L.md);
+    for (auto& L : live) md_free(L.md);
     if (ev_kd) cudaEventDestroy(ev_kd);
     int dev_status = 0;
     cudaMemcpy(&dev_status, d_status, sizeof(int), cudaMemcpyDeviceToHost);
@@ -749,6 +749,7 @@ int irr_serve_run(const irr_serve_config* cfg, irr_serve_stats* st, irr_serve_jo
     cudaFree(d_queue);
     cudaFree(d_status);
     cudaStreamDestroy(s);
+    irr_pool_trim(cfg->device);
     if (rc == IRR_OK && dev_status) rc = IRR_ERR_DEVICE;
     st->makespan_s = makespan;
     st->p50_ms = 1e3 * pct(latency, 0.50);

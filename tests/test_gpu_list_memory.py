@@ -1,0 +1,96 @@
+"""The memory of neighbour lists (GPU): a list can be exported to another
+process, as any allocation of its own; a freed list's block serves the next list
+of about its length, and larger ones go back to the driver, as does what the
+library's pool holds unused above 8 GB."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import random_box
+
+pytestmark = pytest.mark.gpu
+
+GB = 1 << 30
+
+
+def gas(torch, n, neighbours, seed):
+    """(n, 3) float32 positions on the GPU, sites of a sparse grid, and the box side at cutoff 1."""
+    side = float(np.float32((n * 4.0 / 3.0 * np.pi / neighbours) ** (1.0 / 3.0)))
+    m = int(np.ceil((n / 0.8) ** (1.0 / 3.0)))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    site = torch.randperm(m ** 3, generator=g, device="cuda")[:n]
+    cell = torch.stack([site % m, site // m % m, site // (m * m)], 1).float()
+    x = (cell + torch.rand((n, 3), generator=g, device="cuda") * 0.9) * (side / m)
+    x[x >= side] = 0.0
+    return x.contiguous(), side
+
+
+def free_bytes(torch):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_export_to_another_process(built_lib):
+    """cudaIpcGetMemHandle takes the list's address."""
+    torch = pytest.importorskip("torch")
+    import irregular_gb300 as irr
+    torch.zeros(1, device="cuda")
+    pos, side = random_box(5000, 0.9, 1)
+    lst = irr.neighbor_build(pos, float(side), 6.25)
+    cudart = irr._cudart()
+    handle = (C.c_char * 64)()
+    assert cudart.cudaIpcGetMemHandle(handle, C.c_void_p(lst.ptr)) == 0
+    lst.close()
+
+
+def test_next_list(built_lib, oracle_lib):
+    """Blocks taken again hold the next list, whatever was in them; lists of
+    several lengths live at once are apart."""
+    import irregular_gb300 as irr
+    want = {}
+    for k, n in enumerate([4000, 4100, 900, 30000, 3900, 29000]):
+        pos, side = random_box(n, 0.9, k)
+        want[n] = (pos, float(side), oracle_lib.neighbor_half_list(pos, float(side), np.float32(6.25)))
+    rng = np.random.default_rng(3)
+    live = []
+    for _ in range(200):
+        n = int(rng.choice(list(want)))
+        pos, side, ref = want[n]
+        live.append((irr.neighbor_build(pos, side, 6.25), ref))
+        if len(live) > 4:
+            got, ref = live.pop(int(rng.integers(len(live))))
+            assert np.array_equal(got.to_host(), ref)
+            got.close()
+    spans = sorted((x.ptr, x.ptr + 8 * x.count) for x, _ in live)
+    assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
+    for got, ref in live:
+        assert np.array_equal(got.to_host(), ref)
+        got.close()
+
+
+def test_freed_lists_go_back(built_lib):
+    torch = pytest.importorskip("torch")
+    import irregular_gb300 as irr
+    pos, side = gas(torch, 5_000_000, 64, 2)
+    irr.neighbor_build(pos, side, 1.0).close()  # the pool's temporaries, once
+    before = free_bytes(torch)
+    lists = [irr.neighbor_build(pos, side, 1.0) for _ in range(3)]
+    size = 8 * lists[0].count
+    assert size > GB
+    assert before - free_bytes(torch) > 2.9 * size
+    for x in lists:
+        x.close()
+    assert before - free_bytes(torch) < 0.1 * size
+
+
+def test_unused_pool_memory_goes_back(built_lib):
+    """A list whose slots alone take more than the pool keeps."""
+    torch = pytest.importorskip("torch")
+    import irregular_gb300 as irr
+    pos, side = gas(torch, 24_000_000, 64, 4)
+    before = free_bytes(torch)
+    irr.neighbor_build(pos, side, 1.0).close()
+    assert before - free_bytes(torch) < 8.5 * GB
