@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "irr_internal.cuh"
+#include "irr_list_rule.h"
 #include "irr_trace.cuh"
 #include "../../include/irregular_gb300.h"
 
@@ -756,12 +757,11 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
     cell_order_kernel<<<grid_of(n), 256, 0, s>>>(pos, sorted, n, pos_c);
     IRR_CUDA_TRY(cudaGetLastError());
     // rows in order: one search pass into slots, where the cells decide the images
-    // and the slots (a third more than the mean sphere's nodes, and some) fit
     double volume = 1.0;
     for (int c = 0; c < 3; c++) volume *= g.periodic ? (double)box : std::max(g.nc[c] / g.inv[c], std::sqrt((double)cut2));
     const double sphere = volume > 0 ? 4.18879 * cut2 * std::sqrt((double)cut2) * n / volume : (double)n;
-    const uint32_t cap = sphere < kRowSortMax ? ((uint32_t)(1.35 * sphere) + 31u) / 8u * 8u : 0u;
-    if (sort_rows && cap > 0 && cap <= (uint32_t)kRowSortMax && (g.fast || !g.periodic)) {
+    const uint32_t cap = sort_rows && (g.fast || !g.periodic) ? list_slots(sphere, n, kRowSortMax) : 0u;
+    if (cap > 0) {
         int32_t* slots = nullptr;
         if (irr_malloc_async((void**)&slots, sizeof(int32_t) * cap * (size_t)n, s) != cudaSuccess) {
             cudaGetLastError();  // no room: count first
@@ -776,9 +776,7 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
             uint32_t got[2] = {0, 0};
             IRR_CUDA_TRY(cudaMemcpyAsync(got, aux, sizeof(got), cudaMemcpyDeviceToHost, s));
             IRR_CUDA_TRY(cudaStreamSynchronize(s));
-            // (a total that does not fit 32 bits needs rows the slots do not hold, or more
-            // than 2^31 nodes' worth of memory: the counting path reports it)
-            const bool done = !got[1] && (double)cap * (double)n < 4294967296.0 && got[0] <= 0x7fffffffu;
+            const bool done = !got[1] && got[0] <= 0x7fffffffu;
             int2* edges = nullptr;
             if (done && got[0] > 0) {
                 IRR_CUDA_TRY(irr_malloc_list((void**)&edges, sizeof(int2) * got[0]));
