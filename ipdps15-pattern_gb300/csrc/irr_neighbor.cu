@@ -725,133 +725,6 @@ cudaError_t make_grid(const float4* pos, int64_t n, float box, float cut2, Grid*
 
 }  // namespace
 
-cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float cut2,
-                                int2** d_edges, int64_t* num_edges, cudaStream_t s, bool sort_rows)
-{
-    *d_edges = nullptr;
-    *num_edges = 0;
-    if (n <= 1) return cudaSuccess;
-    Grid g{};
-    IRR_CUDA_TRY(make_grid(pos, n, box, cut2, &g, s));
-    const int64_t ncell = (int64_t)g.nc[0] * g.nc[1] * g.nc[2];
-    uint32_t *keys = nullptr, *keys_tmp = nullptr, *cell_start = nullptr, *cnt = nullptr;
-    int32_t *sorted = nullptr, *vals_tmp = nullptr, *nbr = nullptr;
-    IRR_CUDA_TRY(irr_malloc_async((void**)&keys, sizeof(uint32_t) * n, s));
-    IRR_CUDA_TRY(irr_malloc_async((void**)&keys_tmp, sizeof(uint32_t) * n, s));
-    IRR_CUDA_TRY(irr_malloc_async((void**)&sorted, sizeof(int32_t) * n, s));
-    IRR_CUDA_TRY(irr_malloc_async((void**)&vals_tmp, sizeof(int32_t) * n, s));
-    IRR_CUDA_TRY(irr_malloc_async((void**)&cell_start, sizeof(uint32_t) * (ncell + 1), s));
-    // cnt[n + 1]: the flag that some position lies outside the box
-    IRR_CUDA_TRY(irr_malloc_async((void**)&cnt, sizeof(uint32_t) * (n + 2), s));
-    int* outside = reinterpret_cast<int*>(cnt + n + 1);
-    IRR_CUDA_TRY(cudaMemsetAsync(cell_start, 0, sizeof(uint32_t) * (ncell + 1), s));
-    IRR_CUDA_TRY(cudaMemsetAsync(outside, 0, sizeof(int), s));
-    cell_keys_kernel<<<grid_of(n), 256, 0, s>>>(pos, n, g, keys, sorted, cell_start, outside);
-    IRR_CUDA_TRY(cudaGetLastError());
-    int bits = 1;
-    while (bits < 32 && ((int64_t)1 << bits) < ncell) bits++;
-    IRR_CUDA_TRY(radix_sort_pairs(keys, sorted, keys_tmp, vals_tmp, n, bits, s));
-    IRR_CUDA_TRY(scan_exclusive_u32(cell_start, cell_start, ncell + 1, nullptr, s));
-    float4* pos_c = nullptr;
-    IRR_CUDA_TRY(irr_malloc_async((void**)&pos_c, sizeof(float4) * n, s));
-    cell_order_kernel<<<grid_of(n), 256, 0, s>>>(pos, sorted, n, pos_c);
-    IRR_CUDA_TRY(cudaGetLastError());
-    // rows in order: one search pass into slots, where the cells decide the images
-    double volume = 1.0;
-    for (int c = 0; c < 3; c++) volume *= g.periodic ? (double)box : std::max(g.nc[c] / g.inv[c], std::sqrt((double)cut2));
-    const double sphere = volume > 0 ? 4.18879 * cut2 * std::sqrt((double)cut2) * n / volume : (double)n;
-    const uint32_t cap = sort_rows && (g.fast || !g.periodic) ? list_slots(sphere, n, kRowSortMax) : 0u;
-    if (cap > 0) {
-        int32_t* slots = nullptr;
-        if (irr_malloc_async((void**)&slots, sizeof(int32_t) * cap * (size_t)n, s) != cudaSuccess) {
-            cudaGetLastError();  // no room: count first
-        } else {
-            uint32_t* aux = keys_tmp;  // reuse: the total, the flag that slots did not do
-            IRR_CUDA_TRY(cudaMemsetAsync(aux, 0, 2 * sizeof(uint32_t), s));
-            slot_partners_kernel<<<grid_of(n), 256, 0, s>>>(pos_c, keys, cell_start, n, g, outside, cap, cnt, slots,
-                                                            reinterpret_cast<int*>(aux + 1));
-            IRR_CUDA_TRY(cudaGetLastError());
-            IRR_CUDA_TRY(cudaMemsetAsync(cnt + n, 0, sizeof(uint32_t), s));
-            IRR_CUDA_TRY(scan_exclusive_u32(cnt, cnt, n + 1, aux, s));
-            uint32_t got[2] = {0, 0};
-            IRR_CUDA_TRY(cudaMemcpyAsync(got, aux, sizeof(got), cudaMemcpyDeviceToHost, s));
-            IRR_CUDA_TRY(cudaStreamSynchronize(s));
-            const bool done = !got[1] && got[0] <= 0x7fffffffu;
-            int2* edges = nullptr;
-            if (done && got[0] > 0) {
-                IRR_CUDA_TRY(irr_malloc_list((void**)&edges, sizeof(int2) * got[0]));
-                IRR_CUDA_TRY(launch_slot_pairs(cnt, sorted, n, slots, cap, edges, s));
-            }
-            void* tmp[] = {slots, keys, keys_tmp, sorted, vals_tmp, cell_start, cnt, pos_c};
-            for (void* q : tmp)
-                if (done || q == slots) IRR_CUDA_TRY(cudaFreeAsync(q, s));
-            if (done) {
-                IRR_CUDA_TRY(cudaStreamSynchronize(s));
-                *d_edges = edges;
-                *num_edges = got[0];
-                return cudaSuccess;
-            }
-        }
-    }
-    // rows in any order are asked for: the half stencil, where the box allows it
-    const bool half = !sort_rows && g.nc[0] >= 3 && g.nc[1] >= 3 && g.nc[2] >= 3;
-    if (half)
-        pairs_half_kernel<false><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
-                                                            cnt, nullptr, nullptr);
-    else
-        pairs_kernel<false><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside, cnt,
-                                                       nullptr, nullptr, nullptr, 0);
-    IRR_CUDA_TRY(cudaGetLastError());
-    IRR_CUDA_TRY(cudaMemsetAsync(cnt + n, 0, sizeof(uint32_t), s));
-    uint32_t* d_total = keys_tmp;  // reuse as the total's slot
-    IRR_CUDA_TRY(scan_exclusive_u32(cnt, cnt, n + 1, d_total, s));
-    uint32_t total = 0;
-    IRR_CUDA_TRY(cudaMemcpyAsync(&total, d_total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    IRR_CUDA_TRY(cudaStreamSynchronize(s));
-    if ((int64_t)total > 0x7fffffffLL) {
-        void* tmp[] = {keys, keys_tmp, sorted, vals_tmp, cell_start, cnt, pos_c};
-        for (void* q : tmp) cudaFreeAsync(q, s);
-        return cudaErrorInvalidValue;
-    }
-    int2* edges = nullptr;
-    if (total > 0) {
-        IRR_CUDA_TRY(sort_rows ? irr_malloc_list((void**)&edges, sizeof(int2) * total)
-                               : irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
-        if (sort_rows) {
-            uint32_t longest = 0;
-            IRR_CUDA_TRY(max_row_len(cnt, n, &longest, s));
-            const int sort_here = longest > (uint32_t)kRowSortMax;
-            IRR_CUDA_TRY(irr_malloc_async((void**)&nbr, sizeof(int32_t) * total, s));
-            pairs_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
-                                                          nullptr, cnt, nbr, nullptr, sort_here);
-            IRR_CUDA_TRY(cudaGetLastError());
-            if (!sort_here) IRR_CUDA_TRY(launch_row_sort(cnt, n, nbr, s));
-            expand_pairs_kernel<<<grid_of(32 * n), 256, 0, s>>>(cnt, nbr, n, edges);
-            IRR_CUDA_TRY(cudaGetLastError());
-            IRR_CUDA_TRY(cudaFreeAsync(nbr, s));
-        } else if (half) {
-            pairs_half_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g,
-                                                               outside, nullptr, cnt, edges);
-            IRR_CUDA_TRY(cudaGetLastError());
-        } else {
-            pairs_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
-                                                          nullptr, cnt, nullptr, edges, 0);
-            IRR_CUDA_TRY(cudaGetLastError());
-        }
-    }
-    IRR_CUDA_TRY(cudaFreeAsync(keys, s));
-    IRR_CUDA_TRY(cudaFreeAsync(keys_tmp, s));
-    IRR_CUDA_TRY(cudaFreeAsync(sorted, s));
-    IRR_CUDA_TRY(cudaFreeAsync(vals_tmp, s));
-    IRR_CUDA_TRY(cudaFreeAsync(cell_start, s));
-    IRR_CUDA_TRY(cudaFreeAsync(cnt, s));
-    IRR_CUDA_TRY(cudaFreeAsync(pos_c, s));
-    IRR_CUDA_TRY(cudaStreamSynchronize(s));
-    *d_edges = edges;
-    *num_edges = total;
-    return cudaSuccess;
-}
-
 namespace {
 
 // Stream-ordered temporaries freed on every return.
@@ -871,6 +744,152 @@ struct Temps {
         for (void* q : p) cudaFreeAsync(q, s);
     }
 };
+
+// One search pass into slots of cap per node, then the list from them.  *done is
+// false where the slots do not do (no room for them or for the list beside
+// them, a node of more than cap partners, cells that do not decide the images):
+// the caller then counts first.  aux: 2 words.
+cudaError_t list_by_slots(const float4* pos_c, const uint32_t* keys, const int32_t* sorted, const uint32_t* cell_start,
+                          int64_t n, const Grid& g, const int* outside, uint32_t cap, uint32_t* cnt, uint32_t* aux,
+                          int2** d_edges, int64_t* num_edges, bool* done, cudaStream_t s)
+{
+    *done = false;
+    Temps tmp{s, {}};
+    int32_t* slots = nullptr;
+    cudaError_t e = tmp.get(&slots, (size_t)cap * (size_t)n);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
+    IRR_CUDA_TRY(cudaMemsetAsync(aux, 0, 2 * sizeof(uint32_t), s));
+    slot_partners_kernel<<<grid_of(n), 256, 0, s>>>(pos_c, keys, cell_start, n, g, outside, cap, cnt, slots,
+                                                    reinterpret_cast<int*>(aux + 1));
+    IRR_CUDA_TRY(cudaGetLastError());
+    IRR_CUDA_TRY(cudaMemsetAsync(cnt + n, 0, sizeof(uint32_t), s));
+    IRR_CUDA_TRY(scan_exclusive_u32(cnt, cnt, n + 1, aux, s));
+    uint32_t got[2] = {0, 0};
+    IRR_CUDA_TRY(cudaMemcpyAsync(got, aux, sizeof(got), cudaMemcpyDeviceToHost, s));
+    IRR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (got[1] || got[0] > 0x7fffffffu) return cudaSuccess;
+    if (got[0] > 0) {
+        int2* edges = nullptr;
+        e = irr_malloc_list((void**)&edges, sizeof(int2) * got[0]);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
+        e = launch_slot_pairs(cnt, sorted, n, slots, cap, edges, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            irr_free_list(edges);
+            return e;
+        }
+        *d_edges = edges;
+    }
+    *num_edges = got[0];
+    *done = true;
+    return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float cut2,
+                                int2** d_edges, int64_t* num_edges, cudaStream_t s, bool sort_rows)
+{
+    *d_edges = nullptr;
+    *num_edges = 0;
+    if (n <= 1) return cudaSuccess;
+    Grid g{};
+    IRR_CUDA_TRY(make_grid(pos, n, box, cut2, &g, s));
+    const int64_t ncell = (int64_t)g.nc[0] * g.nc[1] * g.nc[2];
+    Temps tmp{s, {}};
+    uint32_t *keys = nullptr, *keys_tmp = nullptr, *cell_start = nullptr, *cnt = nullptr;
+    int32_t *sorted = nullptr, *vals_tmp = nullptr;
+    float4* pos_c = nullptr;
+    IRR_CUDA_TRY(tmp.get(&keys, n));
+    IRR_CUDA_TRY(tmp.get(&keys_tmp, n));
+    IRR_CUDA_TRY(tmp.get(&sorted, n));
+    IRR_CUDA_TRY(tmp.get(&vals_tmp, n));
+    IRR_CUDA_TRY(tmp.get(&cell_start, ncell + 1));
+    // cnt[n + 1]: the flag that some position lies outside the box
+    IRR_CUDA_TRY(tmp.get(&cnt, n + 2));
+    int* outside = reinterpret_cast<int*>(cnt + n + 1);
+    IRR_CUDA_TRY(cudaMemsetAsync(cell_start, 0, sizeof(uint32_t) * (ncell + 1), s));
+    IRR_CUDA_TRY(cudaMemsetAsync(outside, 0, sizeof(int), s));
+    cell_keys_kernel<<<grid_of(n), 256, 0, s>>>(pos, n, g, keys, sorted, cell_start, outside);
+    IRR_CUDA_TRY(cudaGetLastError());
+    int bits = 1;
+    while (bits < 32 && ((int64_t)1 << bits) < ncell) bits++;
+    IRR_CUDA_TRY(radix_sort_pairs(keys, sorted, keys_tmp, vals_tmp, n, bits, s));
+    IRR_CUDA_TRY(scan_exclusive_u32(cell_start, cell_start, ncell + 1, nullptr, s));
+    IRR_CUDA_TRY(tmp.get(&pos_c, n));
+    cell_order_kernel<<<grid_of(n), 256, 0, s>>>(pos, sorted, n, pos_c);
+    IRR_CUDA_TRY(cudaGetLastError());
+    // rows in order: one search pass into slots, where the cells decide the images
+    double volume = 1.0;
+    for (int c = 0; c < 3; c++) volume *= g.periodic ? (double)box : std::max(g.nc[c] / g.inv[c], std::sqrt((double)cut2));
+    const double sphere = volume > 0 ? 4.18879 * cut2 * std::sqrt((double)cut2) * n / volume : (double)n;
+    const uint32_t cap = sort_rows && (g.fast || !g.periodic) ? list_slots(sphere, n, kRowSortMax) : 0u;
+    if (cap > 0) {
+        bool done = false;
+        IRR_CUDA_TRY(list_by_slots(pos_c, keys, sorted, cell_start, n, g, outside, cap, cnt, keys_tmp, d_edges,
+                                   num_edges, &done, s));
+        if (done) return cudaSuccess;
+    }
+    // rows in any order are asked for: the half stencil, where the box allows it
+    const bool half = !sort_rows && g.nc[0] >= 3 && g.nc[1] >= 3 && g.nc[2] >= 3;
+    if (half)
+        pairs_half_kernel<false><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
+                                                            cnt, nullptr, nullptr);
+    else
+        pairs_kernel<false><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside, cnt,
+                                                       nullptr, nullptr, nullptr, 0);
+    IRR_CUDA_TRY(cudaGetLastError());
+    IRR_CUDA_TRY(cudaMemsetAsync(cnt + n, 0, sizeof(uint32_t), s));
+    uint32_t* d_total = keys_tmp;  // reuse as the total's slot
+    IRR_CUDA_TRY(scan_exclusive_u32(cnt, cnt, n + 1, d_total, s));
+    uint32_t total = 0;
+    IRR_CUDA_TRY(cudaMemcpyAsync(&total, d_total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    IRR_CUDA_TRY(cudaStreamSynchronize(s));
+    if ((int64_t)total > 0x7fffffffLL) return cudaErrorInvalidValue;
+    if (total == 0) return cudaSuccess;
+    int2* edges = nullptr;
+    IRR_CUDA_TRY(sort_rows ? irr_malloc_list((void**)&edges, sizeof(int2) * total)
+                           : irr_malloc_async((void**)&edges, sizeof(int2) * total, s));
+    auto write = [&]() -> cudaError_t {
+        if (sort_rows) {
+            uint32_t longest = 0;
+            IRR_CUDA_TRY(max_row_len(cnt, n, &longest, s));
+            const int sort_here = longest > (uint32_t)kRowSortMax;
+            int32_t* nbr = nullptr;
+            IRR_CUDA_TRY(tmp.get(&nbr, total));
+            pairs_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
+                                                          nullptr, cnt, nbr, nullptr, sort_here);
+            IRR_CUDA_TRY(cudaGetLastError());
+            if (!sort_here) IRR_CUDA_TRY(launch_row_sort(cnt, n, nbr, s));
+            expand_pairs_kernel<<<grid_of(32 * n), 256, 0, s>>>(cnt, nbr, n, edges);
+        } else if (half) {
+            pairs_half_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g,
+                                                               outside, nullptr, cnt, edges);
+        } else {
+            pairs_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
+                                                          nullptr, cnt, nullptr, edges, 0);
+        }
+        IRR_CUDA_TRY(cudaGetLastError());
+        return cudaStreamSynchronize(s);
+    };
+    const cudaError_t e = write();
+    if (e != cudaSuccess) {
+        if (sort_rows) {
+            cudaStreamSynchronize(s);
+            irr_free_list(edges);
+        } else {
+            cudaFreeAsync(edges, s);
+        }
+        return e;
+    }
+    *d_edges = edges;
+    *num_edges = total;
+    return cudaSuccess;
+}
+
+namespace {
 
 // Where the nodes are too few warps to hide the search's latency, 8 lanes share
 // a node's candidates: a search 35 us at 2,048 nodes (with a lane each 189 before

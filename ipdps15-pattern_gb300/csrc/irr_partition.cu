@@ -22,6 +22,7 @@
 // 4. Optionally the sliced layout (struct Sliced): the same entries regrouped
 //    so that one warp reads one contiguous line per step.
 #include <algorithm>
+#include <cstdlib>
 #include <mutex>
 #include <vector>
 
@@ -1418,6 +1419,26 @@ constexpr size_t kSpareBytes = 1ull << 30;
 std::mutex g_list_mutex;
 std::vector<ListBlock> g_lists, g_spares;
 
+#ifdef IRR_MEMORY_LIMIT
+// A build that tests what is done where memory is short: the pool and the lists
+// take at most $IRR_MEMORY_LIMIT bytes between them.
+bool no_room(int dev, size_t bytes)
+{
+    const char* v = std::getenv("IRR_MEMORY_LIMIT");
+    const cudaMemPool_t pool = pool_of(dev);
+    if (!v || !pool) return false;
+    cudaDeviceSynchronize();  // what is freed is free
+    uint64_t used = 0;
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    std::lock_guard<std::mutex> lock(g_list_mutex);
+    for (const ListBlock& b : g_lists) used += b.bytes;
+    for (const ListBlock& b : g_spares) used += b.bytes;
+    return used + bytes > std::strtoull(v, nullptr, 10);
+}
+#else
+bool no_room(int, size_t) { return false; }
+#endif
+
 // Frees the device's oldest spares until they take at most `keep` bytes.
 bool drop_spares(int dev, size_t keep)
 {
@@ -1446,7 +1467,10 @@ cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s)
     int dev = 0;
     IRR_CUDA_TRY(cudaGetDevice(&dev));
     const cudaMemPool_t pool = pool_of(dev);
-    auto get = [&]() { return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s); };
+    auto get = [&]() {
+        if (no_room(dev, bytes)) return cudaErrorMemoryAllocation;
+        return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+    };
     cudaError_t e = get();
     if (e == cudaErrorMemoryAllocation && drop_spares(dev, 0)) {
         cudaGetLastError();
@@ -1479,14 +1503,15 @@ cudaError_t irr_malloc_list(void** p, size_t bytes)
     constexpr size_t kPage = 2ull << 20;
     const size_t more = (bytes + bytes / 64 + kPage - 1) / kPage * kPage;
     size_t got = more;
-    cudaError_t e = cudaMalloc(p, got);
+    auto get = [&]() { return no_room(dev, got) ? cudaErrorMemoryAllocation : cudaMalloc(p, got); };
+    cudaError_t e = get();
     if (e == cudaErrorMemoryAllocation) {  // what is kept unused, and no more than the list
         cudaGetLastError();
         drop_spares(dev, 0);
         if (const cudaMemPool_t pool = pool_of(dev)) cudaMemPoolTrimTo(pool, 0);
         cudaGetLastError();
         got = bytes;
-        e = cudaMalloc(p, got);
+        e = get();
     }
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lock(g_list_mutex);
