@@ -623,13 +623,15 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
         if (lanes_per_row == 4 && h->shape.stage_smem) {
             if (!h->st.words) {
                 const RowSource rows{h->part.row_off, h->part.col, h->part.slots, h->part.cap};
-                cudaError_t se = build_staged(rows, n, h->m, false, &h->st, h->stream);
+                // (too little reuse to pay for staging: given up before it is written)
+                const int64_t most = want == IRR_LAYOUT_AUTO ? h->m / kStagedMinReuse : -1;
+                cudaError_t se = build_staged(rows, n, h->m, false, most, &h->st, h->stream);
                 // rows that touch more nodes than its tables hold: the wide limits
                 // (256,000 nodes with 248 neighbours each: 263 us sliced, 136 so).
                 // Where both apply they differ little (90 to 180 neighbours: 40
                 // to 84 us against 40 to 83) and the narrow ones are kept.
                 if (se == cudaErrorNotSupported && want == IRR_LAYOUT_AUTO)
-                    se = build_staged(rows, n, h->m, true, &h->st, h->stream);
+                    se = build_staged(rows, n, h->m, true, most, &h->st, h->stream);
                 if (se != cudaSuccess) {
                     cudaGetLastError();
                     free_staged(&h->st, h->stream);
@@ -641,8 +643,6 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
                                    : cuda_fail(h, se, "build staged layout");
                 }
             }
-            if (want == IRR_LAYOUT_AUTO && h->st.words && h->m < kStagedMinReuse * h->st.nids)
-                free_staged(&h->st, h->stream);  // too little reuse to pay for staging
             staged = h->st.words != nullptr || (n == 0 && want == IRR_LAYOUT_STAGED);
         } else if (want == IRR_LAYOUT_STAGED) {
             return fail(h, IRR_ERR_ARG, "the staged layout needs 4 lanes per row and stage_smem");

@@ -198,9 +198,13 @@ struct RowSource {
 // learns the sizes; the layout's words are still being written on s when it
 // returns, and may read src until then.
 // cudaErrorNotSupported (nothing allocated) when a slice alone exceeds the
-// limits above -- a row of more than ~440 entries (wide: 1023), or 8 rows
+// limits above -- a row of more than 888 entries (wide: 1023), or 8 rows
 // touching more than kHaloTabMax (wide: kHaloWideTabMax) distinct nodes.
-cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, Staged* st, cudaStream_t s);
+// most_ids >= 0: with more table ids than that the layout does not pay and is
+// not written: cudaErrorNotReady, or, from the wide cut, which stops there,
+// cudaErrorNotSupported.
+cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, int64_t most_ids, Staged* st,
+                         cudaStream_t s);
 // The rows back from the layout (items: st's, wherever they are now): col, at
 // row_off, each row ascending.
 cudaError_t rows_of_staged(const Staged& st, const WorkItem* items, const uint32_t* row_off, int64_t n, int32_t* col,

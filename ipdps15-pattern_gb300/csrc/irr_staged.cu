@@ -83,10 +83,11 @@ static_assert(kHaloSlicesPerItem == kPick, "the cut's maps have 8 states");
 static_assert(kHaloWideTabMax * 16 <= 0x3fff + 1, "a row's own offset fits the header's 14 bits");
 
 // What the kernels report.
-enum : uint32_t { kDoesNotFit = 1 };
+enum : uint32_t { kDoesNotFit = 1, kDoesNotPay = 2 };
 struct BuildTotals {
     unsigned long long words;
     unsigned long long ids;
+    unsigned long long cut_ids;  // of the tables cut so far (where they are limited)
     uint32_t items;
     uint32_t runs;
     uint32_t flags;
@@ -380,7 +381,8 @@ __device__ __forceinline__ int length_rank(const uint32_t* key, int m, int k)
 // One CTA per run: its items.  A run whose table fits is one item; else the
 // longest prefixes that fit, block by block.  For an item from row r0 with
 // entries from e0: tab[e0 + r0 + k] the k-th id of its table, place[e] (of the
-// items' entries) and own[r] (of its rows) their places in it.
+// items' entries) and own[r] (of its rows) their places in it.  most_ids: once
+// the tables hold more ids between them, the layout is refused (~0: never).
 template <class V>
 __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src, int64_t n,
                                                                  const int32_t* __restrict__ list,
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
                                                                  CutItem* __restrict__ cut,
                                                                  uint8_t* __restrict__ cuts, uint16_t* own,
                                                                  uint16_t* place, int32_t* __restrict__ tab,
-                                                                 BuildTotals* out)
+                                                                 unsigned long long most_ids, BuildTotals* out)
 {
     __shared__ __align__(16) GroupSet<V::kHash> set;
     __shared__ __align__(16) uint32_t gkey[V::kTab + 4];  // the groups: id / 32 << 6 | ids in the set
@@ -433,6 +435,12 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
         const int nb = run[b0];
         int from = 0;
         while (from < nb) {
+            if (from > 0) {  // (a run of one item does without)
+                __syncthreads();
+                if (tid == 0) refused = *(volatile uint32_t*)&out->flags;
+                __syncthreads();
+                if (refused) return;
+            }
             // all that is left at once; if that does not fit, block by block
             int to = nb;
             reset();
@@ -492,6 +500,8 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
                 cut[b0 + from] = CutItem{(uint32_t)(to - from), (uint32_t)ntab, words};
                 cuts[b0 + from] = 1;
                 atomicMax(&out->entries, src.row_off[r0 + m] - src.row_off[r0]);
+                if (most_ids != ~0ull && atomicAdd(&out->cut_ids, (unsigned long long)ntab) + ntab > most_ids)
+                    atomicOr(&out->flags, kDoesNotPay);
             }
             from = to;
         }
@@ -783,10 +793,12 @@ cudaError_t alloc_n(T** p, int64_t count, cudaStream_t s)
 }
 
 template <class V>
-cudaError_t build(const RowSource& src, int64_t n, int64_t m, Staged* st, cudaStream_t s)
+cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, Staged* st, cudaStream_t s)
 {
     const uint32_t* row_off = src.row_off;
     const int64_t S = (n + 7) / 8;
+    // the narrow cut goes on past the limit: a graph that does not fit may pay with the wide ones
+    const unsigned long long stop_at = V::kTab > kHaloTabMax && most_ids >= 0 ? (unsigned long long)most_ids : ~0ull;
     int dev = 0, sms = 0;
     IRR_CUDA_TRY(cudaGetDevice(&dev));
     IRR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -826,15 +838,15 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, Staged* st, cudaSt
             list_runs_kernel<<<(unsigned)std::min<int64_t>((tiles + 7) / 8, 8192), kRunTile, 0, s>>>(run, enter, S,
                                                                                                     list, d_out);
             cut_runs_kernel<V><<<(unsigned)std::min<int64_t>(S, (int64_t)sms * 128), V::kCutThreads, 0, s>>>(
-                src, n, list, run, cut, cuts, own, place, tab, d_out);
+                src, n, list, run, cut, cuts, own, place, tab, stop_at, d_out);
             place_items_kernel<false><<<kPlaceCtas, kPlaceThreads, 0, s>>>(n, S, cut, cuts, sums, items, d_out);
             place_items_kernel<true><<<kPlaceCtas, kPlaceThreads, 0, s>>>(n, S, cut, cuts, sums, items, d_out);
             IRR_CUDA_TRY(cudaGetLastError());
         }
         IRR_CUDA_TRY(cudaMemcpyAsync(&got, d_out, sizeof(got), cudaMemcpyDeviceToHost, s));
         IRR_CUDA_TRY(cudaStreamSynchronize(s));
-        if ((got.flags & kDoesNotFit) || got.words > 0xffffffffull || got.ids > 0x7fffffffull)
-            return cudaErrorNotSupported;
+        if (got.flags || got.words > 0xffffffffull || got.ids > 0x7fffffffull) return cudaErrorNotSupported;
+        if (most_ids >= 0 && (int64_t)got.ids > most_ids) return cudaErrorNotReady;
         out.nwords = (int64_t)got.words;
         out.nids = (int64_t)got.ids;
         out.nitems = got.items;
@@ -878,10 +890,11 @@ void free_staged(Staged* st, cudaStream_t s)
     *st = Staged{};
 }
 
-cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, Staged* st, cudaStream_t s)
+cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, int64_t most_ids, Staged* st,
+                         cudaStream_t s)
 {
     free_staged(st, s);
-    return wide ? build<WideItem>(src, n, m, st, s) : build<NarrowItem>(src, n, m, st, s);
+    return wide ? build<WideItem>(src, n, m, most_ids, st, s) : build<NarrowItem>(src, n, m, most_ids, st, s);
 }
 
 namespace {
