@@ -685,6 +685,57 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
 
 namespace {
 
+// irr_init without its checks; frees runs early where it can.
+int init_parts(irr_handle* h, uint32_t*& runs)
+{
+    cudaStream_t s = h->stream;
+    const int64_t n = h->n, e = h->e;
+    H_CUDA(h, launch_validate_edges(h->d_edges, e, n, h->d_status, runs, s), "validate edges");
+    int rc = check_status(h);
+    if (rc) return rc;
+    if (h->user_launch) return init_user(h, runs);
+    const size_t nb = (size_t)(n > 0 ? n : 1) * sizeof(float4);
+    H_CUDA(h, dalloc(h, &h->d_pos, nb), "allocate positions");
+    H_CUDA(h, dalloc(h, &h->d_force, nb), "allocate results");
+    H_CUDA(h, cudaMemsetAsync(h->d_force, 0, nb, s), "clear results");
+    h->dev_bytes = 2 * (int64_t)nb + (int64_t)h->raw_cap;
+    if (h->cfg.exec == IRR_EXEC_PLAIN) {
+        H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, nullptr, n, h->d_pos, s), "load node data");
+        h->raw_pending = false;
+        h->dev_bytes += (int64_t)h->edges_cap;
+        h->inited = true;
+        H_CUDA(h, cudaStreamSynchronize(s), "init");
+        return IRR_OK;
+    }
+    // partitioned: positions in the caller's order feed the partitioner
+    H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, nullptr, n, h->d_pos, s), "load node data");
+    PartitionOut p;
+    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, h->cfg.reorder, &p, s, h->cfg.order, runs, true);
+    dfree(h, runs);
+    h->part = p;
+    if (pe != cudaSuccess) {
+        free_layout(h);
+        return cuda_fail(h, pe, "build partition");
+    }
+    rc = apply_shard(h);
+    if (rc) {
+        free_layout(h);
+        return rc;
+    }
+    H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, h->part.perm, n, h->d_pos, s), "gather node data");
+    h->raw_pending = false;
+    H_CUDA(h, dalloc(h, &h->d_inst, sizeof(InstDesc)), "allocate instance descriptor");
+    h->shape.periodic = h->law.periodic;
+    h->inited = true;
+    rc = irr_ensure_layout(h, h->shape.lanes_per_row, h->shape.block_nodes);
+    if (rc) return rc;
+    // the half list is not needed by the partitioned kernel
+    dfree(h, h->d_edges);
+    h->edges_cap = 0;
+    H_CUDA(h, cudaStreamSynchronize(s), "init");
+    return IRR_OK;
+}
+
 int set_nodes_range_common(irr_handle* h, const void* src, int elm, int64_t first, int64_t count,
                            cudaMemcpyKind kind)
 {
@@ -956,58 +1007,19 @@ int irr_init(irr_handle* h)
     if (h->own_hi >= 0 && h->cfg.exec != IRR_EXEC_PARTITIONED)
         return fail(h, IRR_ERR_STATE, "a shard needs the partitioned executor");
     DeviceGuard dev_guard(h->device);
-    cudaStream_t s = h->stream;
-    const int64_t n = h->n, e = h->e;
-    // the list's runs of idx0, for the partitioner
+    // the list's runs of idx0, for the partitioner (which counts without them)
     uint32_t* runs = nullptr;
-    if (h->cfg.exec == IRR_EXEC_PARTITIONED) H_CUDA(h, dalloc(h, &runs, sizeof(uint32_t) * (size_t)(2 * n + 1)), "edge runs");
-    const cudaError_t ve = launch_validate_edges(h->d_edges, e, n, h->d_status, runs, s);
-    int rc = ve == cudaSuccess ? check_status(h) : cuda_fail(h, ve, "validate edges");
-    if (rc || h->user_launch) {
-        if (!rc) rc = init_user(h, runs);
-        dfree(h, runs);
-        return rc;
+    if (h->cfg.exec == IRR_EXEC_PARTITIONED &&
+        dalloc(h, &runs, sizeof(uint32_t) * (size_t)(2 * h->n + 1)) != cudaSuccess) {
+        cudaGetLastError();
+        runs = nullptr;
     }
-    const size_t nb = (size_t)(n > 0 ? n : 1) * sizeof(float4);
-    H_CUDA(h, dalloc(h, &h->d_pos, nb), "allocate positions");
-    H_CUDA(h, dalloc(h, &h->d_force, nb), "allocate results");
-    H_CUDA(h, cudaMemsetAsync(h->d_force, 0, nb, s), "clear results");
-    h->dev_bytes = 2 * (int64_t)nb + (int64_t)h->raw_cap;
-    if (h->cfg.exec == IRR_EXEC_PLAIN) {
-        H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, nullptr, n, h->d_pos, s), "load node data");
-        h->raw_pending = false;
-        h->dev_bytes += (int64_t)h->edges_cap;
-        h->inited = true;
-        H_CUDA(h, cudaStreamSynchronize(s), "init");
-        return IRR_OK;
-    }
-    // partitioned: positions in the caller's order feed the partitioner
-    H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, nullptr, n, h->d_pos, s), "load node data");
-    PartitionOut p;
-    cudaError_t pe = build_partition(h->d_pos, n, h->d_edges, e, h->cfg.reorder, &p, s, h->cfg.order, runs, true);
+    const int rc = init_parts(h, runs);
     dfree(h, runs);
-    h->part = p;
-    if (pe != cudaSuccess) {
-        free_layout(h);
-        return cuda_fail(h, pe, "build partition");
+    if (rc == IRR_ERR_NOMEM || rc == IRR_ERR_CUDA) {
+        free_layout(h);  // nothing half made: the next irr_init starts from the data given
     }
-    rc = apply_shard(h);
-    if (rc) {
-        free_layout(h);
-        return rc;
-    }
-    H_CUDA(h, launch_load_nodes(h->d_raw, h->raw_elm, h->part.perm, n, h->d_pos, s), "gather node data");
-    h->raw_pending = false;
-    H_CUDA(h, dalloc(h, &h->d_inst, sizeof(InstDesc)), "allocate instance descriptor");
-    h->shape.periodic = h->law.periodic;
-    h->inited = true;
-    rc = irr_ensure_layout(h, h->shape.lanes_per_row, h->shape.block_nodes);
-    if (rc) return rc;
-    // the half list is not needed by the partitioned kernel
-    dfree(h, h->d_edges);
-    h->edges_cap = 0;
-    H_CUDA(h, cudaStreamSynchronize(s), "init");
-    return IRR_OK;
+    return rc;
 }
 
 int irr_step(irr_handle* h)

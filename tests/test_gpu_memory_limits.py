@@ -49,3 +49,67 @@ print("done")
 
 def test_list(limited):
     assert "done" in run_script(limited, LIST)
+
+
+HANDLE = """
+import os
+import numpy as np
+import irregular_gb300 as irr
+from helpers import random_box
+from oracle import oracle as O
+n, rc = 100_000, 2.5
+pos, side = random_box(n, 64 / (4.0 / 3.0 * np.pi * rc ** 3), 3)
+edges = O.neighbor_half_list(pos, float(side), np.float32(rc * rc))
+e = len(edges)
+
+
+def handle(**cfg):
+    shard = cfg.pop("shard", False)
+    os.environ.pop("IRR_MEMORY_LIMIT", None)
+    h = irr.Handle(irr.default_config(map_idx=irr.IRR_MAP_LJ_MOLDYN, **cfg))
+    h.set_params(irr.moldyn_params(float(side), rc))
+    if shard:
+        h.set_shard(100, n // 2)
+    h.set_edges(edges)
+    h.set_nodes(pos, 12)
+    return h
+
+
+def result(h):
+    os.environ.pop("IRR_MEMORY_LIMIT", None)
+    h.step()
+    return h.get_result(elm_size=12).view(np.uint32), h.info().layout
+
+
+"""
+
+FAILED = HANDLE + """
+for cfg in (dict(layout=irr.IRR_LAYOUT_CSR), dict(exec=irr.IRR_EXEC_PLAIN), dict()):
+    h = handle(**cfg)
+    for limit in (8 * e + 13 * n, 8 * e + 29 * n, 8 * e + 50 * n, 15 * e) * 20:
+        os.environ["IRR_MEMORY_LIMIT"] = str(limit)
+        for call in (h.init, h.step):  # a step makes the set-up, or says why not
+            try:
+                call()
+            except irr.IrregularError as err:
+                assert err.status == irr.IRR_ERR_NOMEM, str(err)
+            else:
+                assert cfg.get("exec") == irr.IRR_EXEC_PLAIN and limit >= 8 * e + 50 * n, (cfg, limit)
+                h.close()
+                h = handle(**cfg)
+                break
+        if h.info().num_edges != e:
+            h.set_edges(edges)
+    # nothing was lost on the way: the set-up that fits alone fits after them
+    os.environ["IRR_MEMORY_LIMIT"] = str(40 * e)
+    h.init()
+    f64, sabs = O.lj_reduce_f64(pos.astype(np.float64), edges, O.lj_param(rc * rc, float(side), True))
+    got = result(h)[0].view(np.float32)
+    assert np.abs(got - f64).max() <= 1e-6 * np.abs(f64).max()
+    h.close()
+print("done")
+"""
+
+
+def test_failed_setup(limited):
+    assert "done" in run_script(limited, FAILED)
