@@ -374,6 +374,19 @@ int set_edges_common(irr_handle* h, const int32_t* src, int64_t e, cudaMemcpyKin
     return IRR_OK;
 }
 
+// part.col from the partitioner's slots.  Where the rows do not fit beside them
+// they are counted from the half list, which a set-up still holds.
+int pack_slots(irr_handle* h)
+{
+    cudaError_t e = partition_rows(&h->part, h->n, 2 * h->e, h->stream);
+    if (e == cudaErrorMemoryAllocation && h->d_edges) {
+        cudaGetLastError();
+        e = rows_by_counting(&h->part, h->n, h->d_edges, h->e, h->stream);
+    }
+    H_CUDA(h, e, "partition rows");
+    return IRR_OK;
+}
+
 // irr_set_shard: rows outside [own_lo, own_hi) (caller ids) lose their
 // entries; h->m = the entries left.
 int apply_shard(irr_handle* h)
@@ -385,7 +398,8 @@ int apply_shard(irr_handle* h)
     if (h->own_lo < 0 || h->own_lo > h->own_hi || h->own_hi > h->n)
         return fail(h, IRR_ERR_STATE, "shard rows [%lld, %lld) outside the %lld nodes", (long long)h->own_lo,
                     (long long)h->own_hi, (long long)h->n);
-    H_CUDA(h, partition_rows(&h->part, h->n, 2 * h->e, h->stream), "partition rows");
+    const int rc = pack_slots(h);
+    if (rc) return rc;
     H_CUDA(h, keep_rows(&h->part, h->n, h->own_lo, h->own_hi, &h->m, h->stream), "shard rows");
     return IRR_OK;
 }
@@ -598,8 +612,43 @@ int ensure_rows(irr_handle* h)
             return cuda_fail(h, e, "rows of the staged layout");
         }
     }
-    H_CUDA(h, partition_rows(&h->part, h->n, h->m, h->stream), "partition rows");
-    return IRR_OK;
+    return pack_slots(h);
+}
+
+// The staged layout into h->st (IRR_OK without it where AUTO goes without).
+int make_staged(irr_handle* h)
+{
+    const bool any = h->cfg.layout == IRR_LAYOUT_AUTO;
+    const int64_t most = any ? h->m / kStagedMinReuse : -1;  // given up before it is written
+    auto build = [&]() {
+        const RowSource rows{h->part.row_off, h->part.col, h->part.slots, h->part.cap};
+        cudaError_t se = build_staged(rows, h->n, h->m, false, most, &h->st, h->stream);
+        // rows that touch more nodes than its tables hold: the wide limits
+        // (256,000 nodes with 248 neighbours each: 263 us sliced, 136 so).
+        // Where both apply they differ little (90 to 180 neighbours: 40
+        // to 84 us against 40 to 83) and the narrow ones are kept.
+        if (se == cudaErrorNotSupported && any) se = build_staged(rows, h->n, h->m, true, most, &h->st, h->stream);
+        return se;
+    };
+    cudaError_t se = build();
+    if (se == cudaErrorMemoryAllocation && h->d_edges) {
+        // no room beside the slots (12 bytes an edge) and the half list (8): the
+        // rows counted (8), then the list given up
+        cudaGetLastError();
+        if (h->part.slots)
+            H_CUDA(h, rows_by_counting(&h->part, h->n, h->d_edges, h->e, h->stream), "partition rows");
+        dfree(h, h->d_edges);
+        h->edges_cap = 0;
+        se = build();
+    }
+    if (se == cudaSuccess) return IRR_OK;
+    cudaGetLastError();
+    free_staged(&h->st, h->stream);
+    if (any) return IRR_OK;
+    return se == cudaErrorNotSupported
+               ? fail(h, IRR_ERR_CAPACITY, "staged layout: 8 rows touch more than %d nodes, or a row is too long",
+                      kHaloTabMax)
+               : cuda_fail(h, se, "build staged layout");
 }
 
 }  // namespace
@@ -612,7 +661,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     DeviceGuard dev_guard(h->device);
     // no launch may use the old layout: a batch's steps read it on the batch's stream
     H_CUDA(h, h->d_items ? cudaDeviceSynchronize() : cudaStreamSynchronize(h->stream), "layout");
-    const int64_t n = h->n, e = h->e;
+    const int64_t n = h->n;
     h->shape.lanes_per_row = lanes_per_row;
     h->shape.block_nodes = block_nodes;
     const int want = h->cfg.layout;
@@ -622,26 +671,8 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     if (want == IRR_LAYOUT_STAGED || (want == IRR_LAYOUT_AUTO && kAutoStaged && staged_ok)) {
         if (lanes_per_row == 4 && h->shape.stage_smem) {
             if (!h->st.words) {
-                const RowSource rows{h->part.row_off, h->part.col, h->part.slots, h->part.cap};
-                // (too little reuse to pay for staging: given up before it is written)
-                const int64_t most = want == IRR_LAYOUT_AUTO ? h->m / kStagedMinReuse : -1;
-                cudaError_t se = build_staged(rows, n, h->m, false, most, &h->st, h->stream);
-                // rows that touch more nodes than its tables hold: the wide limits
-                // (256,000 nodes with 248 neighbours each: 263 us sliced, 136 so).
-                // Where both apply they differ little (90 to 180 neighbours: 40
-                // to 84 us against 40 to 83) and the narrow ones are kept.
-                if (se == cudaErrorNotSupported && want == IRR_LAYOUT_AUTO)
-                    se = build_staged(rows, n, h->m, true, most, &h->st, h->stream);
-                if (se != cudaSuccess) {
-                    cudaGetLastError();
-                    free_staged(&h->st, h->stream);
-                    if (want == IRR_LAYOUT_STAGED)
-                        return se == cudaErrorNotSupported
-                                   ? fail(h, IRR_ERR_CAPACITY,
-                                          "staged layout: 8 rows touch more than %d nodes, or a row is too long",
-                                          kHaloTabMax)
-                                   : cuda_fail(h, se, "build staged layout");
-                }
+                const int rc = make_staged(h);
+                if (rc) return rc;
             }
             staged = h->st.words != nullptr || (n == 0 && want == IRR_LAYOUT_STAGED);
         } else if (want == IRR_LAYOUT_STAGED) {
@@ -1017,7 +1048,9 @@ int irr_init(irr_handle* h)
     const int rc = init_parts(h, runs);
     dfree(h, runs);
     if (rc == IRR_ERR_NOMEM || rc == IRR_ERR_CUDA) {
-        free_layout(h);  // nothing half made: the next irr_init starts from the data given
+        // nothing half made: the next irr_init starts from the data given
+        free_layout(h);
+        if (!h->d_edges) h->e = -1;
     }
     return rc;
 }

@@ -284,6 +284,24 @@ inline cudaError_t irr_malloc_async(T** p, size_t bytes, cudaStream_t s)
     return irr_malloc_async(reinterpret_cast<void**>(p), bytes, s);
 }
 
+// Stream-ordered temporaries freed on every return.
+struct Temps {
+    cudaStream_t s;
+    std::vector<void*> p;
+    template <typename T>
+    cudaError_t get(T** out, size_t count)
+    {
+        *out = nullptr;
+        const cudaError_t e = irr_malloc_async(out, sizeof(T) * (count ? count : 1), s);
+        if (e == cudaSuccess) p.push_back(*out);
+        return e;
+    }
+    ~Temps()
+    {
+        for (void* q : p) cudaFreeAsync(q, s);
+    }
+};
+
 // Edge lists, which are the caller's: cudaMalloc'd, so that peers and other
 // processes reach them as any device memory.  irr_free_list, after the last use
 // of p by the device, keeps up to 1 GB of freed ones per device for the next
@@ -412,15 +430,18 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
                             int reorder, PartitionOut* out, cudaStream_t s, int curve = 0,
                             const uint32_t* runs = nullptr, bool keep_slots = false);
 // out->col (m entries) from out->slots, which are freed; nothing where there
-// are none.
+// are none.  On an error out is as it was.
 cudaError_t partition_rows(PartitionOut* out, int64_t n, int64_t m, cudaStream_t s);
+// out->row_off and out->col from the edges again, without slots, which are
+// freed: 8 bytes an edge and little more.
+cudaError_t rows_by_counting(PartitionOut* out, int64_t n, const int2* edges, int64_t e, cudaStream_t s);
 // An array of m entries, and the padding that reads of col may touch, cleared.
 cudaError_t alloc_col(int32_t** col, int64_t m, cudaStream_t s);
 // A shard's partition: rows whose caller id is outside [lo, hi) lose their
 // entries (row_off and col rebuilt, order kept); *m_out = entries left.
 cudaError_t keep_rows(PartitionOut* p, int64_t n, int64_t lo, int64_t hi, int64_t* m_out, cudaStream_t s);
-// Half neighbour list (irr_neighbor.cu); *d_edges is from irr_malloc_list
-// (unsorted: from the pool, on s); s is synchronised.
+// Half neighbour list (irr_neighbor.cu), written on s; *d_edges is from
+// irr_malloc_list (unsorted: from the pool, on s).
 // sort_rows == false returns the same pairs (i < j) in no particular order,
 // for a caller that re-sorts them anyway, like the partitioner (found by a
 // half-stencil search when the box has at least 3 cells per axis).

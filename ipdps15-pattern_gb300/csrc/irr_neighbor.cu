@@ -727,24 +727,6 @@ cudaError_t make_grid(const float4* pos, int64_t n, float box, float cut2, Grid*
 
 namespace {
 
-// Stream-ordered temporaries freed on every return.
-struct Temps {
-    cudaStream_t s;
-    std::vector<void*> p;
-    template <typename T>
-    cudaError_t get(T** out, size_t count)
-    {
-        *out = nullptr;
-        const cudaError_t e = irr_malloc_async((void**)out, sizeof(T) * (count ? count : 1), s);
-        if (e == cudaSuccess) p.push_back(*out);
-        return e;
-    }
-    ~Temps()
-    {
-        for (void* q : p) cudaFreeAsync(q, s);
-    }
-};
-
 // One search pass into slots of cap per node, then the list from them.  *done is
 // false where the slots do not do (no room for them or for the list beside
 // them, a node of more than cap partners, cells that do not decide the images):
@@ -775,7 +757,6 @@ cudaError_t list_by_slots(const float4* pos_c, const uint32_t* keys, const int32
         if (e == cudaErrorMemoryAllocation) cudaGetLastError();
         if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
         e = launch_slot_pairs(cnt, sorted, n, slots, cap, edges, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             irr_free_list(edges);
             return e;
@@ -871,8 +852,7 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
             pairs_kernel<true><<<grid_of(n), 256, 0, s>>>(pos_c, sorted, cell_start, n, g, outside,
                                                           nullptr, cnt, nullptr, edges, 0);
         }
-        IRR_CUDA_TRY(cudaGetLastError());
-        return cudaStreamSynchronize(s);
+        return cudaGetLastError();
     };
     const cudaError_t e = write();
     if (e != cudaSuccess) {

@@ -1080,10 +1080,83 @@ cudaError_t alloc_col(int32_t** col, int64_t m, cudaStream_t s)
 cudaError_t partition_rows(PartitionOut* out, int64_t n, int64_t m, cudaStream_t s)
 {
     if (!out->slots) return cudaSuccess;
-    IRR_CUDA_TRY(alloc_col(&out->col, m, s));
-    IRR_CUDA_TRY(launch_row_sort(out->row_off, n, out->col, s, out->slots, (uint32_t)out->cap));
+    int32_t* col = nullptr;
+    cudaError_t err = alloc_col(&col, m, s);
+    if (err == cudaSuccess) err = launch_row_sort(out->row_off, n, col, s, out->slots, (uint32_t)out->cap);
+    if (err != cudaSuccess) {
+        if (col) cudaFreeAsync(col, s);
+        return err;
+    }
+    out->col = col;
     IRR_CUDA_TRY(cudaFreeAsync(out->slots, s));
     out->slots = nullptr;
+    return cudaSuccess;
+}
+
+cudaError_t rows_by_counting(PartitionOut* out, int64_t n, const int2* edges, int64_t e, cudaStream_t s)
+{
+    if (out->slots) IRR_CUDA_TRY(cudaFreeAsync(out->slots, s));
+    out->slots = nullptr;
+    Temps tmp{s, {}};
+    uint32_t* deg = out->row_off;  // counted in place, then scanned
+    IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
+    int32_t* col = nullptr;
+    auto fill = [&]() -> cudaError_t {
+        IRR_CUDA_TRY(alloc_col(&col, 2 * e, s));
+        if (e > 0 && n > 0) {
+            // rows of at most kRowSortMax entries (every MD list): count, scan,
+            // fill at per-row cursors, sort each row -- the same (row, col) layout
+            // as the sorts below, in about a third of the passes
+            degree_kernel<<<grid_for(e), 256, 0, s>>>(edges, e, out->inv, deg);
+            IRR_CUDA_TRY(cudaGetLastError());
+            uint32_t* d_max = nullptr;
+            IRR_CUDA_TRY(tmp.get(&d_max, 1));
+            IRR_CUDA_TRY(cudaMemsetAsync(d_max, 0, sizeof(uint32_t), s));
+            max_u32_kernel<<<grid_for(n), 256, 0, s>>>(deg, n, d_max);
+            IRR_CUDA_TRY(cudaGetLastError());
+            uint32_t max_deg = 0;
+            IRR_CUDA_TRY(cudaMemcpyAsync(&max_deg, d_max, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            IRR_CUDA_TRY(cudaStreamSynchronize(s));
+            if (max_deg <= (uint32_t)kRowSortMax) {
+                IRR_CUDA_TRY(scan_exclusive_u32(deg, out->row_off, n + 1, nullptr, s));
+                uint32_t* cursor = nullptr;
+                IRR_CUDA_TRY(tmp.get(&cursor, (size_t)n));
+                IRR_CUDA_TRY(cudaMemcpyAsync(cursor, out->row_off, sizeof(uint32_t) * (size_t)n,
+                                             cudaMemcpyDeviceToDevice, s));
+                fill_rows_kernel<<<grid_for(e), 256, 0, s>>>(edges, e, out->inv, cursor, col);
+                IRR_CUDA_TRY(cudaGetLastError());
+                return launch_row_sort(out->row_off, n, col, s);
+            }
+            IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
+        }
+        if (e > 0) {
+            const int64_t m = 2 * e;
+            uint32_t *rows = nullptr, *rows_tmp = nullptr;
+            int32_t* cols_tmp = nullptr;
+            IRR_CUDA_TRY(tmp.get(&rows, (size_t)m));
+            IRR_CUDA_TRY(tmp.get(&rows_tmp, (size_t)m));
+            IRR_CUDA_TRY(tmp.get(&cols_tmp, (size_t)m));
+            entries_kernel<<<grid_for(e), 256, 0, s>>>(edges, e, out->inv, rows, col, deg);
+            IRR_CUDA_TRY(cudaGetLastError());
+            int bits = 1;
+            while (bits < 31 && ((int64_t)1 << bits) < n) bits++;
+            // (row, col) order: stable by column, then stable by row.  Ascending
+            // columns inside a row put the lanes of one gather on fewer cache
+            // lines (the rows of a warp are curve neighbours and share most of
+            // their neighbourhood), and make the layout independent of the
+            // order of the edge list.
+            IRR_CUDA_TRY(radix_sort_pairs(reinterpret_cast<uint32_t*>(col), reinterpret_cast<int32_t*>(rows), rows_tmp,
+                                          cols_tmp, m, bits, s));
+            IRR_CUDA_TRY(radix_sort_pairs(rows, col, rows_tmp, cols_tmp, m, bits, s));
+        }
+        return scan_exclusive_u32(deg, out->row_off, n + 1, nullptr, s);
+    };
+    const cudaError_t err = fill();
+    if (err != cudaSuccess) {
+        if (col) cudaFreeAsync(col, s);
+        return err;
+    }
+    out->col = col;
     return cudaSuccess;
 }
 
@@ -1098,22 +1171,19 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
     IRR_CUDA_TRY(alloc_async(&out->row_off, n + 1, s));
     const int g = grid_for(n);
     if (reorder && n > 1) {
+        Temps tmp{s, {}};
         // the box stays on the device: the host has no use for it
         float* box = nullptr;
-        IRR_CUDA_TRY(alloc_async(&box, 6 + 6 * kBboxParts, s));
+        IRR_CUDA_TRY(tmp.get(&box, 6 + 6 * kBboxParts));
         IRR_CUDA_TRY(launch_bbox(pos_user, n, box, s));
         uint32_t *keys = nullptr, *keys_tmp = nullptr;
         int32_t* vals_tmp = nullptr;
-        IRR_CUDA_TRY(alloc_async(&keys, n, s));
-        IRR_CUDA_TRY(alloc_async(&keys_tmp, n, s));
-        IRR_CUDA_TRY(alloc_async(&vals_tmp, n, s));
+        IRR_CUDA_TRY(tmp.get(&keys, (size_t)n));
+        IRR_CUDA_TRY(tmp.get(&keys_tmp, (size_t)n));
+        IRR_CUDA_TRY(tmp.get(&vals_tmp, (size_t)n));
         curve_key_kernel<<<g, 256, 0, s>>>(pos_user, n, box, curve, keys, out->perm);
-        IRR_CUDA_TRY(cudaFreeAsync(box, s));
         IRR_CUDA_TRY(cudaGetLastError());
         IRR_CUDA_TRY(radix_sort_pairs(keys, out->perm, keys_tmp, vals_tmp, n, 30, s));
-        IRR_CUDA_TRY(cudaFreeAsync(keys, s));
-        IRR_CUDA_TRY(cudaFreeAsync(keys_tmp, s));
-        IRR_CUDA_TRY(cudaFreeAsync(vals_tmp, s));
     } else if (n > 0) {
         iota_kernel<<<g, 256, 0, s>>>(out->perm, n);
         IRR_CUDA_TRY(cudaGetLastError());
@@ -1123,92 +1193,37 @@ cudaError_t build_partition(const float4* pos_user, int64_t n, const int2* edges
         IRR_CUDA_TRY(cudaGetLastError());
     }
     // directed entries, binned by row
-    uint32_t* deg = out->row_off;  // counted in place, then scanned
-    IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
     // slots of half as many entries again as the average row's, and some: MD rows
     // vary by a few standard deviations of a Poisson count
     const int64_t cap = n > 0 ? (3 * e / n + 24 + 7) / 8 * 8 : 0;
     if (runs && e > 0 && n > 0 && cap <= kRowSortMax) {
-        int* over = nullptr;
         if (alloc_async(&out->slots, n * cap, s) != cudaSuccess) {
             cudaGetLastError();  // no room: count first
             out->slots = nullptr;
         } else {
+            Temps tmp{s, {}};
+            uint32_t* deg = out->row_off;  // counted in place, then scanned
             out->cap = cap;
-            IRR_CUDA_TRY(alloc_async(&over, 1, s));
+            int* over = nullptr;
+            IRR_CUDA_TRY(tmp.get(&over, 1));
             IRR_CUDA_TRY(cudaMemsetAsync(over, 0, sizeof(int), s));
-            slot_rows_kernel<<<grid_for(32 * ((n + kSlotNodes - 1) / kSlotNodes)), 256, 0, s>>>(edges, runs, out->perm, out->inv, n, (uint32_t)cap, deg,
-                                                             out->slots, over);
+            IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
+            slot_rows_kernel<<<grid_for(32 * ((n + kSlotNodes - 1) / kSlotNodes)), 256, 0, s>>>(
+                edges, runs, out->perm, out->inv, n, (uint32_t)cap, deg, out->slots, over);
             IRR_CUDA_TRY(cudaGetLastError());
             int was_over = 0;
             IRR_CUDA_TRY(cudaMemcpyAsync(&was_over, over, sizeof(int), cudaMemcpyDeviceToHost, s));
-            IRR_CUDA_TRY(cudaFreeAsync(over, s));
             IRR_CUDA_TRY(cudaStreamSynchronize(s));
             if (!was_over) {
                 IRR_CUDA_TRY(scan_exclusive_u32(deg, out->row_off, n + 1, nullptr, s));
-                return keep_slots ? cudaSuccess : partition_rows(out, n, 2 * e, s);
+                if (keep_slots) return cudaSuccess;
+                const cudaError_t err = partition_rows(out, n, 2 * e, s);
+                if (err != cudaErrorMemoryAllocation) return err;
+                cudaGetLastError();  // no room for the rows beside their slots
             }
-            IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
-            IRR_CUDA_TRY(cudaFreeAsync(out->slots, s));
-            out->slots = nullptr;
         }
     }
-    IRR_CUDA_TRY(alloc_col(&out->col, 2 * e, s));
-    if (e > 0 && n > 0) {
-        // rows of at most kRowSortMax entries (every MD list): count, scan,
-        // fill at per-row cursors, sort each row -- the same (row, col) layout
-        // as the sorts below, in about a third of the passes
-        degree_kernel<<<grid_for(e), 256, 0, s>>>(edges, e, out->inv, deg);
-        IRR_CUDA_TRY(cudaGetLastError());
-        uint32_t* d_max = nullptr;
-        IRR_CUDA_TRY(alloc_async(&d_max, 1, s));
-        IRR_CUDA_TRY(cudaMemsetAsync(d_max, 0, sizeof(uint32_t), s));
-        max_u32_kernel<<<grid_for(n), 256, 0, s>>>(deg, n, d_max);
-        IRR_CUDA_TRY(cudaGetLastError());
-        uint32_t max_deg = 0;
-        IRR_CUDA_TRY(cudaMemcpyAsync(&max_deg, d_max, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        IRR_CUDA_TRY(cudaFreeAsync(d_max, s));
-        IRR_CUDA_TRY(cudaStreamSynchronize(s));
-        if (max_deg <= (uint32_t)kRowSortMax) {
-            IRR_CUDA_TRY(scan_exclusive_u32(deg, out->row_off, n + 1, nullptr, s));
-            uint32_t* cursor = nullptr;
-            IRR_CUDA_TRY(alloc_async(&cursor, n, s));
-            IRR_CUDA_TRY(cudaMemcpyAsync(cursor, out->row_off, sizeof(uint32_t) * (size_t)n,
-                                         cudaMemcpyDeviceToDevice, s));
-            fill_rows_kernel<<<grid_for(e), 256, 0, s>>>(edges, e, out->inv, cursor, out->col);
-            IRR_CUDA_TRY(cudaGetLastError());
-            IRR_CUDA_TRY(cudaFreeAsync(cursor, s));
-            IRR_CUDA_TRY(launch_row_sort(out->row_off, n, out->col, s));
-            return cudaSuccess;
-        }
-        IRR_CUDA_TRY(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * (size_t)(n + 1), s));
-    }
-    if (e > 0) {
-        const int64_t m = 2 * e;
-        uint32_t *rows = nullptr, *rows_tmp = nullptr;
-        int32_t* cols_tmp = nullptr;
-        IRR_CUDA_TRY(alloc_async(&rows, m, s));
-        IRR_CUDA_TRY(alloc_async(&rows_tmp, m, s));
-        IRR_CUDA_TRY(alloc_async(&cols_tmp, m, s));
-        entries_kernel<<<grid_for(e), 256, 0, s>>>(edges, e, out->inv, rows, out->col, deg);
-        IRR_CUDA_TRY(cudaGetLastError());
-        int bits = 1;
-        while (bits < 31 && ((int64_t)1 << bits) < n) bits++;
-        // (row, col) order: stable by column, then stable by row.  Ascending
-        // columns inside a row put the lanes of one gather on fewer cache
-        // lines (the rows of a warp are curve neighbours and share most of
-        // their neighbourhood), and make the layout independent of the
-        // order of the edge list.
-        IRR_CUDA_TRY(radix_sort_pairs(reinterpret_cast<uint32_t*>(out->col),
-                                      reinterpret_cast<int32_t*>(rows), rows_tmp,
-                                      cols_tmp, m, bits, s));
-        IRR_CUDA_TRY(radix_sort_pairs(rows, out->col, rows_tmp, cols_tmp, m, bits, s));
-        IRR_CUDA_TRY(cudaFreeAsync(rows, s));
-        IRR_CUDA_TRY(cudaFreeAsync(rows_tmp, s));
-        IRR_CUDA_TRY(cudaFreeAsync(cols_tmp, s));
-    }
-    IRR_CUDA_TRY(scan_exclusive_u32(deg, out->row_off, n + 1, nullptr, s));
-    return cudaSuccess;
+    return rows_by_counting(out, n, edges, e, s);
 }
 
 namespace {

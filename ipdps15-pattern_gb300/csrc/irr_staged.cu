@@ -83,15 +83,16 @@ static_assert(kHaloSlicesPerItem == kPick, "the cut's maps have 8 states");
 static_assert(kHaloWideTabMax * 16 <= 0x3fff + 1, "a row's own offset fits the header's 14 bits");
 
 // What the kernels report.
-enum : uint32_t { kDoesNotFit = 1, kDoesNotPay = 2 };
+enum : uint32_t { kDoesNotFit = 1, kDoesNotPay = 2, kNoScratch = 4 };
 struct BuildTotals {
     unsigned long long words;
     unsigned long long ids;
-    unsigned long long cut_ids;  // of the tables cut so far (where they are limited)
+    unsigned long long cut_ids;  // of the tables cut so far
     uint32_t items;
     uint32_t runs;
     uint32_t flags;
     uint32_t entries;  // of the largest item
+    uint32_t scratch;  // kNoScratch (no reason to stop the cut)
 };
 
 // One item as cut_runs_kernel finds it, at its first block.
@@ -99,6 +100,8 @@ struct CutItem {
     uint32_t blocks;
     uint32_t ntab;
     uint32_t words;
+    uint32_t pad;
+    unsigned long long tab0;  // its table's place in the scratch
 };
 
 // ---- the cut into runs
@@ -379,10 +382,11 @@ __device__ __forceinline__ int length_rank(const uint32_t* key, int m, int k)
 }
 
 // One CTA per run: its items.  A run whose table fits is one item; else the
-// longest prefixes that fit, block by block.  For an item from row r0 with
-// entries from e0: tab[e0 + r0 + k] the k-th id of its table, place[e] (of the
-// items' entries) and own[r] (of its rows) their places in it.  most_ids: once
-// the tables hold more ids between them, the layout is refused (~0: never).
+// longest prefixes that fit, block by block.  An item's table goes to the next
+// free place of tab (room ids in all: without room for a table the items are
+// counted on, and the layout is not to be written), place[e] (of the items'
+// entries) and own[r] (of its rows) are their places in it.  most_ids: once the
+// tables hold more ids between them, the layout is refused (~0: never).
 template <class V>
 __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src, int64_t n,
                                                                  const int32_t* __restrict__ list,
@@ -390,7 +394,8 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
                                                                  CutItem* __restrict__ cut,
                                                                  uint8_t* __restrict__ cuts, uint16_t* own,
                                                                  uint16_t* place, int32_t* __restrict__ tab,
-                                                                 unsigned long long most_ids, BuildTotals* out)
+                                                                 unsigned long long room, unsigned long long most_ids,
+                                                                 BuildTotals* out)
 {
     __shared__ __align__(16) GroupSet<V::kHash> set;
     __shared__ __align__(16) uint32_t gkey[V::kTab + 4];  // the groups: id / 32 << 6 | ids in the set
@@ -400,6 +405,7 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
     __shared__ int count;          // ids
     __shared__ uint32_t words;
     __shared__ uint32_t refused;
+    __shared__ unsigned long long tab0;
     const int tid = threadIdx.x;
     // other CTAs may raise the flag now: one thread looks, for all to leave or none
     if (tid == 0) refused = *(volatile uint32_t*)&out->flags;
@@ -470,6 +476,7 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
                     gat[x] = (uint16_t)k;
                 }
             }
+            if (tid == 0) tab0 = atomicAdd(&out->cut_ids, (unsigned long long)ntab);
             if (tid < 8 * kPick) key[tid] = tid < m ? length_key(src.row_off[r0 + tid + 1] - src.row_off[r0 + tid], tid) : 0u;
             __syncthreads();
             const int groups = ngroups;
@@ -477,7 +484,8 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
             // the item's words: slice j is as long as the row of rank 8 j
             if (tid < m && (length_rank(key, m, tid) & 7) == 0) atomicAdd(&words, 32u * (((key[tid] >> 6) + 7u) / 8u + 1u));
             __syncthreads();
-            const int64_t t0 = r0 + src.row_off[r0];
+            const unsigned long long t0 = tab0;
+            const bool fits = t0 + ntab <= room;
             for (int k = tid; k < groups; k += V::kCutThreads) {
                 const uint32_t mine = gkey[k];
                 uint32_t slot = 0;
@@ -489,7 +497,7 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
                 const uint32_t at = gat[k];
                 set.group[at].y = slot;
                 const int32_t id0 = (int32_t)(mine >> 6) << 5;
-                for (uint32_t b = set.group[at].x; b; b &= b - 1) tab[t0 + slot++] = id0 + __ffs(b) - 1;
+                for (uint32_t b = fits ? set.group[at].x : 0u; b; b &= b - 1) tab[t0 + slot++] = id0 + __ffs(b) - 1;
             }
             __syncthreads();
             // places: each thread those that it wrote
@@ -497,11 +505,11 @@ __global__ void __launch_bounds__(V::kCutThreads) cut_runs_kernel(RowSource src,
             if (tid < m) own[r0 + tid] = slot_of(own[r0 + tid]);
             place_slots(src.row_off, r0, m, place, slot_of);
             if (tid == 0) {
-                cut[b0 + from] = CutItem{(uint32_t)(to - from), (uint32_t)ntab, words};
+                cut[b0 + from] = CutItem{(uint32_t)(to - from), (uint32_t)ntab, words, 0u, t0};
                 cuts[b0 + from] = 1;
                 atomicMax(&out->entries, src.row_off[r0 + m] - src.row_off[r0]);
-                if (most_ids != ~0ull && atomicAdd(&out->cut_ids, (unsigned long long)ntab) + ntab > most_ids)
-                    atomicOr(&out->flags, kDoesNotPay);
+                if (t0 + ntab > most_ids) atomicOr(&out->flags, kDoesNotPay);
+                if (!fits) atomicOr(&out->scratch, kNoScratch);
             }
             from = to;
         }
@@ -540,7 +548,7 @@ __global__ void __launch_bounds__(kPlaceThreads) place_items_kernel(int64_t n, i
     for (int64_t t0 = s0; t0 < s1; t0 += kPlaceThreads) {
         const int64_t q = t0 + tid;
         const bool is = q < s1 && cuts[q];
-        CutItem c{0, 0, 0};
+        CutItem c{0, 0, 0, 0, 0};
         if (is) c = cut[q];
         Places v{is ? 1ull : 0ull, c.ntab, c.words};
         for (int off = 1; off < 32; off <<= 1) {
@@ -665,8 +673,8 @@ __device__ __forceinline__ void order_by_bank(uint16_t* row, uint32_t l, int shi
 template <class V>
 __global__ void __launch_bounds__(V::kFillWarps * 32, V::kFillCtas) fill_items_kernel(
     const uint32_t* __restrict__ row_off, const uint16_t* __restrict__ own_place, const uint16_t* __restrict__ place,
-    const int32_t* __restrict__ tab, int num_items, const WorkItem* __restrict__ items,
-    uint32_t* __restrict__ slice_off, int32_t* __restrict__ ids, uint32_t* __restrict__ words)
+    const int32_t* __restrict__ tab, const CutItem* __restrict__ cut, int num_items,
+    const WorkItem* __restrict__ items, uint32_t* __restrict__ slice_off, int32_t* __restrict__ ids, uint32_t* __restrict__ words)
 {
     constexpr int kWarps = V::kFillWarps, kThreads = 32 * kWarps, kRows = 8 * kPick / kWarps;
     static_assert(kRows <= 32, "a thread per row of the warp");
@@ -697,7 +705,8 @@ __global__ void __launch_bounds__(V::kFillWarps * 32, V::kFillCtas) fill_items_k
         for (int k = tid; k <= m; k += kThreads) off[k] = (uint32_t)(row_off[w.row0 + k] - base);
         for (int k = tid; k < 8 * kPick; k += kThreads)
             key[k] = k < m ? length_key(row_off[w.row0 + k + 1] - row_off[w.row0 + k], k) : 0u;
-        for (uint32_t k = tid; k < w.ntab; k += kThreads) ids[(int64_t)w.tab0 + k] = tab[e0 + w.row0 + k];
+        const int32_t* from = tab + cut[w.row0 / 8].tab0;
+        for (uint32_t k = tid; k < w.ntab; k += kThreads) ids[(int64_t)w.tab0 + k] = from[k];
         __syncthreads();
         for (int k = tid; k < m; k += kThreads) order[length_rank(key, m, k)] = k;
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -793,7 +802,7 @@ cudaError_t alloc_n(T** p, int64_t count, cudaStream_t s)
 }
 
 template <class V>
-cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, Staged* st, cudaStream_t s)
+cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, int64_t room, Staged* st, cudaStream_t s)
 {
     const uint32_t* row_off = src.row_off;
     const int64_t S = (n + 7) / 8;
@@ -828,7 +837,7 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, 
         IRR_CUDA_TRY(alloc_n(&d_out, 1, s));
         IRR_CUDA_TRY(alloc_n(&own, n, s));
         IRR_CUDA_TRY(alloc_n(&place, m + 8, s));  // read in whole eights
-        IRR_CUDA_TRY(alloc_n(&tab, n + m, s));    // a table is at most its item's rows and entries
+        IRR_CUDA_TRY(alloc_n(&tab, room, s));
         IRR_CUDA_TRY(cudaMemsetAsync(d_out, 0, sizeof(BuildTotals), s));
         IRR_CUDA_TRY(cudaMemsetAsync(cuts, 0, (size_t)(S > 0 ? S : 1), s));
         if (S > 0) {
@@ -838,7 +847,7 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, 
             list_runs_kernel<<<(unsigned)std::min<int64_t>((tiles + 7) / 8, 8192), kRunTile, 0, s>>>(run, enter, S,
                                                                                                     list, d_out);
             cut_runs_kernel<V><<<(unsigned)std::min<int64_t>(S, (int64_t)sms * 128), V::kCutThreads, 0, s>>>(
-                src, n, list, run, cut, cuts, own, place, tab, stop_at, d_out);
+                src, n, list, run, cut, cuts, own, place, tab, (unsigned long long)room, stop_at, d_out);
             place_items_kernel<false><<<kPlaceCtas, kPlaceThreads, 0, s>>>(n, S, cut, cuts, sums, items, d_out);
             place_items_kernel<true><<<kPlaceCtas, kPlaceThreads, 0, s>>>(n, S, cut, cuts, sums, items, d_out);
             IRR_CUDA_TRY(cudaGetLastError());
@@ -847,6 +856,7 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, 
         IRR_CUDA_TRY(cudaStreamSynchronize(s));
         if (got.flags || got.words > 0xffffffffull || got.ids > 0x7fffffffull) return cudaErrorNotSupported;
         if (most_ids >= 0 && (int64_t)got.ids > most_ids) return cudaErrorNotReady;
+        if (got.scratch) return cudaErrorMemoryAllocation;
         out.nwords = (int64_t)got.words;
         out.nids = (int64_t)got.ids;
         out.nitems = got.items;
@@ -863,7 +873,7 @@ cudaError_t build(const RowSource& src, int64_t n, int64_t m, int64_t most_ids, 
             static_assert((2 * V::kStream + 22) * sizeof(uint16_t) + 4096 <= 48 * 1024,
                           "with the kernel's own arrays inside the shared memory a launch may have unasked");
             fill_items_kernel<V><<<(unsigned)std::min<int64_t>(got.items, (int64_t)sms * 128), 32 * V::kFillWarps, smem, s>>>(
-                row_off, own, place, tab, (int)got.items, out.items, out.slice_off, out.ids, out.words);
+                row_off, own, place, tab, cut, (int)got.items, out.items, out.slice_off, out.ids, out.words);
             IRR_CUDA_TRY(cudaGetLastError());
         }
         return cudaSuccess;
@@ -894,7 +904,18 @@ cudaError_t build_staged(const RowSource& src, int64_t n, int64_t m, bool wide, 
                          cudaStream_t s)
 {
     free_staged(st, s);
-    return wide ? build<WideItem>(src, n, m, most_ids, st, s) : build<NarrowItem>(src, n, m, most_ids, st, s);
+    // Scratch for the tables: a table is at most its item's rows and entries; where
+    // all of them are limited, what is beyond need not be held; and where that does
+    // not fit, a reuse of 2, then 6, may do (8 and more on MD-like graphs).
+    int64_t room = n + m;
+    if (most_ids >= 0) room = std::min(room, most_ids);
+    for (;;) {
+        const cudaError_t e = wide ? build<WideItem>(src, n, m, most_ids, room, st, s)
+                                   : build<NarrowItem>(src, n, m, most_ids, room, st, s);
+        if (e != cudaErrorMemoryAllocation || room <= m / 6) return e;
+        cudaGetLastError();
+        room = room > m / 2 ? m / 2 : m / 6;
+    }
 }
 
 namespace {

@@ -113,3 +113,62 @@ print("done")
 
 def test_failed_setup(limited):
     assert "done" in run_script(limited, FAILED)
+
+
+SETUP = HANDLE + """
+h = handle(layout=irr.IRR_LAYOUT_STAGED)
+h.init()
+st = h.staged()
+h.close()
+words = 4 * (len(st["words"]) + len(st["ids"]) + len(st["slice_off"])) + 32 * len(st["items"])
+# without slots: the half list and the rows, records, positions, results and
+# orders, a cursor per node; then the layout beside them
+bare = 16 * e + (12 + 32 + 12 + 4) * n + (2 << 20)
+slots = 4 * n * ((3 * e // n + 24 + 7) // 8 * 8)
+sliced = 4 * 2 * e * 5 // 4
+configs = {
+    "auto": ({}, bare + words, bare - (2 << 20) - 4 * e),
+    "staged": (dict(layout=irr.IRR_LAYOUT_STAGED), bare + words, bare - (2 << 20) - 4 * e),
+    "sliced": (dict(layout=irr.IRR_LAYOUT_SLICED), bare + sliced, bare - (2 << 20) - 4 * e),
+    "csr": (dict(layout=irr.IRR_LAYOUT_CSR), bare, bare - (2 << 20) - 4 * e),
+    "shard": (dict(layout=irr.IRR_LAYOUT_CSR, shard=True), bare + 4 * e, bare - (2 << 20) - 4 * e),
+}
+for name, (cfg, least, too_little) in configs.items():
+    # less than the slots take with what is made of them: the rows, or the staged layout and its scratch
+    assert least < 8 * e + 44 * n + slots + (4 * e + words if name in ("auto", "staged") else 8 * e), name
+    h = handle(**cfg)
+    want = result(h)
+    h.close()
+    for limit in (4 * least, least, least, too_little, 12 * e, 8 * e + 13 * n):
+        h = handle(**cfg)
+        os.environ["IRR_MEMORY_LIMIT"] = str(limit)
+        try:
+            h.init()
+        except irr.IrregularError as err:
+            assert err.status == irr.IRR_ERR_NOMEM and limit < least, (name, limit, least, str(err))
+            # nothing half made: no step, and the same handle once there is room
+            for _ in range(3):
+                try:
+                    h.step()
+                    raise SystemExit("a step without a set-up")
+                except irr.IrregularError as again:
+                    status = again.status
+                    assert status in (irr.IRR_ERR_NOMEM, irr.IRR_ERR_STATE), str(again)
+            os.environ.pop("IRR_MEMORY_LIMIT")
+            if status == irr.IRR_ERR_STATE:  # the half list was given up
+                h.set_edges(edges)
+            h.init()
+        else:
+            assert limit >= least or name == "auto", (name, limit)
+        got = result(h)
+        if limit >= least:
+            assert got[1] == want[1], (name, limit, got[1], want[1])
+        if got[1] == want[1]:
+            assert np.array_equal(got[0], want[0]), (name, limit)
+        h.close()
+print("done")
+"""
+
+
+def test_setup(limited):
+    assert "done" in run_script(limited, SETUP)
