@@ -662,8 +662,6 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     // no launch may use the old layout: a batch's steps read it on the batch's stream
     H_CUDA(h, h->d_items ? cudaDeviceSynchronize() : cudaStreamSynchronize(h->stream), "layout");
     const int64_t n = h->n;
-    h->shape.lanes_per_row = lanes_per_row;
-    h->shape.block_nodes = block_nodes;
     const int want = h->cfg.layout;
     bool staged = false;
     if (want == IRR_LAYOUT_STAGED && !staged_ok)
@@ -679,13 +677,17 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
             return fail(h, IRR_ERR_ARG, "the staged layout needs 4 lanes per row and stage_smem");
         }
     }
+    if (!staged) {  // (on an error the handle keeps the layout that it has)
+        const int rc = ensure_rows(h);
+        if (rc) return rc;
+    }
+    h->shape.lanes_per_row = lanes_per_row;
+    h->shape.block_nodes = block_nodes;
     h->shape.staged = staged ? (h->st.wide ? 2 : 1) : 0;
     if (staged) {
         free_sliced(&h->sl, h->stream);
         dfree(h, h->part.slots);  // the layout holds the entries now
     } else {
-        const int rc = ensure_rows(h);
-        if (rc) return rc;
         free_staged(&h->st, h->stream);
         if (want == IRR_LAYOUT_CSR) {
             free_sliced(&h->sl, h->stream);

@@ -172,3 +172,44 @@ print("done")
 
 def test_setup(limited):
     assert "done" in run_script(limited, SETUP)
+
+
+RELAYOUT = HANDLE + """
+star = np.stack([np.zeros(3000, np.int32), np.arange(1, 3001, dtype=np.int32)], 1)
+hub = irr.Handle(irr.default_config(map_idx=irr.IRR_MAP_LJ_MOLDYN))
+hub.set_params(irr.moldyn_params(float(side), rc))
+hub.set_edges(star)
+hub.set_nodes(pos[:3001], 12)
+hub.init()
+assert hub.info().layout != irr.IRR_LAYOUT_STAGED
+h = handle()
+h.init()
+assert h.info().layout == irr.IRR_LAYOUT_STAGED
+want, shape = result(h)[0], (h.info().lanes_per_row, h.info().block_nodes, h.info().num_blocks)
+for _ in range(5):
+    b = irr.Batch(0)
+    b.add(h)
+    b.add(hub)
+    os.environ["IRR_MEMORY_LIMIT"] = str(8 * e)  # not the rows beside the layout
+    try:
+        b.finalize()
+        raise SystemExit("laid out without room")
+    except irr.IrregularError as err:
+        assert err.status == irr.IRR_ERR_NOMEM, str(err)
+    got, layout = result(h)
+    assert layout == irr.IRR_LAYOUT_STAGED and np.array_equal(got, want)
+    assert shape == (h.info().lanes_per_row, h.info().block_nodes, h.info().num_blocks)
+    b.close()
+b = irr.Batch(0)
+b.add(h)
+b.add(hub)
+b.finalize()
+assert h.info().layout != irr.IRR_LAYOUT_STAGED
+b.close()
+print("done")
+"""
+
+
+def test_failed_relayout(limited):
+    """The handle keeps the layout that it had."""
+    assert "done" in run_script(limited, RELAYOUT)
