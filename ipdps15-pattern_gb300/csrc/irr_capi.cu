@@ -615,6 +615,16 @@ int ensure_rows(irr_handle* h)
     return pack_slots(h);
 }
 
+// What a set-up partitioned handle holds.
+void count_bytes(irr_handle* h)
+{
+    const int64_t n = h->n;
+    h->dev_bytes = 2 * (int64_t)(n > 0 ? n : 1) * (int64_t)sizeof(float4) + (int64_t)h->raw_cap +
+                   (int64_t)(2 * n + n + 1) * 4 + (h->part.col ? h->m * 4 : 0) +
+                   (h->sl.lanes ? 4 * (h->sl.words + h->sl.slices + 1) : 0) +
+                   (h->shape.staged ? 4 * (h->st.nwords + h->st.nids + h->st.slices + 1) : 0);
+}
+
 // The staged layout into h->st (IRR_OK without it where AUTO goes without).
 int make_staged(irr_handle* h)
 {
@@ -709,10 +719,7 @@ int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int sta
     if (rc) return rc;
     rc = upload_items(h);
     if (rc) return rc;
-    h->dev_bytes = 2 * (int64_t)(n > 0 ? n : 1) * (int64_t)sizeof(float4) + (int64_t)h->raw_cap +
-                   (int64_t)(2 * n + n + 1) * 4 + (h->part.col ? h->m * 4 : 0) +
-                   (h->sl.lanes ? 4 * (h->sl.words + h->sl.slices + 1) : 0) +
-                   (h->shape.staged ? 4 * (h->st.nwords + h->st.nids + h->st.slices + 1) : 0);
+    count_bytes(h);
     return IRR_OK;
 }
 
@@ -1234,9 +1241,10 @@ int irr_get_partition(irr_handle* h, int32_t* perm, int64_t* row_off, int32_t* c
     if (!h->inited) return fail(h, IRR_ERR_STATE, "no partition before irr_init");
     DeviceGuard dev_guard(h->device);
     const int64_t n = h->n, m = h->m;
-    if (col && m > 0) {
+    if (col && m > 0 && !h->part.col) {  // made, and kept
         const int rc = ensure_rows(h);
         if (rc) return rc;
+        count_bytes(h);
     }
     if (perm && n > 0)
         H_CUDA(h, cudaMemcpyAsync(perm, h->part.perm, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, h->stream), "copy perm");
