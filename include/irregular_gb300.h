@@ -97,7 +97,10 @@ enum irr_order {
 
 /* Partitioned: how each node block's directed entries are laid out. */
 enum irr_layout {
-    /* Sliced when its padding is at most half the entry count, else CSR. */
+    /* Staged where it applies -- to the limits below, or else to wider ones
+     * (1008 nodes, rows of 1023 entries) -- and its tables hold at most a third
+     * as many ids as the rows hold entries (and there is memory for it); else
+     * sliced when its padding is at most half the entry count; else CSR. */
     IRR_LAYOUT_AUTO = 0,
     /* Rows of entries (CSR), columns ascending within a row. */
     IRR_LAYOUT_CSR = 1,
@@ -114,8 +117,8 @@ enum irr_layout {
      * summed in an order chosen to spread shared-memory banks (not the CSR
      * order), so results differ from CSR / sliced in the last bits; 4 lanes
      * per row.  Applies when every 8 consecutive rows touch at most 640
-     * distinct nodes and no row exceeds ~440 entries; else IRR_ERR_CAPACITY
-     * (AUTO falls back). */
+     * distinct nodes and no row exceeds 888 entries; else IRR_ERR_CAPACITY
+     * (AUTO takes wider limits or another layout). */
     IRR_LAYOUT_STAGED = 3
 };
 
@@ -168,7 +171,7 @@ typedef struct irr_info {
     int32_t lanes_per_row;
     int32_t stage_smem;
     int32_t exec;
-    int32_t layout;          /* enum irr_layout in use (CSR or SLICED)              */
+    int32_t layout;          /* enum irr_layout in use (CSR, SLICED or STAGED)      */
     int32_t order;           /* enum irr_order of the node order                    */
     int64_t num_slots;       /* entry slots stored: num_entries plus padding        */
     int64_t own_lo;          /* rows reduced: caller ids [own_lo, own_hi)           */
@@ -212,7 +215,8 @@ IRR_API int irr_set_edges_device(irr_handle *h, const int32_t *d_edges, int64_t 
  * memory on a 16-byte boundary is read in place, asynchronously: leave it
  * unchanged until the next irr_get_result or irr_sync returns. */
 IRR_API int irr_set_nodes(irr_handle *h, const void *node_data, int elm_size, int64_t num_nodes);
-/* Same, from device memory. */
+/* Same, from device memory (of any GPU), in the order of the handle's stream:
+ * after irr_init, this GPU's is read in place at its record's alignment. */
 IRR_API int irr_set_nodes_device(irr_handle *h, const void *d_node_data, int elm_size,
                          int64_t num_nodes);
 
@@ -273,8 +277,9 @@ IRR_API int irr_get_info(const irr_handle *h, irr_info *info);
 /* Partition outputs (partitioned mode, after irr_init), copied to host:
  * perm[new] = old node id, row_off[num_nodes + 1] (int64) and col[num_entries]
  * (the neighbour's new id of every directed entry, rows in node order,
- * entries within a row in edge-list order, idx0 side first).  Any pointer may
- * be NULL. */
+ * ascending within a row).  Any pointer may be NULL.  A handle on the staged
+ * layout keeps no rows: the first call with col makes them (4 bytes an entry
+ * of device memory, kept). */
 IRR_API int irr_get_partition(irr_handle *h, int32_t *perm, int64_t *row_off, int32_t *col);
 
 /* The staged layout of a handle that uses it (IRR_ERR_STATE otherwise),
@@ -431,10 +436,10 @@ IRR_API int irr_batch_add(irr_batch *b, irr_handle *h);
  * candidate shapes (lanes per node row x rows per work item) on this data and
  * keeps the fastest, remembered per GPU and size class for the process. */
 IRR_API int irr_batch_finalize(irr_batch *b, int autotune);
-/* One reduction of every instance: one queue reset + one launch, or one CUDA
- * graph replay once irr_batch_capture has run.  Enqueued; does not wait. */
+/* One reduction of every instance: one launch, or one CUDA graph replay once
+ * irr_batch_capture has run.  Enqueued; does not wait. */
 IRR_API int irr_batch_step(irr_batch *b);
-/* Captures one step (queue reset + launch) into a CUDA graph replayed by
+/* Captures one step (one launch) into a CUDA graph replayed by
  * later irr_batch_step calls; needs a non-default stream. */
 IRR_API int irr_batch_capture(irr_batch *b);
 IRR_API int irr_batch_sync(irr_batch *b);

@@ -8,7 +8,7 @@
 // serves all of them: its CTAs claim (instance, block) items from one queue,
 // which is the reference's per-part atomicAdd queue (gpu_kernel.cu:64-72)
 // generalised across instances.  After irr_batch_capture a step is one CUDA
-// graph replay (queue reset + launch).
+// graph replay (of that one launch, which leaves its queue cleared).
 //
 // Autotuning: candidate shapes (lanes per node row x rows per work item) are
 // timed on the actual data with CUDA events, a few launches each; the fastest

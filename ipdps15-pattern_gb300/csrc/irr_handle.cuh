@@ -93,12 +93,12 @@ struct irr_handle {
     int64_t coord_n = -1;
 };
 
+// Brings the row offsets to the host, where CSR and sliced work items are cut
+// from them (once per partition; the staged layout needs none).
+int irr_host_row_off(irr_handle* h);
 // (Re)builds the handle's entry layout for G lanes per row as its config asks
 // (staged, sliced or CSR), then its instance descriptor and work items, so
 // that the three always agree.  staged_ok = 0 keeps an AUTO handle off the
 // staged layout (a handle configured IRR_LAYOUT_STAGED then fails with
 // IRR_ERR_STATE).  Partitioned, initialised handles only.
-// Brings the row offsets to the host, where CSR and sliced work items are cut
-// from them (once per partition; the staged layout needs none).
-int irr_host_row_off(irr_handle* h);
 int irr_ensure_layout(irr_handle* h, int lanes_per_row, int block_nodes, int staged_ok = 1);

@@ -175,9 +175,13 @@ struct Staged {
 };
 // The wide limits, for rows that touch more nodes.  An item of 6,400 words and
 // its table take about two thirds of the halo kernel's ring, so that much of the
-// next one loads beside it: 1,048,576 nodes with ~248 neighbours 489 us a step
-// at 9,984 words (64 rows an item, the whole ring) -> 450, 473 at 6,000 (fewer
-// rows share a table); with 300 neighbours 195 -> 187 (262,144 nodes).
+// next one loads beside it; smaller items share a table among fewer rows.  A
+// reduction, us, at 5,600, 6,400, 6,900, 7,424 and 8,400 words (random box, then
+// fcc): 1,000,000 nodes with 250 neighbours 431 422 412 417 436, 439 at each;
+// 262,144 with 300 170 170 169 169 178, 178 178 186 186 192; with 350 230 216 216
+// 222 224, 232 227 227 231 231; with 420 312 313 313 315 316, 310 310 307 305 306;
+// up to 250 neighbours at 100,000 and 262,144 nodes all alike.  9,984 words (the
+// whole ring) were 9 % slower at 1,048,576 nodes with 248.
 constexpr int kHaloWideTabMax = 1008;
 constexpr int kHaloWideStreamMax = 6400;
 // Where a graph's rows are, in execution order, each row's columns in any

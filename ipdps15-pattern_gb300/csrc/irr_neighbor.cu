@@ -10,11 +10,14 @@
 //      contiguous and each is one load, not an id load and then a dependent
 //      position load;
 //   4. one thread per node (in cell order, so a warp shares cells) scans the
-//      27 surrounding cells for partners j > i with r2 <= cut2, first counting,
-//      then -- after a scan of the counts -- writing them; a warp per row then
-//      sorts each row by j.  A caller that re-sorts the pairs anyway gets
-//      them in no particular order, from a half stencil (pairs_half_kernel:
-//      each pair found once, from one end), written straight as pairs.
+//      27 surrounding cells for partners j > i with r2 <= cut2 and writes them
+//      into slots of its own (slot_partners_kernel); warps then sort each row
+//      by j and write its pairs (slot_pairs_kernel).  Where the cells do not
+//      decide the images, a node has more partners than slots, or the slots do
+//      not fit, partners are counted first and written after a scan of the
+//      counts (pairs_kernel), then sorted and expanded.  A caller that re-sorts
+//      the pairs anyway gets them in no particular order, from a half stencil
+//      (pairs_half_kernel: each pair found once, from one end).
 // The pair rule is shared bit for bit with the CPU oracle: d = x_i - x_j in
 // float, wrapped once by +-box when |d| > box/2 (periodic), r2 = ((dx*dx +
 // dy*dy) + dz*dz) with every operation rounded.  Output: pairs (i, j), i < j,
@@ -872,9 +875,10 @@ cudaError_t build_neighbor_list(const float4* pos, int64_t n, float box, float c
 namespace {
 
 // Where the nodes are too few warps to hide the search's latency, 8 lanes share
-// a node's candidates: a search 35 us at 2,048 nodes (with a lane each 189 before
-// its loop lost its branches), 28 against 53 at 6,912, 39 against 55 at 16,384; at
-// 32,000 100 MD steps with 5 rebuilds 2.54 against 2.63 ms; 94 against 66 at 55,296.
+// a node's candidates.  100 MD steps with 5 rebuilds, us with 8 lanes a node and
+// with one: 6,912 nodes 1980 and 2195, 16,384 2274 and 2497, 32,000 2513 and 2602,
+// 37,044 2966 and 3028, 42,592 3163 and 3131, 55,296 3329 and 3256, 70,304 3907 and
+// 3728.
 constexpr int64_t kLanesNodes = 40000;
 
 template <int MODE>

@@ -11,12 +11,15 @@
 //      (default) or Morton index (bits interleaved);
 //   2. stable LSD radix sort of (key, node) -> perm[new] = old, inv[old] = new;
 //   3. every half edge (i, j) at list position t becomes the directed entries
-//      (inv[i] <- inv[j]) and (inv[j] <- inv[i]), laid out in (row, col)
-//      order: a degree count + scan gives the row offsets, the entries are
-//      filled at per-row cursors and each row is sorted by one warp, in
-//      registers (rows up to 256 entries) or in shared memory (up to
-//      kRowSortMax); a graph with a longer row is put in order by stable radix
-//      sorts by column, then by row.
+//      (inv[i] <- inv[j]) and (inv[j] <- inv[i]) of its two rows.  A list sorted
+//      by idx0 is counted as it is filled into slots per row (slot_rows_kernel),
+//      from which the staged layout is made; CSR and slices want (row, col)
+//      order: each row is sorted by one warp, in registers (rows up to 256
+//      entries) or in shared memory (up to kRowSortMax).  Other lists, rows
+//      longer than the slots and slots that do not fit: a degree count + scan
+//      gives the row offsets, the entries are filled at per-row cursors and
+//      sorted so; a graph with a row above kRowSortMax is put in order by stable
+//      radix sorts by column, then by row.
 // Node blocks are then consecutive ranges of rows.  Every output is an
 // integer function of the inputs, reproduced bit for bit by the CPU oracle.
 // 4. Optionally the sliced layout (struct Sliced): the same entries regrouped

@@ -856,9 +856,11 @@ __device__ __forceinline__ void halo_slice(const HaloSlice& sl, const InstHot& I
     write_row<4>(I.force, (int64_t)sl.row0 + ((hdr >> 24) & 0x3fu), !(hdr >> 31), ax, ay, az, lane);
 }
 
-// WIDE: items to the wide limits, each up to the whole ring: a CTA loads and
-// computes in turn while the SM's other CTAs compute.  Its table's ids are too
-// many for the producer's registers and are read when there is room for them.
+// WIDE: items to the wide limits, each up to two thirds of the ring, beside which
+// much of the next one loads.  Its table's ids are too many for the producer's
+// registers and are read when there is room for them, so ids and positions are
+// one chain, and that, not issue, bounds it: 262,144 nodes with 248 neighbours
+// issue in 48 % of the active cycles (narrow items at 64 neighbours: 77 %).
 template <bool PERIODIC, bool WIDE, class Src>
 __global__ void __launch_bounds__(kPipeThreads, kCtasPerSm) halo_kernel(
     const InstDesc* __restrict__ insts, const WorkItem* __restrict__ items, int num_items,
@@ -1076,8 +1078,10 @@ cudaError_t launch_halo_src(const InstDesc* d_insts, const WorkItem* d_items, in
     if (grid <= 0 || num_items <= 0) return cudaSuccess;
     // claims run two items ahead of a CTA's positions, which with a few items
     // per CTA leaves some with three and others with one: up to 4 items per CTA
-    // they are dealt out in turn (65,536 nodes, 1.7 items per CTA: 10.0 -> 8.7
-    // us; 4M nodes, 108 per CTA, dealt out: 386 -> 429)
+    // they are dealt out in turn.  Claimed and dealt, us at 64 neighbours: 1 item
+    // per CTA 8.9 and 8.6, 1.5 13.6 and 10.9, 2.5 18.0 and 14.5, 3.5 21.5 and
+    // 19.5, 4 22.4 and 22.3, 5 26.8 and 24.5, 6 29.8 and 29.7, 8 36.3 and 38.1, 16
+    // 63.8 and 69.6, 108 386 and 429; at 32 neighbours they cross at 6 too.
     int* const queue = num_items <= 4 * grid ? nullptr : d_queue;
     return launch_chained(kern, (unsigned)std::min(grid, num_items), kPipeThreads, kHaloRingBytes, s, d_insts,
                           d_items, num_items, queue, d_status, wp.wait_ns, wp.withhold, src);
