@@ -17,7 +17,8 @@
  * Device memory: handles, systems and set-ups allocate from a memory pool of
  * the library's own (one per device, made by cudaMemPoolCreate).  What they free
  * stays there for the next; irr_destroy, irr_md_destroy, irr_device_free and the
- * end of irr_serve_run give back to the driver what is unused above 8 GB.
+ * end of irr_serve_run give back to the driver what is unused above 6 GB (with
+ * the lists that irr_device_free keeps, at most 8 GB stay with the library).
  */
 #ifndef IRREGULAR_GB300_H_
 #define IRREGULAR_GB300_H_
@@ -462,8 +463,8 @@ IRR_API int irr_neighbor_build(int device, void *stream, const void *pos, int po
                                int pos_on_device, int64_t n, float box, float list_cut2,
                                int32_t **d_edges, int64_t *num_edges);
 /* Frees a list, after all work on the device (a plain cudaMalloc'd block: peers
- * and cudaIpcGetMemHandle take its address).  Up to 1 GB of freed lists per
- * device is kept for the next ones; larger ones go back to the driver. */
+ * and cudaIpcGetMemHandle take its address).  Up to 2 GB of freed lists per
+ * device is kept for the next ones; what is beyond goes back to the driver. */
 IRR_API int irr_device_free(int device, void *d_ptr);
 
 /* ------------------------------------------------- molecular dynamics

@@ -279,7 +279,7 @@ inline bool sliced_pays(const Sliced& sl, int64_t entries)
 // cudaFreeAsync stay in the pool for the next allocation instead of going back
 // to the driver at every synchronisation (the default pool's behaviour), so a
 // rebuild that frees and re-allocates ~300 MB of layout does not re-map it.
-// What is freed stays in the pool, up to 8 GB of it after a handle, a list or a
+// What is freed stays in the pool, up to 6 GB of it after a handle, a list or a
 // system is freed (irr_pool_trim).
 cudaError_t irr_malloc_async(void** p, size_t bytes, cudaStream_t s);
 template <class T>
@@ -308,14 +308,14 @@ struct Temps {
 
 // Edge lists, which are the caller's: cudaMalloc'd, so that peers and other
 // processes reach them as any device memory.  irr_free_list, after the last use
-// of p by the device, keeps up to 1 GB of freed ones per device for the next
+// of p by the device, keeps up to 2 GB of freed ones per device for the next
 // list: of 370 MB, 1,000,003 nodes' list, the cudaMalloc takes 140 to 200 us and the
 // cudaFree 180 to 200, the search 960.  Memory that the library did not give out
 // as a list is cudaFree'd.
 cudaError_t irr_malloc_list(void** p, size_t bytes);
 cudaError_t irr_free_list(void* p);
 
-// Gives back to the driver what the pool of `device` holds unused above 8 GB.
+// Gives back to the driver what the pool of `device` holds unused above 6 GB.
 void irr_pool_trim(int device);
 
 // How long a kernel's device-side waits may last before it gives up

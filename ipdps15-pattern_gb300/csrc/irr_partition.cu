@@ -1426,14 +1426,14 @@ cudaMemPool_t pool_of(int dev)  // null: none could be made
     return pool;
 }
 
-// Lists in the caller's hands, and freed ones kept for the next list (the
-// longest kept first).
+// Lists in the caller's hands, and freed ones kept for the next list, the oldest
+// first.
 struct ListBlock {
     void* p;
     size_t bytes;
     int device;
 };
-constexpr size_t kSpareBytes = 1ull << 30;
+constexpr size_t kSpareBytes = 2ull << 30;
 std::mutex g_list_mutex;
 std::vector<ListBlock> g_lists, g_spares;
 
@@ -1501,12 +1501,16 @@ cudaError_t irr_malloc_list(void** p, size_t bytes)
 {
     int dev = 0;
     IRR_CUDA_TRY(cudaGetDevice(&dev));
+    // whole pages of 2 MB (of 64 KB for short lists), and a 64th more: the next
+    // list is seldom just as long
+    const size_t page = bytes < (16ull << 20) ? 64ull << 10 : 2ull << 20;
+    const size_t more = (bytes + bytes / 64 + page - 1) / page * page;
     {
         std::lock_guard<std::mutex> lock(g_list_mutex);
         size_t best = g_spares.size();
         for (size_t k = 0; k < g_spares.size(); k++) {
             const ListBlock& b = g_spares[k];
-            if (b.device == dev && b.bytes >= bytes && b.bytes / 4 * 3 <= bytes &&
+            if (b.device == dev && b.bytes >= bytes && b.bytes / 4 * 3 <= more &&
                 (best == g_spares.size() || b.bytes < g_spares[best].bytes))
                 best = k;
         }
@@ -1517,9 +1521,6 @@ cudaError_t irr_malloc_list(void** p, size_t bytes)
             return cudaSuccess;
         }
     }
-    // whole 2 MB pages, and a 64th more: the next list is seldom just as long
-    constexpr size_t kPage = 2ull << 20;
-    const size_t more = (bytes + bytes / 64 + kPage - 1) / kPage * kPage;
     size_t got = more;
     auto get = [&]() { return no_room(dev, got) ? cudaErrorMemoryAllocation : cudaMalloc(p, got); };
     cudaError_t e = get();
@@ -1561,7 +1562,7 @@ cudaError_t irr_free_list(void* p)
 
 void irr_pool_trim(int device)
 {
-    constexpr uint64_t kKeep = 8ull << 30;
+    constexpr uint64_t kKeep = 6ull << 30;
     if (device < 0 || device >= kMaxPoolDevices) return;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
     const cudaMemPool_t pool = g_pools[device];
