@@ -1547,6 +1547,8 @@ cudaError_t irr_free_list(void* p)
     ListBlock b{p, 0, -1};
     {
         std::lock_guard<std::mutex> lock(g_list_mutex);
+        for (const ListBlock& spare : g_spares)
+            if (spare.p == p) return cudaErrorInvalidValue;  // freed before
         for (size_t k = 0; k < g_lists.size(); k++) {
             if (g_lists[k].p != p) continue;
             b = g_lists[k];

@@ -84,6 +84,23 @@ def test_same_block_again(built_lib, n):
     assert len(seen) == 1
 
 
+def test_freed_twice(built_lib, oracle_lib):
+    """The second free is refused, and the block is not given out twice."""
+    import irregular_gb300 as irr
+    pos, side = random_box(4000, 0.9, 2)
+    want = oracle_lib.neighbor_half_list(pos, float(side), np.float32(6.25))
+    first = irr.neighbor_build(pos, float(side), 6.25)
+    ptr, free = C.c_void_p(first.ptr), irr.load().irr_device_free
+    assert free(0, ptr) == irr.IRR_OK
+    assert free(0, ptr) == irr.IRR_ERR_CUDA
+    first.ptr = 0
+    lists = [irr.neighbor_build(pos, float(side), 6.25) for _ in range(3)]
+    assert len({x.ptr for x in lists}) == 3
+    for x in lists:
+        assert np.array_equal(x.to_host(), want)
+        x.close()
+
+
 def test_freed_lists_go_back(built_lib):
     torch = pytest.importorskip("torch")
     import irregular_gb300 as irr
