@@ -3,6 +3,7 @@ process, as any allocation of its own; a freed list's block serves the next list
 of about its length, and what is kept beyond 2 GB goes back to the driver, as does
 what the library's pool holds unused above 6 GB."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -82,6 +83,40 @@ def test_same_block_again(built_lib, n):
         seen.add(lst.ptr)
         lst.close()
     assert len(seen) == 1
+
+
+def test_several_threads(built_lib, oracle_lib):
+    """Lists made and freed by six threads at once, from the same kept blocks."""
+    import irregular_gb300 as irr
+    want = []
+    for k, n in enumerate([3000, 3050, 12_000, 700]):
+        pos, side = random_box(n, 0.9, k)
+        want.append((pos, float(side), oracle_lib.neighbor_half_list(pos, float(side), np.float32(6.25))))
+    failed = []
+
+    def work(t):
+        rng = np.random.default_rng(t)
+        try:
+            held = []
+            for _ in range(80):
+                pos, side, ref = want[int(rng.integers(len(want)))]
+                held.append((irr.neighbor_build(pos, side, 6.25), ref))
+                if len(held) > 2:
+                    got, ref = held.pop(int(rng.integers(len(held))))
+                    assert np.array_equal(got.to_host(), ref)
+                    got.close()
+            for got, ref in held:
+                assert np.array_equal(got.to_host(), ref)
+                got.close()
+        except BaseException as e:  # noqa: BLE001 -- told to the test's own thread
+            failed.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
 
 
 def test_freed_twice(built_lib, oracle_lib):
